@@ -243,6 +243,20 @@ int linf_norm_dist_backward_weight(const float* grad_output, const float* input,
                                    int B, int CO, int CI, int G, int HW,
                                    float* grad_weight, float p, void* stream);
 
+/*
+ * One or both of the two gradients above (either pointer may be NULL, not both) in one pass over the terms.
+ * The workspace (256-byte aligned, contents irrelevant, free again when the call's work on the stream is done) has
+ * the size the query answers for the same arguments; 0, or a NULL workspace, means the separate kernels are used.
+ * Same fixed summation order in every run.
+ */
+size_t linf_norm_dist_backward_workspace_bytes(int B, int CO, int CI, int G, int HW, float p,
+                                               int want_input, int want_weight);
+int linf_norm_dist_backward(const float* grad_output, const float* input,
+                            const float* weight, const float* output,
+                            int B, int CO, int CI, int G, int HW,
+                            float* grad_input, float* grad_weight, float p,
+                            void* workspace, size_t workspace_bytes, void* stream);
+
 /* ---------------------------------------------------------------------------------
  * optimiser step (next to the distance neuron on the training path)
  * --------------------------------------------------------------------------------- */

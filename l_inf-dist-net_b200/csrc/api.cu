@@ -292,4 +292,23 @@ int linf_norm_dist_backward_weight(const float* grad_output, const float* input,
     return lp_backward_weight(grad_output, input, weight, output, d, grad_weight, p, as_stream(stream));
 }
 
+size_t linf_norm_dist_backward_workspace_bytes(int B, int CO, int CI, int G, int HW, float p, int want_input, int want_weight) {
+    Dims d;
+    if (bad_p(p) || make_dims(B, CO, CI, G, HW, &d)) return 0;
+    return lp_backward_both_workspace(d, p, want_input != 0, want_weight != 0);
+}
+
+int linf_norm_dist_backward(const float* grad_output, const float* input, const float* weight, const float* output,
+                            int B, int CO, int CI, int G, int HW, float* grad_input, float* grad_weight, float p,
+                            void* workspace, size_t workspace_bytes, void* stream) {
+    if (!grad_output || !input || !weight || !output) return LINF_ERR_NULL;
+    if (!grad_input && !grad_weight) return LINF_ERR_NULL;
+    if (bad_p(p)) return LINF_ERR_P;
+    Dims d;
+    int rc = make_dims(B, CO, CI, G, HW, &d);
+    if (rc) return rc;
+    return lp_backward_both(grad_output, input, weight, output, d, grad_input, grad_weight, p, workspace, workspace_bytes,
+                            as_stream(stream));
+}
+
 }  // extern "C"

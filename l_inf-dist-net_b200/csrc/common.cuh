@@ -99,6 +99,10 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, int src
     unsigned s = (unsigned)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(s), "l"(gmem), "r"(src_bytes));
 }
+__device__ __forceinline__ void cp_async4(void* smem, const void* gmem, int src_bytes) {
+    unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(s), "l"(gmem), "r"(src_bytes));
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N)); }
@@ -170,5 +174,9 @@ int lp_backward_input(const float* g, const float* x, const float* w, const floa
                       const Dims& d, float* gx, float p, cudaStream_t st);
 int lp_backward_weight(const float* g, const float* x, const float* w, const float* y,
                        const Dims& d, float* gw, float p, cudaStream_t st);
+// one or both gradients in one pass (lp_backward.cu); without workspace, or where that is 0 bytes: the two above
+size_t lp_backward_both_workspace(const Dims& d, float p, bool dox, bool dow);
+int lp_backward_both(const float* g, const float* x, const float* w, const float* y, const Dims& d,
+                     float* gx, float* gw, float p, void* ws, size_t ws_bytes, cudaStream_t st);
 
 }  // namespace linf

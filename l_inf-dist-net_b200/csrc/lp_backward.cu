@@ -1,0 +1,472 @@
+// Both gradients of the finite-p distance neuron in one pass over the (b, o, i) terms, for dense layers
+// (HW == 1, at least 32 channels per group on either side; no alignment or divisibility is asked for).
+//
+//   T[b,o,i]  = g[b,o] * s * |s|^(p-2),   s = (x[b,i] - w[o,i]) / y[b,o]
+//   gx[b,i]   =  sum_o T        gw[o,i] = -sum_b T
+//
+// Bound: FP32 issue (p with a fraction: the special-function unit, one log2 / exp2 pair per term).  What a term costs is
+// its power, and the two gradients want the same power, so a thread
+// that owns (b, i) pairs walks over the outputs o, adds every term to its gx register and to a running sum
+// over its own rows for gw.  The rows of a thread are 16 of the batch and its columns two neighbours of the input, lanes
+// run along i: nothing is exchanged between lanes, the warps' gw sums meet in shared memory once per
+// eight outputs.  All arithmetic is packed two rows at a time (f32x2).
+//
+// p = 8 and 16 run without the division by y: T = h * t^(p-1) with h = g / y^(p-1) worked out once per (b, o)
+// by the preparation kernel, which also looks whether every y lies where neither factor can leave the range of
+// a float; if one does not, the kernel takes the scaled form instead (`flag`).  Per term of both gradients:
+// 7 lane operations at p = 8 (subtraction, four products, two multiply-adds) against 2 x 7 of two separate passes.
+//
+// Work split.  A CTA owns 64 input columns, a range of outputs and a range of batch tiles (16 rows per warp).
+// It takes its batch tiles one after the other; the gw sums of the first are stored, the later ones added by
+// the same thread with `red` (program order, so the result is the same in every run).  Ranges
+// of outputs leave partial gx, ranges of batch tiles partial gw in the workspace, added up in ascending
+// order by a last kernel.  `plan_both` chooses the number of ranges.
+//
+// Measured on one B200, both gradients, us, two separate kernels (lp_tiled.cu) -> here:
+//   B = 512, Din = Dout = 5120: p = 8: 6585 -> 3323, 16: 8060 -> 4143, 64: 11142 -> 10680, 23.7: 20513 -> 10965, 200.3: 26120 -> 15582
+//   B = 8, Din = Dout = 5120, p = 8: 1023 -> 275     B = 16384, Din = 576, Dout = 128, p = 8: 1934 -> 391
+//   B = 203, Din = 1027, Dout = 1333 (the generic kernels before), p = 8: 1058 -> 135
+#include <math.h>
+
+#include "common.cuh"
+
+namespace linf {
+namespace {
+
+typedef unsigned long long u64;
+
+__device__ __forceinline__ u64 mul2(u64 a, u64 b) { u64 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) { u64 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+__device__ __forceinline__ u64 pack2(float a, float b) { u64 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ u64 abs2(u64 a) { return a & 0x7fffffff7fffffffULL; }
+__device__ __forceinline__ float lg2_approx(float a) { float r; asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a)); return r; }
+__device__ __forceinline__ float ex2_approx(float a) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a)); return r; }
+
+struct PowQ { int m; float f; };       // p - 2 = m + f
+
+template <int E>
+__device__ __forceinline__ u64 pow2_ct(u64 a) {       // a^E, E >= 1
+    if constexpr (E == 1) return a;
+    else if constexpr (E % 2 == 0) { const u64 h = pow2_ct<E / 2>(a); return mul2(h, h); }
+    else if constexpr (E % 4 == 3) { const u64 h = pow2_ct<(E - 1) / 2>(a); return mul2(mul2(h, a), h); }   // (h * a) * h
+    else return mul2(pow2_ct<E - 1>(a), a);
+}
+
+// s * |s|^(p-2) for a pair.  IP > 0: p is that even integer (the sign comes with the odd power).  IP <= 0: p - 2 = q.m + q.f at run time,
+// q.m < 2^-IP; the bit tests are uniform over the grid.
+template <int IP>
+__device__ __forceinline__ u64 factor2(u64 s, const PowQ q) {
+    if constexpr (IP > 0) {
+        return pow2_ct<IP - 1>(s);
+    } else {
+        constexpr int NB = -IP;
+        u64 v = s;
+        if (q.m & 1) v = mul2(v, abs2(s));
+        u64 b = s;
+#pragma unroll
+        for (int k = 1; k < NB; ++k) {
+            if ((q.m >> k) == 0) break;
+            b = mul2(b, b);
+            if ((q.m >> k) & 1) v = mul2(v, b);
+        }
+        if (q.f != 0.f) {
+            float s0, s1;
+            unpack_f32x2(s, s0, s1);
+            // s = 0: exp2(-inf) = 0
+            v = mul2(v, pack2(ex2_approx(q.f * lg2_approx(fabsf(s0))), ex2_approx(q.f * lg2_approx(fabsf(s1)))));
+        }
+        return v;
+    }
+}
+
+constexpr int KO = 8;            // outputs per stage
+constexpr int TI = 64;           // input columns per CTA (two per lane)
+constexpr int RW = 16;           // batch rows per warp
+constexpr int STAGES = 3;
+
+struct BothParams {
+    const float* x; const float* w;
+    const float* h; const float* g; const float* r;      // [CO][Bp]: g / y^(p-1) (p = 8, 16 only), g, 1 / y
+    const int* flag;                                     // [1]: some y needs the scaled form (p = 8, 16 only)
+    float* gx; float* gw;                                // results, or the partial results of range 0
+    size_t gx_step, gw_step;                             // floats between the partial results of consecutive ranges
+    int B, Bp, COg, CIg, G, CI;
+    int tiles_i, n_o, n_b;                               // 64-column tiles per group, ranges of outputs / of batch tiles
+    PowQ q;
+};
+
+template <int WARPS, bool SCALED>
+__host__ __device__ constexpr int stage_floats() { return KO * TI + (SCALED ? 2 : 1) * KO * WARPS * RW; }
+
+template <int IP, int WARPS, bool DOX, bool DOW, bool AL, bool SCALED>
+__device__ __forceinline__ void both_body(const BothParams& p, float* smem) {
+    constexpr int NT = WARPS * 32, BT = WARPS * RW;
+    constexpr int STAGE = stage_floats<WARPS, SCALED>();
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    float* part = smem + STAGES * STAGE;                 // [2][WARPS][KO][TI]
+    int id = blockIdx.x;
+    const int ti = id % p.tiles_i; id /= p.tiles_i;
+    const int g = id % p.G; id /= p.G;
+    const int ro = id % p.n_o, rb = id / p.n_o;
+    const int KT_all = (p.COg + KO - 1) / KO, BT_all = p.Bp / BT;
+    const int kt0 = (int)((long long)KT_all * ro / p.n_o), kt1 = (int)((long long)KT_all * (ro + 1) / p.n_o);
+    const int bt0 = (int)((long long)BT_all * rb / p.n_b), bt1 = (int)((long long)BT_all * (rb + 1) / p.n_b);
+    const int i0 = ti * TI, ic = i0 + 2 * lane;          // first of this thread's two columns
+    const float* wg = p.w + (size_t)g * p.COg * p.CIg;
+    const float* sa = (SCALED ? p.g : p.h) + (size_t)g * p.COg * p.Bp;
+    const float* sr = p.r + (size_t)g * p.COg * p.Bp;
+    float* gw = p.gw + (DOW ? (size_t)rb * p.gw_step : 0) + (size_t)g * p.COg * p.CIg;
+
+    for (int bt = bt0; bt < bt1; ++bt) {
+        const int b_first = bt * BT;
+        // Outputs past the group and rows past the batch read the last valid row of w and x instead of zeros: their h and g are
+        // zero, but t^(p-1) has to stay finite, as it is for every pair that has a y.
+        auto load = [&](int s, int kt) {
+            float* st = smem + s * STAGE;
+            const int o0 = kt * KO;
+            if (AL) {
+#pragma unroll
+                for (int q = tid; q < KO * TI / 4; q += NT) {
+                    const int r = q / (TI / 4), c = (q % (TI / 4)) * 4;
+                    const bool in = i0 + c < p.CIg;
+                    cp_async16(st + r * TI + c, wg + (in ? (size_t)min(o0 + r, p.COg - 1) * p.CIg + i0 + c : 0), in ? 16 : 0);
+                }
+            } else {
+#pragma unroll
+                for (int q = tid; q < KO * TI; q += NT) {
+                    const int r = q / TI, c = q % TI;
+                    const bool in = i0 + c < p.CIg;
+                    cp_async4(st + r * TI + c, wg + (in ? (size_t)min(o0 + r, p.COg - 1) * p.CIg + i0 + c : 0), in ? 4 : 0);
+                }
+            }
+#pragma unroll
+            for (int q = tid; q < KO * BT / 4; q += NT) {
+                const int r = q / (BT / 4), c = (q % (BT / 4)) * 4;
+                const bool in = o0 + r < p.COg;
+                const size_t off = in ? (size_t)(o0 + r) * p.Bp + b_first + c : 0;
+                cp_async16(st + KO * TI + r * BT + c, sa + off, in ? 16 : 0);
+                if (SCALED) cp_async16(st + KO * TI + KO * BT + r * BT + c, sr + off, in ? 16 : 0);
+            }
+        };
+        // the warps' sums of one stage, added in warp order and stored (first batch tile of the range) or added to memory
+        auto flush = [&](int kt) {
+            const float* src = part + (kt & 1) * (WARPS * KO * TI);
+#pragma unroll
+            for (int q = tid; q < KO * TI / 2; q += NT) {
+                const int r = q / (TI / 2), c = (q % (TI / 2)) * 2;
+                float2 v = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int k = 0; k < WARPS; ++k) {
+                    const float2 t = *reinterpret_cast<const float2*>(src + k * (KO * TI) + r * TI + c);
+                    v.x -= t.x; v.y -= t.y;
+                }
+                const int o = kt * KO + r, i = i0 + c;
+                if (o < p.COg && i < p.CIg) {
+                    float* dst = gw + (size_t)o * p.CIg + i;
+                    if (AL) {                            // CIg is a multiple of four: both columns exist and the pair is aligned
+                        if (bt == bt0) *reinterpret_cast<float2*>(dst) = v;
+                        else asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(dst), "f"(v.x), "f"(v.y) : "memory");
+                    } else {
+                        const bool two = i + 1 < p.CIg;
+                        if (bt == bt0) { dst[0] = v.x; if (two) dst[1] = v.y; }
+                        else {
+                            asm volatile("red.global.add.f32 [%0], %1;" ::"l"(dst), "f"(v.x) : "memory");
+                            if (two) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(dst + 1), "f"(v.y) : "memory");
+                        }
+                    }
+                }
+            }
+        };
+#pragma unroll
+        for (int s = 0; s < STAGES - 1; ++s) { if (kt0 + s < kt1) load(s, kt0 + s); cp_async_commit(); }
+
+        u64 xp[RW / 2][2], acc[DOX ? RW / 2 : 1][2];     // rows 2k, 2k + 1 of the warp's rows, two columns
+#pragma unroll
+        for (int k = 0; k < RW / 2; ++k)
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const int b = b_first + warp * RW + 2 * k;
+                const float* xs = p.x + (size_t)g * p.CIg + min(ic + c, p.CIg - 1);
+                xp[k][c] = pack2(__ldg(xs + (size_t)min(b, p.B - 1) * p.CI), __ldg(xs + (size_t)min(b + 1, p.B - 1) * p.CI));
+                if (DOX) acc[k][c] = 0;
+            }
+        int rd = 0, wr = STAGES - 1;
+        for (int kt = kt0; kt < kt1; ++kt) {
+            cp_async_wait<STAGES - 2>();
+            __syncthreads();
+            if (kt + STAGES - 1 < kt1) load(wr, kt + STAGES - 1);
+            cp_async_commit();
+            if (DOW && kt > kt0) flush(kt - 1);
+            const float* ws = smem + rd * STAGE + 2 * lane;
+            const float* hs = smem + rd * STAGE + KO * TI + warp * RW;
+            const float* rs = hs + KO * BT;
+            float* pt = part + ((kt & 1) * WARPS + warp) * (KO * TI) + 2 * lane;
+#pragma unroll (IP == 8 ? 2 : 1)
+            for (int o = 0; o < KO; ++o) {
+                const float2 wv = *reinterpret_cast<const float2*>(ws + o * TI);
+                const u64 w2[2] = {pack2(wv.x, wv.x), pack2(wv.y, wv.y)};
+                u64 sum[2] = {0, 0};
+#pragma unroll
+                for (int k = 0; k < RW / 2; k += 2) {
+                    const ulonglong2 hv = *reinterpret_cast<const ulonglong2*>(hs + o * BT + 2 * k);
+                    ulonglong2 rv;
+                    if (SCALED) rv = *reinterpret_cast<const ulonglong2*>(rs + o * BT + 2 * k);
+#pragma unroll
+                    for (int e = 0; e < 2; ++e)
+#pragma unroll
+                        for (int c = 0; c < 2; ++c) {
+                            u64 s = sub_f32x2(xp[k + e][c], w2[c]);
+                            if (SCALED) s = mul2(s, e ? rv.y : rv.x);
+                            const u64 f = factor2<IP>(s, p.q);
+                            if (DOX) acc[k + e][c] = fma2(e ? hv.y : hv.x, f, acc[k + e][c]);
+                            if (DOW) sum[c] = fma2(e ? hv.y : hv.x, f, sum[c]);
+                        }
+                }
+                if (DOW) {
+                    float a0, a1, b0, b1;
+                    unpack_f32x2(sum[0], a0, a1);
+                    unpack_f32x2(sum[1], b0, b1);
+                    *reinterpret_cast<float2*>(pt + o * TI) = make_float2(a0 + a1, b0 + b1);
+                }
+            }
+            rd = (rd + 1 == STAGES) ? 0 : rd + 1;
+            wr = (wr + 1 == STAGES) ? 0 : wr + 1;
+        }
+        cp_async_wait<0>();
+        __syncthreads();
+        if (DOW && kt1 > kt0) flush(kt1 - 1);
+        if (DOX) {
+            float* gx = p.gx + (size_t)ro * p.gx_step + (size_t)g * p.CIg + ic;
+#pragma unroll
+            for (int k = 0; k < RW / 2; ++k) {
+                const int b = b_first + warp * RW + 2 * k;
+                float a0, a1, b0, b1;
+                unpack_f32x2(acc[k][0], a0, a1);
+                unpack_f32x2(acc[k][1], b0, b1);
+                float* dst = gx + (size_t)b * p.CI;
+                if (AL) {
+                    if (ic < p.CIg && b < p.B) *reinterpret_cast<float2*>(dst) = make_float2(a0, b0);
+                    if (ic < p.CIg && b + 1 < p.B) *reinterpret_cast<float2*>(dst + p.CI) = make_float2(a1, b1);
+                } else {
+                    if (ic < p.CIg && b < p.B) dst[0] = a0;
+                    if (ic + 1 < p.CIg && b < p.B) dst[1] = b0;
+                    if (ic < p.CIg && b + 1 < p.B) dst[p.CI] = a1;
+                    if (ic + 1 < p.CIg && b + 1 < p.B) dst[p.CI + 1] = b1;
+                }
+            }
+        }
+    }
+}
+
+// 16 warps per SM whatever the CTA's width: 128 registers a thread
+template <int IP, int WARPS, bool DOX, bool DOW, bool AL>
+__global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
+lp_backward_both_kernel(const BothParams p) {
+    extern __shared__ __align__(16) float smem[];
+    if constexpr (IP == 8 || IP == 16) {
+        if (*p.flag == 0) { both_body<IP, WARPS, DOX, DOW, AL, false>(p, smem); return; }
+    }
+    both_body<IP, WARPS, DOX, DOW, AL, true>(p, smem);
+}
+
+// grad_output and 1 / y (0 where y is not positive) transposed to [CO][Bp] (rows past the batch: zero), and for
+// p = 8 / 16 the factor h = g / y^(p-1) with the look at the range of y.  With y in [2^-8, 2^8] (p = 8) or [2^-3, 2^4] (p = 16)
+// y^(p-1) and its reciprocal stay within 2^+-60, and a difference whose power underflows is below 2^-70 of its row's y^(p-1).
+template <int IP>
+__global__ void __launch_bounds__(256)
+lp_backward_prepare_kernel(const float* __restrict__ g, const float* __restrict__ y, int B, int Bp, int CO,
+                           float* __restrict__ gt, float* __restrict__ rt, float* __restrict__ ht, int* __restrict__ flag) {
+    __shared__ float gs[32][33], ys[32][33];
+    const int o0 = blockIdx.x * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    constexpr float LO = IP == 8 ? 0x1p-8f : 0x1p-3f, HI = IP == 8 ? 0x1p8f : 0x1p4f;
+    bool bad = false;
+    for (int b0 = blockIdx.y * 32; b0 < Bp; b0 += gridDim.y * 32) {
+#pragma unroll
+        for (int k = 0; k < 32; k += 8) {
+            const int b = b0 + ty + k, o = o0 + tx;
+            const bool in = b < B && o < CO;
+            gs[ty + k][tx] = in ? __ldg(g + (size_t)b * CO + o) : 0.f;
+            ys[ty + k][tx] = in ? __ldg(y + (size_t)b * CO + o) : 0.f;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 32; k += 8) {
+            const int o = o0 + ty + k, b = b0 + tx;
+            if (o < CO) {
+                const float gv = gs[tx][ty + k], yv = ys[tx][ty + k];
+                const size_t a = (size_t)o * Bp + b;
+                gt[a] = gv;
+                rt[a] = yv > 0.f ? 1.f / yv : 0.f;
+                if (IP == 8 || IP == 16) {
+                    bad |= b < B && !(yv >= LO && yv <= HI);
+                    float pw = yv, sq = yv;                   // y^(2^k - 1): 7 or 15
+#pragma unroll
+                    for (int n = 2; n < IP; n *= 2) { sq *= sq; pw *= sq; }
+                    ht[a] = b < B ? gv / pw : 0.f;
+                }
+            }
+        }
+        __syncthreads();
+    }
+    if ((IP == 8 || IP == 16) && __syncthreads_or(bad) && threadIdx.x == 0) atomicOr(flag, 1);
+}
+
+// out = part[0] + part[1] + ... in that order
+__global__ void __launch_bounds__(256)
+lp_backward_sum_kernel(const float* __restrict__ part, size_t n, int parts, size_t step, float* __restrict__ out, int vec) {
+    const size_t t0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
+    size_t done = 0;
+    if (vec) {
+        const size_t n4 = n / 4;
+        for (size_t e = t0; e < n4; e += stride) {
+            float4 s = __ldcs(reinterpret_cast<const float4*>(part) + e);
+            for (int k = 1; k < parts; ++k) {
+                const float4 v = __ldcs(reinterpret_cast<const float4*>(part + k * step) + e);
+                s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+            }
+            reinterpret_cast<float4*>(out)[e] = s;
+        }
+        done = n4 * 4;
+    }
+    for (size_t e = done + t0; e < n; e += stride) {
+        float s = __ldcs(part + e);
+        for (int k = 1; k < parts; ++k) s += __ldcs(part + k * step + e);
+        out[e] = s;
+    }
+}
+
+size_t up64(size_t n) { return (n + 63) & ~(size_t)63; }
+
+struct BothPlan {
+    int warps, Bp, tiles_i, n_o, n_b;
+    size_t gx_step, gw_step;          // floats of one partial result
+    size_t words;                     // floats of workspace in all
+};
+
+// Rows per CTA: 128 where that pads the batch little more than the narrower tiles do (a wider CTA reads every weight fewer
+// times and adds to gw in memory fewer times).  Ranges: the pair (n_o, n_b) with the smallest estimate of waves of CTAs
+// times the work of one, plus the traffic of the partial results (at most 1.5 GB of it).
+BothPlan plan_both(const Dims& d, float p, bool dox, bool dow) {
+    BothPlan pl{};
+    auto pad = [&](int t) { return (d.R + t - 1) / t * t; };
+    pl.warps = d.R <= 32 ? 2 : (long long)pad(128) * 10 <= (long long)pad(64) * 11 ? 8 : 4;
+    const int bt = pl.warps * RW;
+    pl.Bp = pad(bt);
+    pl.tiles_i = (d.CIg + TI - 1) / TI;
+    const int KT = (d.COg + KO - 1) / KO, BTs = pl.Bp / bt;
+    const int per_sm = 16 / pl.warps, sms = sm_count();
+    const double base = (double)pl.tiles_i * d.G;
+    // microseconds of one stage of one batch tile on an SM that holds per_sm CTAs
+    const double stage_us = (double)KO * bt * TI * per_sm * ((p == 8.f ? 7.0 : 9.0) + 2.0) / 128.0 / 1900.0;
+    double best = 1e300;
+    pl.n_o = pl.n_b = 1;
+    for (int n_b = 1; n_b <= BTs && n_b <= 32; ++n_b)
+        for (int n_o = 1; n_o <= KT && n_o <= 64; ++n_o) {
+            if (n_b > 1 && n_o * 8 < KT && n_o < 8) continue;      // partial gw is the larger tensor: split the outputs first
+            const double units = base * n_o * n_b;
+            const double slots = (double)per_sm * sms;
+            const double full = floor(units / slots), rest = units - full * slots;
+            const double waves = full + (rest > 0 ? 0.3 + 0.7 * ceil(rest / sms) / per_sm : 0.0);
+            const double work = (double)((KT + n_o - 1) / n_o) * ((BTs + n_b - 1) / n_b) + 2.0;
+            double bytes = 0;
+            if (dox && n_o > 1) bytes += 4.0 * (2 * n_o + 1) * d.R * d.CI;
+            if (dow && n_b > 1) bytes += 4.0 * (2 * n_b + 1) * d.CO * d.CIg;
+            if (bytes > 1.5e9) continue;
+            const double us = waves * work * stage_us + bytes / 4e6 + (dox && n_o > 1 ? 3.0 : 0.0) + (dow && n_b > 1 ? 3.0 : 0.0);
+            if (us < best) { best = us; pl.n_o = n_o; pl.n_b = n_b; }
+        }
+    pl.gx_step = up64((size_t)d.R * d.CI);
+    pl.gw_step = up64((size_t)d.CO * d.CIg);
+    pl.words = 64 + 3 * up64((size_t)d.CO * pl.Bp) + (dox && pl.n_o > 1 ? pl.n_o * pl.gx_step : 0) +
+               (dow && pl.n_b > 1 ? pl.n_b * pl.gw_step : 0);
+    return pl;
+}
+
+template <int IP, int WARPS, bool DOX, bool DOW, bool AL>
+int launch_both(const BothParams& P, int grid, cudaStream_t st) {
+    constexpr int bytes = (STAGES * stage_floats<WARPS, true>() + (DOW ? 2 * WARPS * KO * TI : 0)) * 4;
+    auto kern = lp_backward_both_kernel<IP, WARPS, DOX, DOW, AL>;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return LINF_ERR_LAUNCH;
+    kern<<<grid, WARPS * 32, bytes, st>>>(P);
+    return launch_status();
+}
+
+template <int IP, int WARPS, bool AL>
+int launch_which(const BothParams& P, int grid, bool dox, bool dow, cudaStream_t st) {
+    if (dox && dow) return launch_both<IP, WARPS, true, true, AL>(P, grid, st);
+    if (dox) return launch_both<IP, WARPS, true, false, AL>(P, grid, st);
+    return launch_both<IP, WARPS, false, true, AL>(P, grid, st);
+}
+
+template <int IP>
+int launch_ip(const BothParams& P, int grid, int warps, bool al, bool dox, bool dow, cudaStream_t st) {
+    if (warps == 8) return al ? launch_which<IP, 8, true>(P, grid, dox, dow, st) : launch_which<IP, 8, false>(P, grid, dox, dow, st);
+    if (warps == 4) return al ? launch_which<IP, 4, true>(P, grid, dox, dow, st) : launch_which<IP, 4, false>(P, grid, dox, dow, st);
+    return al ? launch_which<IP, 2, true>(P, grid, dox, dow, st) : launch_which<IP, 2, false>(P, grid, dox, dow, st);
+}
+
+}  // namespace
+
+// Which calls take this path: dense layers with at least 32 channels per group on both sides and 2 <= p < 1026
+// (below 2 the power s * |s|^(p-2) has no integer part to start from).
+static bool both_ok(const Dims& d, float p) {
+    return d.HW == 1 && d.COg >= 32 && d.CIg >= 32 && p >= 2.f && p < 1026.f;
+}
+
+size_t lp_backward_both_workspace(const Dims& d, float p, bool dox, bool dow) {
+    if (!both_ok(d, p) || !(dox || dow)) return 0;
+    return plan_both(d, p, dox, dow).words * sizeof(float);
+}
+
+int lp_backward_both(const float* g, const float* x, const float* w, const float* y, const Dims& d,
+                     float* gx, float* gw, float p, void* ws, size_t ws_bytes, cudaStream_t st) {
+    const bool dox = gx != nullptr, dow = gw != nullptr;
+    const size_t need = lp_backward_both_workspace(d, p, dox, dow);
+    if (need == 0 || ws == nullptr) {        // another path, one gradient at a time
+        if (dox) { const int rc = lp_backward_input(g, x, w, y, d, gx, p, st); if (rc) return rc; }
+        return dow ? lp_backward_weight(g, x, w, y, d, gw, p, st) : LINF_OK;
+    }
+    if (ws_bytes < need || (reinterpret_cast<uintptr_t>(ws) & 255u)) return LINF_ERR_WORKSPACE;
+    const BothPlan pl = plan_both(d, p, dox, dow);
+    const size_t act = up64((size_t)d.CO * pl.Bp);
+    float* base = reinterpret_cast<float*>(ws);
+    int* flag = reinterpret_cast<int*>(base);
+    float* gt = base + 64; float* rt = gt + act; float* ht = rt + act;
+    float* next = ht + act;
+    BothParams P{};
+    P.x = x; P.w = w; P.h = ht; P.g = gt; P.r = rt; P.flag = flag;
+    P.B = d.R; P.Bp = pl.Bp; P.COg = d.COg; P.CIg = d.CIg; P.G = d.G; P.CI = d.CI;
+    P.tiles_i = pl.tiles_i; P.n_o = pl.n_o; P.n_b = pl.n_b;
+    P.gx = gx; P.gw = gw;
+    if (dox && pl.n_o > 1) { P.gx = next; P.gx_step = pl.gx_step; next += pl.n_o * pl.gx_step; }
+    if (dow && pl.n_b > 1) { P.gw = next; P.gw_step = pl.gw_step; }
+    const float e = p - 2.f, fl = floorf(e);
+    P.q.m = (int)fl; P.q.f = e - fl;
+    const long long grid = (long long)pl.tiles_i * d.G * pl.n_o * pl.n_b;
+    if (grid > 0x7fffffffLL) return LINF_ERR_DIMS;
+    const bool al = (d.CIg & 3) == 0 && aligned16(w) && (!dox || aligned16(gx)) && (!dow || aligned16(gw));
+
+    const dim3 pg((d.CO + 31) / 32, (unsigned)min((pl.Bp + 31) / 32, 64));
+    const bool plain = p == 8.f || p == 16.f;
+    if (plain && cudaMemsetAsync(flag, 0, sizeof(int), st) != cudaSuccess) return LINF_ERR_LAUNCH;
+    if (p == 8.f) lp_backward_prepare_kernel<8><<<pg, 256, 0, st>>>(g, y, d.R, pl.Bp, d.CO, gt, rt, ht, flag);
+    else if (p == 16.f) lp_backward_prepare_kernel<16><<<pg, 256, 0, st>>>(g, y, d.R, pl.Bp, d.CO, gt, rt, ht, flag);
+    else lp_backward_prepare_kernel<0><<<pg, 256, 0, st>>>(g, y, d.R, pl.Bp, d.CO, gt, rt, ht, flag);
+    int rc = launch_status();
+    if (rc) return rc;
+    if (p == 8.f) rc = launch_ip<8>(P, (int)grid, pl.warps, al, dox, dow, st);
+    else if (p == 16.f) rc = launch_ip<16>(P, (int)grid, pl.warps, al, dox, dow, st);
+    else if (P.q.m < 32) rc = launch_ip<-5>(P, (int)grid, pl.warps, al, dox, dow, st);
+    else rc = launch_ip<-10>(P, (int)grid, pl.warps, al, dox, dow, st);
+    if (rc) return rc;
+    auto add_up = [&](const float* part, size_t n, int parts, size_t step, float* out) {
+        const int blocks = (int)min((size_t)(8 * sm_count()), (n / 4 + 255) / 256 + 1);
+        lp_backward_sum_kernel<<<blocks, 256, 0, st>>>(part, n, parts, step, out, aligned16(out) ? 1 : 0);
+        return launch_status();
+    };
+    if (dox && pl.n_o > 1) { rc = add_up(P.gx, (size_t)d.R * d.CI, pl.n_o, pl.gx_step, gx); if (rc) return rc; }
+    if (dow && pl.n_b > 1) { rc = add_up(P.gw, (size_t)d.CO * d.CIg, pl.n_b, pl.gw_step, gw); if (rc) return rc; }
+    return LINF_OK;
+}
+
+}  // namespace linf

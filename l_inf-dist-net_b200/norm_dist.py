@@ -162,18 +162,16 @@ class DistF(torch.autograd.Function):
             else:
                 x, weight, y = ctx.saved_tensors
                 B, CO, CI, G, HW = _shape5(x, weight, ctx.group)
-                if need_x:
-                    gx = torch.empty_like(x)
-                    rc = lib.linf_norm_dist_backward_input(
-                        grad_output.data_ptr(), x.data_ptr(), weight.data_ptr(), y.data_ptr(),
-                        B, CO, CI, G, HW, gx.data_ptr(), float(ctx.p), _stream())
-                    _lib.check(rc, "norm_dist_backward_input")
-                if need_w:
-                    gw = torch.empty_like(weight)
-                    rc = lib.linf_norm_dist_backward_weight(
-                        grad_output.data_ptr(), x.data_ptr(), weight.data_ptr(), y.data_ptr(),
-                        B, CO, CI, G, HW, gw.data_ptr(), float(ctx.p), _stream())
-                    _lib.check(rc, "norm_dist_backward_weight")
+                gx = torch.empty_like(x) if need_x else None
+                gw = torch.empty_like(weight) if need_w else None
+                if need_x or need_w:
+                    need = lib.linf_norm_dist_backward_workspace_bytes(B, CO, CI, G, HW, float(ctx.p), need_x, need_w)
+                    ws = torch.empty(need, dtype=torch.uint8, device=x.device) if need else None
+                    rc = lib.linf_norm_dist_backward(
+                        grad_output.data_ptr(), x.data_ptr(), weight.data_ptr(), y.data_ptr(), B, CO, CI, G, HW,
+                        gx.data_ptr() if need_x else None, gw.data_ptr() if need_w else None, float(ctx.p),
+                        ws.data_ptr() if need else None, need, _stream())
+                    _lib.check(rc, "norm_dist_backward")
         if ctx.rows and gx is not None:
             gx = _from_rows(gx, *ctx.shape)
         return gx, gw, None, None, None

@@ -1,0 +1,78 @@
+"""Finite-p kernels of dense layers at the sizes where they can go wrong (edges of tiles and of the packed rows, sizes that are
+multiples of nothing, groups, the smallest and the largest p), against the same sums in double precision."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def reference(x, w, g, G, p):
+    B, CI = x.shape
+    CO, cig = w.shape
+    cog = CO // G
+    x, w, g = x.double(), w.double(), g.double()
+    y = torch.empty(B, CO, dtype=torch.float64, device=x.device)
+    gx = torch.zeros(B, CI, dtype=torch.float64, device=x.device)
+    gw = torch.zeros(CO, cig, dtype=torch.float64, device=x.device)
+    for k in range(G):
+        rows, cols = slice(k * cog, (k + 1) * cog), slice(k * cig, (k + 1) * cig)
+        t = x[:, cols][:, None, :] - w[None, rows]
+        M = t.abs().amax(-1, keepdim=True).clamp_min(1e-300)
+        yk = M[..., 0] * ((t.abs() / M) ** p).sum(-1) ** (1 / p)
+        f = g[:, rows, None] * (t.abs() / yk[..., None].clamp_min(1e-300)) ** (p - 1) * t.sign()
+        y[:, rows], gx[:, cols], gw[rows] = yk, f.sum(1), -f.sum(0)
+    return y, gx, gw
+
+
+def norm_error(a, b):
+    return float((a.double() - b).norm() / b.norm())
+
+
+def check(L, x, w, g, G, p):
+    """A term's rounding (a few units of 2^-24) is raised to the power p: 2^-22 + p * 2^-23 in the 2-norm."""
+    x, w = x.clone().requires_grad_(), w.clone().requires_grad_()
+    y = L.norm_dist(x, w, G, p)
+    gx, gw = torch.autograd.grad(y, [x, w], g)
+    ref = reference(x.detach()[:, :, 0], w.detach(), g[:, :, 0], G, p)
+    limit = 2.0 ** -22 * 4 + p * 2.0 ** -23
+    for name, a, b in zip(("y", "grad_input", "grad_weight"), (y.detach()[:, :, 0], gx[:, :, 0], gw), ref):
+        assert norm_error(a, b) <= limit, (name, norm_error(a, b), limit)
+    return y.detach(), gx, gw
+
+
+@pytest.mark.parametrize("p", [2.0, 2.5, 8.0, 16.0, 23.7, 40.0, 64.0, 97.3, 1000.0])
+@pytest.mark.parametrize("B,CI,CO,G", [(33, 33, 33, 1), (8, 64, 32, 1), (70, 96, 130, 2), (130, 68, 36, 1), (203, 207, 101, 1), (1030, 64, 64, 1)])
+def test_dense_gradients(cuda, lib, B, CI, CO, G, p):
+    import linfdist_b200 as L
+    torch.manual_seed(B)
+    x, w, g = (torch.randn(*s, device="cuda") for s in ((B, CI, 1), (CO, CI // G), (B, CO, 1)))
+    y, gx, gw = check(L, x, w, g, G, p)
+    # one gradient alone: the same numbers to the rounding of another summation order
+    for need in (0, 1):
+        t = [x.clone(), w.clone()]
+        t[need].requires_grad_()
+        one, = torch.autograd.grad(L.norm_dist(t[0], t[1], G, p), t[need], g)
+        both = (gx, gw)[need]
+        assert torch.linalg.norm(one - both) <= 1e-5 * torch.linalg.norm(both)
+
+
+@pytest.mark.parametrize("p", [8.0, 16.0, 23.7, 64.0])
+@pytest.mark.parametrize("scale", [1e-6, 1e6])
+def test_dense_far_from_one(cuda, lib, p, scale):
+    """Differences whose p-th power leaves the range of a float."""
+    import linfdist_b200 as L
+    torch.manual_seed(1)
+    x, w, g = (torch.randn(*s, device="cuda") for s in ((130, 100, 1), (65, 100), (130, 65, 1)))
+    check(L, x * scale, w * scale, g, 1, p)
+
+
+@pytest.mark.parametrize("p", [8.0, 16.0])
+def test_dense_large_common_offset(cuda, lib, p):
+    """Inputs and weights far from zero with small differences: neither the rows past the batch nor the outputs past the
+    group, which exist only to fill a tile, may bring in the power of a lone large number."""
+    import linfdist_b200 as L
+    torch.manual_seed(2)
+    x, w, g = (torch.randint(-4, 5, s, device="cuda").float() for s in ((33, 36, 1), (33, 36), (33, 33, 1)))
+    x, w = x + 2.0 ** 20, w + 2.0 ** 20
+    x[:, 0] += 1
+    check(L, x, w, g, 1, p)
