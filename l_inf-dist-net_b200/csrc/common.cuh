@@ -164,9 +164,12 @@ int inf_forward_skinny(const float* x, const float* w, const Dims& d, float* y, 
                        const Post& post);
 int inf_bound_skinny(const float* xl, const float* xu, const float* w, const Dims& d, float* yl, float* yu,
                      cudaStream_t st, const Post& post);
-// register-tiled finite-p kernels for dense, aligned layers (lp_tiled.cu)
+// finite-p forward of dense layers (lp_forward.cu); where lp_forward_wants_max(p), y holds max_i |x - w| on entry
+bool lp_forward_dense_ok(const Dims& d);
+bool lp_forward_wants_max(float p);
+int lp_forward_dense(const float* x, const float* w, const Dims& d, float* y, float p, cudaStream_t st);
+// register-tiled finite-p gradients for dense, aligned layers (lp_tiled.cu)
 bool lp_tiled_ok(const Dims& d, const void* a, const void* b, const void* c, const void* e, const void* f);
-int lp_forward_tiled(const float* x, const float* w, const Dims& d, float* y, float p, cudaStream_t st);
 int lp_backward_tiled(const float* g, const float* x, const float* w, const float* y, const Dims& d,
                       float* out, float p, bool wrt_weight, cudaStream_t st);
 int lp_forward(const float* x, const float* w, const Dims& d, float* y, float p, cudaStream_t st);

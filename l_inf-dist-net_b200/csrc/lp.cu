@@ -12,7 +12,7 @@
 // few ulp of correctly rounded arithmetic; integer p (the common test points 8, 16, 64) never
 // touches the special-function unit at all.
 //
-// Forward normalisation.  M is produced first by the inf-dist forward kernel (value-only mode)
+// Forward normalisation (dense layers: lp_forward.cu).  M is produced first by the inf-dist forward kernel (value-only mode)
 // straight into `output`; the power-sum kernel reads it from there and overwrites it with y.
 #include <math.h>
 
@@ -344,9 +344,11 @@ bool grid_ok(const dim3& g) { return g.y <= 65535u && g.z <= 65535u; }
 }  // namespace
 
 int lp_forward(const float* x, const float* w, const Dims& d, float* y, float p, cudaStream_t st) {
+    const bool dense = lp_forward_dense_ok(d);
+    if (dense && !lp_forward_wants_max(p)) return lp_forward_dense(x, w, d, y, p, st);
     int rc = inf_forward(x, w, d, y, nullptr, nullptr, 0, st);
     if (rc != LINF_OK) return rc;
-    if (lp_tiled_ok(d, x, w, y, nullptr, nullptr)) return lp_forward_tiled(x, w, d, y, p, st);
+    if (dense) return lp_forward_dense(x, w, d, y, p, st);
     if (skinny_ok(d, x, w, nullptr)) {
         if (d.COg <= 4) return launch_lp_skinny<4, 4>(x, w, d, y, p, st);
         if (d.COg <= 8) return launch_lp_skinny<8, 2>(x, w, d, y, p, st);

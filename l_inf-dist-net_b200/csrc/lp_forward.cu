@@ -1,0 +1,310 @@
+// Forward of the finite-p distance neuron on dense layers (HW == 1, at least 32 outputs and 32 inputs per group; no
+// alignment or divisibility is asked for):   y[b,o] = (sum_i |x[b,i] - w[o,i]|^p)^(1/p).
+//
+// Bound: FP32 issue for integer p, the special-function unit (one log2 per term, half an exp2) otherwise.
+//
+// A term needs a scale only so that its power stays within the range of a float, and any scale does: the sum is divided
+// by the same factor in the end.  So the maximum max_i |x - w|, which costs a pass of its own over all terms, is
+// not needed:
+//   p = 8, 16          no scale at all.  Sums in [2^-64, 2^120] are kept: nothing overflowed, and a
+//                      difference whose power underflows is below 2^-60 of the sum.
+//   other p <= 80      one scale per output, from the largest of its first 32 (p > 32: 64) differences times 1.5, which is about where the
+//                      maximum of a long row lies (the closer to it, the smaller the exponents and their rounding).  Kept by the same rule:
+//                      the maximum of the row may be 5 times the sample's at p = 64, 4 times at 80, 20 times at 32.
+//   p > 80, or a sum outside the range (also: NaN, infinities, a row of zeros)
+//                      the literal rule: M = max_i |x - w| first, then sum (|x - w| / M)^p, y = M * sum^(1/p).  p > 80 gets M
+//                      from the value-only inf-dist kernel, a tile with a sum outside the range works it out itself.
+// 64 x 64 (or 64 x 48) output tile per CTA of 128 threads, 8 x 4 (8 x 3) outputs per thread, operand tiles through a ring of
+// three cp.async stages; two neighbouring terms of an output sit in one register pair, so subtraction,
+// scale and squarings are packed (f32x2).
+//
+// Per term: p = 8: subtraction, two squarings, one multiply-add = 4 lane operations (literal rule: 6, and the maximum pass).
+// Run-time p: half of the exp2 run as a polynomial on the FP32 pipe (4 lg2 + 2 ex2 of the special-function unit for 4 terms =
+// 12 cycles per term and scheduler; all on the unit: 16).
+// Measured on one B200, us, maximum pass + literal rule -> here: B = 512, Din = Dout = 5120: p = 8: 3069 -> 1870,
+// 16: 3466 -> 2254, 64: 4230 -> 3468, 23.7: 7129 -> 5279; B = 203, Din = 1027, Dout = 1333 (generic kernels before), p = 8: 683 -> 117.
+#include <math.h>
+
+#include "common.cuh"
+
+namespace linf {
+namespace {
+
+typedef unsigned long long u64;
+
+__device__ __forceinline__ u64 mul2(u64 a, u64 b) { u64 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ u64 add2(u64 a, u64 b) { u64 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) { u64 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+__device__ __forceinline__ u64 pack2(float a, float b) { u64 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ float lg2_approx(float a) { float r; asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a)); return r; }
+__device__ __forceinline__ float ex2_approx(float a) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a)); return r; }
+
+// 2^e for a pair on the FP32 pipe: e = n + f with the nearest integer n (the usual addition of 1.5 * 2^23), 2^f by the degree-5
+// interpolation of 2^f at the Chebyshev nodes of [-1/2, 1/2] (relative error in fp32 at most 2.2e-7, as ex2.approx), n added to the
+// exponent.  e is held within [-125, 127] (a NaN stays one): below, the term is lost against a sum of at least 2^-64; above, the sum
+// ends outside the accepted range.
+__device__ __forceinline__ float clamp_exp(float e) {
+    float r;
+    asm("max.NaN.f32 %0, %1, 0fC2FA0000;" : "=f"(r) : "f"(e));      // -125
+    asm("min.NaN.f32 %0, %1, 0f42FE0000;" : "=f"(r) : "f"(r));      // 127
+    return r;
+}
+__device__ __forceinline__ u64 ex2_poly2(u64 e) {
+    float e0, e1;
+    unpack_f32x2(e, e0, e1);
+    const u64 c = pack2(clamp_exp(e0), clamp_exp(e1));
+    const u64 z = add2(c, pack2(12582912.f, 12582912.f));
+    const u64 f = sub_f32x2(c, sub_f32x2(z, pack2(12582912.f, 12582912.f)));
+    u64 r = pack2(1.339086331e-03f, 1.339086331e-03f);
+    r = fma2(r, f, pack2(9.676031768e-03f, 9.676031768e-03f));
+    r = fma2(r, f, pack2(5.550356954e-02f, 5.550356954e-02f));
+    r = fma2(r, f, pack2(2.402210683e-01f, 2.402210683e-01f));
+    r = fma2(r, f, pack2(6.931471825e-01f, 6.931471825e-01f));
+    r = fma2(r, f, pack2(1.000000119e+00f, 1.000000119e+00f));
+    float r0, r1, z0, z1;
+    unpack_f32x2(r, r0, r1);
+    unpack_f32x2(z, z0, z1);
+    // A NaN ends as the canonical NaN 0x7fffffff in r and z; the addition below then gives 0x7f7fffff, the largest float,
+    // and the sum leaves the accepted range: the literal rule answers.
+    const float s0 = __int_as_float(__float_as_int(r0) + (__float_as_int(z0) << 23));
+    const float s1 = __int_as_float(__float_as_int(r1) + (__float_as_int(z1) << 23));
+    return pack2(s0, s1);
+}
+
+// a^E of a pair, E a power of two
+template <int E>
+__device__ __forceinline__ u64 pow2_ct(u64 a) {
+    if constexpr (E == 1) return a;
+    else { const u64 h = pow2_ct<E / 2>(a); return mul2(h, h); }
+}
+template <int E>
+__device__ __forceinline__ float pow_ct(float a) {
+    if constexpr (E == 1) return a;
+    else { const float h = pow_ct<E / 2>(a); return h * h; }
+}
+
+constexpr int TM = 64, NT = 128, BK = 16, LDK = BK + 4, STAGES = 3;
+constexpr float kSumLow = 0x1p-64f, kSumHigh = 0x1p120f;
+constexpr float kSampledP = 80.f;
+constexpr float kLower = 2.f / 3.f;
+
+struct FwdParams {
+    const float* x; const float* w; float* y;
+    int B, COg, CIg, G, CI, CO;
+    float p, inv_p;
+    int sample;                 // k-tiles the scale is taken from
+    int have_max;               // y holds max_i |x - w|
+};
+
+template <int ROWS, bool AL>
+__device__ __forceinline__ void load_rows(float* dst, const float* __restrict__ src, size_t ld, int row0, int rows, int k0, int cols, int tid) {
+    if (AL) {
+#pragma unroll
+        for (int q = tid; q < ROWS * (BK / 4); q += NT) {
+            const int r = q / (BK / 4), c = (q % (BK / 4)) * 4;
+            const bool in = row0 + r < rows && k0 + c < cols;
+            cp_async16(dst + r * LDK + c, src + (in ? (size_t)(row0 + r) * ld + k0 + c : 0), in ? 16 : 0);
+        }
+    } else {
+#pragma unroll 2                      // unrolled fully, the copies' addresses alone exhaust the registers
+        for (int q = tid; q < ROWS * BK; q += NT) {
+            const int r = q / BK, c = q % BK;
+            const bool in = row0 + r < rows && k0 + c < cols;
+            cp_async4(dst + r * LDK + c, src + (in ? (size_t)(row0 + r) * ld + k0 + c : 0), in ? 4 : 0);
+        }
+    }
+}
+
+// IP: 8, 16, 64 at compile time (8 and 16 without a scale), 0: p at run time.  TJ: output columns per thread.
+template <int IP, int TJ, bool AL>
+__global__ void __launch_bounds__(NT, 3)
+lp_forward_kernel(const FwdParams p) {
+    extern __shared__ __align__(16) float smem[];
+    constexpr int TN = 16 * TJ, NO = 8 * TJ, STAGE = (TM + TN) * LDK;
+    constexpr bool PLAIN = IP == 8 || IP == 16;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int wm = warp & 1, wn = warp >> 1, lm = lane >> 3, ln = lane & 7;
+    const int row_off = wm * 32 + lm, col_off = wn * (8 * TJ) + ln;       // + 4i rows, + 8j columns
+    const int tiles_m = (p.B + TM - 1) / TM, tiles_n = (p.COg + TN - 1) / TN;
+    const int g = blockIdx.x / (tiles_m * tiles_n), tg = blockIdx.x % (tiles_m * tiles_n);
+    const int n0 = (tg / tiles_m) * TN, m0 = (tg % tiles_m) * TM;
+    const float* xg = p.x + (size_t)g * p.CIg;
+    const float* wg = p.w + (size_t)g * p.COg * p.CIg;
+    const int KT = (p.CIg + BK - 1) / BK;
+
+    // runs body(e, t01, t23) over the differences of the first n_tiles k-tiles, four terms of an output at a time
+    auto sweep = [&](int n_tiles, auto&& body) {
+        auto load = [&](int s, int kt) {
+            float* st = smem + s * STAGE;
+            load_rows<TM, AL>(st, xg, p.CI, m0, p.B, kt * BK, p.CIg, tid);
+            load_rows<TN, AL>(st + TM * LDK, wg, p.CIg, n0, p.COg, kt * BK, p.CIg, tid);
+        };
+        __syncthreads();
+#pragma unroll
+        for (int s = 0; s < STAGES - 1; ++s) { if (s < n_tiles) load(s, s); cp_async_commit(); }
+        int rd = 0, wr = STAGES - 1;
+        for (int kt = 0; kt < n_tiles; ++kt) {
+            cp_async_wait<STAGES - 2>();
+            __syncthreads();
+            if (kt + STAGES - 1 < n_tiles) load(wr, kt + STAGES - 1);
+            cp_async_commit();
+            const float* As = smem + rd * STAGE + row_off * LDK;
+            const float* Bs = smem + rd * STAGE + (TM + col_off) * LDK;
+            // two of the four k4 steps per trip (one where a term is long): the fully unrolled body runs into instruction fetch stalls
+#pragma unroll (IP == 8 ? 2 : 1)
+            for (int k4 = 0; k4 < BK / 4; ++k4) {
+                ulonglong2 bf[TJ];
+#pragma unroll
+                for (int j = 0; j < TJ; ++j) bf[j] = *reinterpret_cast<const ulonglong2*>(Bs + (8 * j) * LDK + k4 * 4);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const ulonglong2 af = *reinterpret_cast<const ulonglong2*>(As + (4 * i) * LDK + k4 * 4);
+#pragma unroll
+                    for (int j = 0; j < TJ; ++j) body(i * TJ + j, sub_f32x2(af.x, bf[j].x), sub_f32x2(af.y, bf[j].y));
+                }
+            }
+            rd = (rd + 1 == STAGES) ? 0 : rd + 1;
+            wr = (wr + 1 == STAGES) ? 0 : wr + 1;
+        }
+        cp_async_wait<0>();
+    };
+    auto out = [&](int e) { return p.y + (size_t)(m0 + row_off + 4 * (e / TJ)) * p.CO + (size_t)g * p.COg + n0 + col_off + 8 * (e % TJ); };
+    auto inside = [&](int e) { return m0 + row_off + 4 * (e / TJ) < p.B && n0 + col_off + 8 * (e % TJ) < p.COg; };
+
+    float S[NO];
+    if (!p.have_max) {
+        [[maybe_unused]] float r[PLAIN ? 1 : NO];
+#pragma unroll
+        for (int e = 0; e < NO; ++e) S[e] = 0.f;
+        if constexpr (PLAIN) {
+            sweep(KT, [&](int e, u64 t01, u64 t23) {
+                float a, b;
+                unpack_f32x2(pow2_ct<IP / 2>(t01), a, b);
+                S[e] = fmaf(a, a, S[e]); S[e] = fmaf(b, b, S[e]);
+                unpack_f32x2(pow2_ct<IP / 2>(t23), a, b);
+                S[e] = fmaf(a, a, S[e]); S[e] = fmaf(b, b, S[e]);
+            });
+        } else {
+            sweep(min(KT, p.sample), [&](int e, u64 t01, u64 t23) {
+                float a, b, c, d;
+                unpack_f32x2(t01, a, b); unpack_f32x2(t23, c, d);
+                S[e] = max3(max3(S[e], fabsf(a), fabsf(b)), fabsf(c), fabsf(d));
+            });
+#pragma unroll
+            for (int e = 0; e < NO; ++e) { r[e] = S[e] > 0.f ? kLower / S[e] : 0.f; S[e] = 0.f; }
+            const u64 pp = pack2(p.p, p.p);
+            sweep(KT, [&](int e, u64 t01, u64 t23) {
+                const u64 rr = pack2(r[e], r[e]);
+                const u64 u01 = mul2(t01, rr), u23 = mul2(t23, rr);
+                float a, b;
+                if constexpr (IP > 0) {
+                    unpack_f32x2(pow2_ct<IP / 2>(u01), a, b);
+                    S[e] = fmaf(a, a, S[e]); S[e] = fmaf(b, b, S[e]);
+                    unpack_f32x2(pow2_ct<IP / 2>(u23), a, b);
+                    S[e] = fmaf(a, a, S[e]); S[e] = fmaf(b, b, S[e]);
+                } else {
+                    unpack_f32x2(u01, a, b);
+                    const u64 e01 = mul2(pack2(lg2_approx(fabsf(a)), lg2_approx(fabsf(b))), pp);
+                    unpack_f32x2(u23, a, b);
+                    const u64 e23 = mul2(pack2(lg2_approx(fabsf(a)), lg2_approx(fabsf(b))), pp);
+                    unpack_f32x2(e01, a, b);
+                    S[e] += ex2_approx(a); S[e] += ex2_approx(b);
+                    unpack_f32x2(ex2_poly2(e23), a, b);
+                    S[e] += a; S[e] += b;
+                }
+            });
+        }
+        bool bad = false;
+#pragma unroll
+        for (int e = 0; e < NO; ++e) bad |= inside(e) && !(S[e] >= kSumLow && S[e] <= kSumHigh);
+        if (!__syncthreads_or(bad)) {
+#pragma unroll
+            for (int e = 0; e < NO; ++e)
+                if (inside(e)) *out(e) = PLAIN ? powf(S[e], p.inv_p) : powf(S[e], p.inv_p) / r[PLAIN ? 0 : e];
+            return;
+        }
+        // the maximum of every output, left in y for the literal rule (each thread reads back what it wrote)
+#pragma unroll
+        for (int e = 0; e < NO; ++e) S[e] = 0.f;
+        sweep(KT, [&](int e, u64 t01, u64 t23) {
+            float a, b, c, d;
+            unpack_f32x2(t01, a, b); unpack_f32x2(t23, c, d);
+            S[e] = max3(max3(S[e], fabsf(a), fabsf(b)), fabsf(c), fabsf(d));
+        });
+#pragma unroll
+        for (int e = 0; e < NO; ++e) if (inside(e)) *out(e) = S[e];
+    }
+    float rM[NO];
+#pragma unroll
+    for (int e = 0; e < NO; ++e) {
+        const float M = inside(e) ? *out(e) : 0.f;
+        rM[e] = M > 0.f ? 1.f / M : 0.f;
+        S[e] = 0.f;
+    }
+    sweep(KT, [&](int e, u64 t01, u64 t23) {
+        float t[4];
+        unpack_f32x2(t01, t[0], t[1]); unpack_f32x2(t23, t[2], t[3]);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const float u = fabsf(t[q]) * rM[e];
+            if constexpr (IP > 0) { const float h = pow_ct<IP / 2>(u); S[e] = fmaf(h, h, S[e]); }
+            else S[e] += ex2_approx(p.p * lg2_approx(u));
+        }
+    });
+#pragma unroll
+    for (int e = 0; e < NO; ++e)
+        if (inside(e)) {
+            float* yo = out(e);
+            const float M = *yo;
+            *yo = M > 0.f ? powf(S[e], p.inv_p) * M : 0.f;
+        }
+}
+
+template <int IP, int TJ, bool AL>
+int launch_fwd(const FwdParams& P, int grid, cudaStream_t st) {
+    constexpr int bytes = STAGES * (TM + 16 * TJ) * LDK * 4;
+    auto kern = lp_forward_kernel<IP, TJ, AL>;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return LINF_ERR_LAUNCH;
+    kern<<<grid, NT, bytes, st>>>(P);
+    return launch_status();
+}
+template <int IP>
+int launch_fwd_ip(const FwdParams& P, int grid, bool narrow, bool al, cudaStream_t st) {
+    if (narrow) return al ? launch_fwd<IP, 3, true>(P, grid, st) : launch_fwd<IP, 3, false>(P, grid, st);
+    return al ? launch_fwd<IP, 4, true>(P, grid, st) : launch_fwd<IP, 4, false>(P, grid, st);
+}
+
+}  // namespace
+
+bool lp_forward_dense_ok(const Dims& d) { return d.HW == 1 && d.COg >= 32 && d.CIg >= 32; }
+bool lp_forward_wants_max(float p) { return p > kSampledP; }
+
+int lp_forward_width = 0;   // 0: tile width by shape; 1: 64 columns; 2: 48 columns (benchmarking knob)
+
+int lp_forward_dense(const float* x, const float* w, const Dims& d, float* y, float p, cudaStream_t st) {
+    // The kernel is bound by throughput: an SM of the last, partial wave takes a third of a full wave per CTA it
+    // holds.  48-wide tiles cost 3/4 of 64-wide ones and are taken when that buys a shorter launch
+    // (B = 512, Dout = 5120: 640 tiles on 444 slots = 1 + 2/3 waves, against 856 tiles = 2 x 3/4).
+    const int tiles_m = (d.R + TM - 1) / TM, slots = 3 * sm_count(), sms = sm_count();
+    auto count = [&](int tn) { return (long long)tiles_m * ((d.COg + tn - 1) / tn) * d.G; };
+    auto cost = [&](int tn) {
+        const long long tiles = count(tn), rest = tiles % slots;
+        return (tn / 64.0) * ((tiles / slots) + ((rest + sms - 1) / sms) / 3.0);
+    };
+    const bool narrow = lp_forward_width == 2 || (lp_forward_width == 0 && d.COg >= 48 && cost(48) < 0.97 * cost(64));
+    const long long grid = count(narrow ? 48 : 64);
+    if (grid > 0x7fffffffLL) return LINF_ERR_DIMS;
+    FwdParams P;
+    P.x = x; P.w = w; P.y = y;
+    P.B = d.R; P.COg = d.COg; P.CIg = d.CIg; P.G = d.G; P.CI = d.CI; P.CO = d.CO;
+    P.p = p; P.inv_p = 1.f / p;
+    P.sample = p > 32.f ? 4 : 2;
+    P.have_max = lp_forward_wants_max(p) ? 1 : 0;
+    const bool al = (d.CIg & 3) == 0 && aligned16(x) && aligned16(w);
+    if (p == 8.f) return launch_fwd_ip<8>(P, (int)grid, narrow, al, st);
+    if (p == 16.f) return launch_fwd_ip<16>(P, (int)grid, narrow, al, st);
+    if (p == 64.f) return launch_fwd_ip<64>(P, (int)grid, narrow, al, st);
+    return launch_fwd_ip<0>(P, (int)grid, narrow, al, st);
+}
+
+}  // namespace linf

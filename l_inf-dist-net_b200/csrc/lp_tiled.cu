@@ -1,10 +1,9 @@
-// Register-tiled kernels for the finite-p distance neuron on dense layers (HW == 1, channel
-// counts per group multiples of 4, 16-byte aligned tensors).  64 x 64 output tile per CTA of 128
+// Register-tiled gradients of the finite-p distance neuron on dense layers (HW == 1, channel
+// counts per group multiples of 4, 16-byte aligned tensors), one gradient per launch and no workspace: what
+// linf_norm_dist_backward_input / _weight run.  (lp_backward.cu produces both in one pass.)  64 x 64 output tile per CTA of 128
 // threads, 8 x 4 outputs per thread, operand tiles staged through shared memory with cp.async in a
 // multi-stage ring (the geometry of the inf-dist forward).
 //
-//   forward          S[b,o] = sum_i (|x[b,i] - w[o,i]| / M[b,o])^p        reduce over i
-//                    (M is read from `y`, which the caller filled with max_i |x - w|; y := M * S^(1/p))
 //   backward input   gx[b,i] = sum_o g[b,o] * s * |s|^(p-2),  s = (x[b,i] - w[o,i]) / y[b,o]   reduce over o
 //   backward weight  gw[o,i] = sum_b g[b,o] * s * |s|^(p-2),  s = (w[o,i] - x[b,i]) / y[b,o]   reduce over b
 //
@@ -58,14 +57,6 @@ __device__ __forceinline__ float pow_ct(float a) {
 // Template parameter IP of the kernels: IP > 0 is an integer p fixed at compile time; IP <= 0 takes
 // p at run time (backward: -IP = number of bits of the integer part of p - 1).
 
-// term of the forward sum: u^p, u >= 0.  The run-time path is one log2/exp2 pair: its relative
-// error of about p * 2e-7 per term shrinks by 1/p again in the final S^(1/p).
-template <int IP>
-__device__ __forceinline__ float fwd_term(float u, const Pw q, float p) {
-    if (IP > 0) return pow_ct<(IP > 0 ? IP : 1)>(u);
-    return ex2_approx(p * lg2_approx(u));
-}
-
 // backward factor s * |s|^(p-2) (q holds p - 1 for the run-time path)
 template <int IP>
 __device__ __forceinline__ float bwd_factor(float s, const Pw q) {
@@ -91,99 +82,9 @@ __device__ __forceinline__ void load_tile(float* dst, const float* __restrict__ 
 struct LpParams {
     const float* x; const float* w; const float* g; float* y; float* out;
     int B, COg, CIg, G, CI, CO;
-    Pw q; float inv_p, pf;
+    Pw q;
     int ksplit;        // backward: CTAs per output tile, each with an equal share of the reduction (1 or 2)
 };
-
-// ------------------------------------------------------------------------------------------------
-// forward: tile = 64 rows (b) x 64 outputs (o), reduce over i; x and w tiles are K-contiguous
-// ------------------------------------------------------------------------------------------------
-// TJ = output columns per thread (4: 64-wide tiles; 3: 48-wide tiles, for shapes whose 64-wide tiles
-// leave much of their last wave of CTAs idle)
-template <int IP, int TJ>
-__global__ void __launch_bounds__(NT, 3)
-lp_forward_tiled_kernel(const LpParams p) {
-    extern __shared__ __align__(16) float smem[];
-    constexpr int TNF = 16 * TJ, NO = 8 * TJ;
-    constexpr int STAGE = (TM + TNF) * LDK;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int wm = warp & 1, wn = warp >> 1, lm = lane >> 3, ln = lane & 7;
-    const int row_off = wm * 32 + lm, col_off = wn * (8 * TJ) + ln;       // + 4i rows, + 8j columns
-    const int tiles_m = (p.B + TM - 1) / TM, tiles_n = (p.COg + TNF - 1) / TNF;
-    const int g = blockIdx.x / (tiles_m * tiles_n), tg = blockIdx.x % (tiles_m * tiles_n);
-    const int n0 = (tg / tiles_m) * TNF, m0 = (tg % tiles_m) * TM;
-    const float* xg = p.x + (size_t)g * p.CIg;
-    const float* wg = p.w + (size_t)g * p.COg * p.CIg;
-    const int KT = (p.CIg + BK - 1) / BK;
-
-    float S[NO], rM[NO];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < TJ; ++j) {
-            const int m = min(m0 + row_off + 4 * i, p.B - 1), n = min(n0 + col_off + 8 * j, p.COg - 1);
-            const float M = p.y[(size_t)m * p.CO + (size_t)g * p.COg + n];
-            rM[i * TJ + j] = M > 0.f ? 1.f / M : 0.f;
-            S[i * TJ + j] = 0.f;
-        }
-    auto load = [&](int s, int kt) {
-        float* st = smem + s * STAGE;
-        load_tile<TM, BK, LDK>(st, xg, p.CI, m0, p.B, kt * BK, p.CIg, tid);
-        load_tile<TNF, BK, LDK>(st + TM * LDK, wg, p.CIg, n0, p.COg, kt * BK, p.CIg, tid);
-    };
-#pragma unroll
-    for (int s = 0; s < STAGES - 1; ++s) { if (s < KT) load(s, s); cp_async_commit(); }
-    int rd = 0, wr = STAGES - 1;
-    for (int kt = 0; kt < KT; ++kt) {
-        cp_async_wait<STAGES - 2>();
-        __syncthreads();
-        if (kt + STAGES - 1 < KT) load(wr, kt + STAGES - 1);
-        cp_async_commit();
-        const float* As = smem + rd * STAGE + row_off * LDK;
-        const float* Bs = smem + rd * STAGE + (TM + col_off) * LDK;
-        // two of the four k4 steps per loop trip: the fully unrolled body (4 x 128 power sums) ran into instruction
-        // fetch stalls (p = 64: 6.7 ms unrolled, 4.6 ms so)
-#pragma unroll 2
-        for (int k4 = 0; k4 < BK / 4; ++k4) {
-            ulonglong2 bf[TJ];
-#pragma unroll
-            for (int j = 0; j < TJ; ++j) bf[j] = *reinterpret_cast<const ulonglong2*>(Bs + (8 * j) * LDK + k4 * 4);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const ulonglong2 af = *reinterpret_cast<const ulonglong2*>(As + (4 * i) * LDK + k4 * 4);
-#pragma unroll
-                for (int j = 0; j < TJ; ++j) {
-                    float t0, t1, t2, t3;
-                    unpack_f32x2(sub_f32x2(af.x, bf[j].x), t0, t1);
-                    unpack_f32x2(sub_f32x2(af.y, bf[j].y), t2, t3);
-                    const float r = rM[i * TJ + j];
-                    float s = S[i * TJ + j];
-                    s += fwd_term<IP>(fabsf(t0) * r, p.q, p.pf);
-                    s += fwd_term<IP>(fabsf(t1) * r, p.q, p.pf);
-                    s += fwd_term<IP>(fabsf(t2) * r, p.q, p.pf);
-                    s += fwd_term<IP>(fabsf(t3) * r, p.q, p.pf);
-                    S[i * TJ + j] = s;
-                }
-            }
-        }
-        rd = (rd + 1 == STAGES) ? 0 : rd + 1;
-        wr = (wr + 1 == STAGES) ? 0 : wr + 1;
-    }
-    cp_async_wait<0>();
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int m = m0 + row_off + 4 * i;
-#pragma unroll
-        for (int j = 0; j < TJ; ++j) {
-            const int n = n0 + col_off + 8 * j;
-            if (m < p.B && n < p.COg) {
-                float* yo = p.y + (size_t)m * p.CO + (size_t)g * p.COg + n;
-                const float M = *yo;                     // still the normaliser: nobody else writes this element
-                *yo = M > 0.f ? powf(S[i * TJ + j], p.inv_p) * M : 0.f;
-            }
-        }
-    }
-}
 
 // ------------------------------------------------------------------------------------------------
 // backward: one kernel for both gradients.
@@ -361,51 +262,18 @@ bool lp_tiled_ok(const Dims& d, const void* a, const void* b, const void* c, con
 }
 
 static LpParams make_params(const float* x, const float* w, const float* g, float* y, float* out,
-                            const Dims& d, float q, float p) {
+                            const Dims& d, float q) {
     LpParams P;
     P.x = x; P.w = w; P.g = g; P.y = y; P.out = out;
     P.B = d.R; P.COg = d.COg; P.CIg = d.CIg; P.G = d.G; P.CI = d.CI; P.CO = d.CO;
-    P.q = make_pw(q); P.inv_p = 1.f / p; P.pf = p;
+    P.q = make_pw(q);
     P.ksplit = 1;
     return P;
 }
 
-int lp_forward_width = 0;   // 0: tile width by shape; 1: 64 columns; 2: 48 columns (benchmarking knob)
-
-// `y` holds max_i |x - w| on entry and the L_p distance on exit
-int lp_forward_tiled(const float* x, const float* w, const Dims& d, float* y, float p, cudaStream_t st) {
-    const LpParams P = make_params(x, w, nullptr, y, nullptr, d, p, p);
-    // The kernel is bound by FP32 throughput: an SM of the last, partial wave takes a third of a full wave per CTA
-    // it holds.  48-wide tiles cost 3/4 of 64-wide ones and are taken when that buys a shorter launch
-    // (B = 512, Dout = 5120: 640 tiles on 444 slots = 1 + 2/3 waves, against 856 tiles = 2 x 3/4).
-    const int tiles_m = (d.R + TM - 1) / TM, slots = 3 * sm_count(), sms = sm_count();
-    auto cost = [&](int tn) {
-        const int tiles = tiles_m * ((d.COg + tn - 1) / tn) * d.G, rest = tiles % slots;
-        return (tn / 64.0) * ((tiles / slots) + ((rest + sms - 1) / sms) / 3.0);
-    };
-    const bool narrow = lp_forward_width == 2 || (lp_forward_width == 0 && d.COg >= 48 && cost(48) < 0.97 * cost(64));
-    const int tn = narrow ? 48 : 64;
-    const int grid = tiles_m * ((d.COg + tn - 1) / tn) * d.G;
-    const int smem = STAGES * (TM + tn) * LDK * 4;
-#define LINF_FWD(IPV)                                                                                       \
-    { if (narrow) {                                                                                         \
-          if (set_smem(lp_forward_tiled_kernel<IPV, 3>, smem)) return LINF_ERR_LAUNCH;                      \
-          lp_forward_tiled_kernel<IPV, 3><<<grid, NT, smem, st>>>(P);                                       \
-      } else {                                                                                              \
-          if (set_smem(lp_forward_tiled_kernel<IPV, 4>, smem)) return LINF_ERR_LAUNCH;                      \
-          lp_forward_tiled_kernel<IPV, 4><<<grid, NT, smem, st>>>(P);                                       \
-      }                                                                                                     \
-      return launch_status(); }
-    if (p == 8.f) LINF_FWD(8)
-    if (p == 16.f) LINF_FWD(16)
-    if (p == 64.f) LINF_FWD(64)
-    LINF_FWD(0)
-#undef LINF_FWD
-}
-
 int lp_backward_tiled(const float* g, const float* x, const float* w, const float* y, const Dims& d,
                       float* out, float p, bool wrt_weight, cudaStream_t st) {
-    LpParams P = make_params(x, w, g, const_cast<float*>(y), out, d, p - 1.f, p);
+    LpParams P = make_params(x, w, g, const_cast<float*>(y), out, d, p - 1.f);
     const int mt = wrt_weight ? d.COg : d.R;
     int grid = ((mt + TM - 1) / TM) * ((d.CIg + TN - 1) / TN) * d.G;
     {
