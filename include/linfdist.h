@@ -257,6 +257,23 @@ int linf_norm_dist_backward(const float* grad_output, const float* input,
                             float* grad_input, float* grad_weight, float p,
                             void* workspace, size_t workspace_bytes, void* stream);
 
+/*
+ * The p = inf forward (pos may be NULL: value only) and bounds, with the per-channel epilogue of the _post entry points, by
+ * looking only at the large entries of either side where the data allow it; the results are those of the full scan, bit for bit.
+ * The workspace (256-byte aligned, contents irrelevant, free again when the call's work on the stream is done)
+ * has the size the query answers for the same sizes; 0, or a NULL workspace, means the full scan.
+ */
+size_t linf_inf_dist_forward_pruned_workspace_bytes(int B, int CO, int CI, int G, int HW);
+int linf_inf_dist_forward_pruned(const float* input, const float* weight, int B, int CO, int CI, int G, int HW,
+                                 const float* sub, const float* add, int negate, float* output, int* pos,
+                                 void* workspace, size_t workspace_bytes, void* stream);
+size_t linf_inf_dist_bound_pruned_workspace_bytes(int B, int CO, int CI, int G, int HW);
+int linf_inf_dist_bound_pruned(const float* input_lower, const float* input_upper, const float* weight,
+                               int B, int CO, int CI, int G, int HW,
+                               const float* sub, const float* add, int negate,
+                               float* output_lower, float* output_upper,
+                               void* workspace, size_t workspace_bytes, void* stream);
+
 /* ---------------------------------------------------------------------------------
  * optimiser step (next to the distance neuron on the training path)
  * --------------------------------------------------------------------------------- */

@@ -311,4 +311,39 @@ int linf_norm_dist_backward(const float* grad_output, const float* input, const 
                             as_stream(stream));
 }
 
+size_t linf_inf_dist_forward_pruned_workspace_bytes(int B, int CO, int CI, int G, int HW) {
+    Dims d;
+    if (make_dims(B, CO, CI, G, HW, &d)) return 0;
+    return inf_forward_pruned_workspace(d);
+}
+
+int linf_inf_dist_forward_pruned(const float* input, const float* weight, int B, int CO, int CI, int G, int HW,
+                                 const float* sub, const float* add, int negate, float* output, int* pos,
+                                 void* workspace, size_t workspace_bytes, void* stream) {
+    if (!input || !weight || !output) return LINF_ERR_NULL;
+    Dims d;
+    int rc = make_dims(B, CO, CI, G, HW, &d);
+    if (rc) return rc;
+    const Post post{sub, add, negate ? 1 : 0};
+    return inf_forward_pruned(input, weight, d, output, pos, workspace, workspace_bytes, as_stream(stream), post);
+}
+
+size_t linf_inf_dist_bound_pruned_workspace_bytes(int B, int CO, int CI, int G, int HW) {
+    Dims d;
+    if (make_dims(B, CO, CI, G, HW, &d)) return 0;
+    return inf_bound_pruned_workspace(d);
+}
+
+int linf_inf_dist_bound_pruned(const float* input_lower, const float* input_upper, const float* weight,
+                               int B, int CO, int CI, int G, int HW, const float* sub, const float* add, int negate,
+                               float* output_lower, float* output_upper, void* workspace, size_t workspace_bytes, void* stream) {
+    if (!input_lower || !input_upper || !weight || !output_lower || !output_upper) return LINF_ERR_NULL;
+    Dims d;
+    int rc = make_dims(B, CO, CI, G, HW, &d);
+    if (rc) return rc;
+    const Post post{sub, add, negate ? 1 : 0};
+    return inf_bound_pruned(input_lower, input_upper, weight, d, output_lower, output_upper, workspace, workspace_bytes,
+                            as_stream(stream), post);
+}
+
 }  // extern "C"

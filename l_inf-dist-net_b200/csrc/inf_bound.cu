@@ -40,7 +40,8 @@ template <bool ROW_FAST>
 __global__ void __launch_bounds__(256)
 inf_bound_generic_kernel(const float* __restrict__ xl, const float* __restrict__ xu,
                          const float* __restrict__ w, Dims d,
-                         float* __restrict__ yl, float* __restrict__ yu, Post post) {
+                         float* __restrict__ yl, float* __restrict__ yu, Post post, const int* __restrict__ only_if) {
+    if (only_if != nullptr && *only_if == 0) return;
     __shared__ float ls[GT][GT + 1], us[GT][GT + 1], ws[GT][GT + 1];
     const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
     const int g = blockIdx.z, r0 = blockIdx.x * GT, c0 = blockIdx.y * GT;
@@ -95,6 +96,7 @@ struct BoundParams {
     int M, N, K, G, lda, ldo, tiles_m, tiles_n, KT;
     int ksplit;            // CTAs per output tile, each with an equal share of the k-tiles (1 or 2)
     Post post;             // per-channel epilogue of the stored bounds (all null: none; ksplit == 1 only)
+    const int* only_if;    // not null: the launch does nothing where this word is 0
 };
 
 __device__ __forceinline__ void load_stage(float* stage, const BoundParams& p, int g, int m0, int n0,
@@ -213,6 +215,7 @@ __device__ __forceinline__ bool run_tile(float* smem, const BoundParams& p, int 
 
 __global__ void __launch_bounds__(NT, 3)
 inf_bound_tiled_kernel(const BoundParams p) {
+    if (p.only_if != nullptr && *p.only_if == 0) return;
     extern __shared__ __align__(16) float smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int wm = warp & 1, wn = warp >> 1, lm = lane >> 3, ln = lane & 7;
@@ -285,21 +288,22 @@ inf_bound_post_kernel(float* __restrict__ yl, float* __restrict__ yu, size_t n, 
 }  // namespace
 
 int inf_bound(const float* xl, const float* xu, const float* w, const Dims& d,
-              float* yl, float* yu, cudaStream_t st, const Post& post) {
+              float* yl, float* yu, cudaStream_t st, const Post& post, const int* only_if) {
     const bool tiled = d.HW == 1 && (d.CIg % 4) == 0 && aligned16(xl) && aligned16(xu) && aligned16(w) &&
                        d.COg >= 32;
     if (!tiled) {
-        if (skinny_ok(d, xl, xu, w)) return inf_bound_skinny(xl, xu, w, d, yl, yu, st, post);
+        if (only_if == nullptr && skinny_ok(d, xl, xu, w)) return inf_bound_skinny(xl, xu, w, d, yl, yu, st, post);
         dim3 grid((d.R + GT - 1) / GT, (d.COg + GT - 1) / GT, d.G);
         if (grid.y > 65535u || grid.z > 65535u) return LINF_ERR_DIMS;
-        if (d.HW > 1) inf_bound_generic_kernel<true><<<grid, 256, 0, st>>>(xl, xu, w, d, yl, yu, post);
-        else inf_bound_generic_kernel<false><<<grid, 256, 0, st>>>(xl, xu, w, d, yl, yu, post);
+        if (d.HW > 1) inf_bound_generic_kernel<true><<<grid, 256, 0, st>>>(xl, xu, w, d, yl, yu, post, only_if);
+        else inf_bound_generic_kernel<false><<<grid, 256, 0, st>>>(xl, xu, w, d, yl, yu, post, only_if);
         return launch_status();
     }
     BoundParams p;
     p.xl = xl; p.xu = xu; p.w = w; p.yl = yl; p.yu = yu;
     p.M = d.R; p.N = d.COg; p.K = d.CIg; p.G = d.G; p.lda = d.CI; p.ldo = d.CO;
     p.post = post;
+    p.only_if = only_if;
     p.ksplit = 1;
     p.tiles_m = (d.R + BM - 1) / BM; p.tiles_n = (d.COg + BN - 1) / BN;
     p.KT = (d.CIg + BK - 1) / BK;
@@ -309,7 +313,8 @@ int inf_bound(const float* xl, const float* xu, const float* w, const Dims& d,
         // 1.2 ms at B = 512, Din = 3072, Dout = 5120: 640 tiles on 444 CTA slots).
         const int slots = 3 * sm_count();
         auto fill = [&](int n) { return (double)n / ((double)((n + slots - 1) / slots) * slots); };
-        if (p.KT >= 64 && fill(2 * grid) > 1.15 * fill(grid)) {
+        // (not behind the list pass: the outputs would have to be cleared under its condition)
+        if (only_if == nullptr && p.KT >= 64 && fill(2 * grid) > 1.15 * fill(grid)) {
             const size_t bytes = (size_t)d.R * d.CO * sizeof(float);
             if (cudaMemsetAsync(yl, 0, bytes, st) != cudaSuccess || cudaMemsetAsync(yu, 0, bytes, st) != cudaSuccess)
                 return LINF_ERR_LAUNCH;
@@ -330,6 +335,21 @@ int inf_bound(const float* xl, const float* xu, const float* w, const Dims& d,
         launched = 2;
     }
     return launch_status(launched);
+}
+
+// The bounds through lists of large entries where that may pay (inf_prune.cu), the dense kernel behind.
+size_t inf_bound_pruned_workspace(const Dims& d) { return inf_prune_workspace(d, true); }
+
+int inf_bound_pruned(const float* xl, const float* xu, const float* w, const Dims& d, float* yl, float* yu,
+                     void* ws, size_t ws_bytes, cudaStream_t st, const Post& post) {
+    const size_t need = inf_bound_pruned_workspace(d);
+    if (need == 0 || ws == nullptr) return inf_bound(xl, xu, w, d, yl, yu, st, post);
+    if (ws_bytes < need || (reinterpret_cast<uintptr_t>(ws) & 255u)) return LINF_ERR_WORKSPACE;
+    const int* only_if = nullptr;
+    const bool tiled = (d.CIg % 4) == 0 && aligned16(xl) && aligned16(xu) && aligned16(w);
+    const int rc = inf_prune(xl, xu, w, d, yl, nullptr, yu, true, ws, st, post, tiled ? 1.f : 0.25f, &only_if);
+    if (rc) return rc;
+    return inf_bound(xl, xu, w, d, yl, yu, st, post, only_if);
 }
 
 }  // namespace linf

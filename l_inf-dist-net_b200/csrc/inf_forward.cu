@@ -41,7 +41,8 @@ constexpr int GT = 32;  // generic tile edge
 template <bool ROW_FAST>
 __global__ void __launch_bounds__(256)
 inf_forward_generic_kernel(const float* __restrict__ x, const float* __restrict__ w, Dims d,
-                           float* __restrict__ y, int* __restrict__ pos, Post post) {
+                           float* __restrict__ y, int* __restrict__ pos, Post post, const int* __restrict__ only_if) {
+    if (only_if != nullptr && *only_if == 0) return;
     __shared__ float xs[GT][GT + 1];  // [k][row]
     __shared__ float ws[GT][GT + 1];  // [k][col]
     const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
@@ -120,6 +121,7 @@ struct TiledParams {
     int slots_cta;         // CTAs the partial-result area was sized for
     int tile0;             // whole mode: CTA b owns output tile tile0 + b
     Post post;             // per-channel epilogue of the stored values (all null: none)
+    const int* only_if;    // not null: the launch does nothing where this word is 0
     int* tickets;          // one counter per output tile (split mode), else nullptr
     float* part_val;       // [slots_cta][2][TILE_OUT]
     int* part_cid;         // [slots_cta][2][TILE_OUT]
@@ -360,6 +362,7 @@ __device__ __forceinline__ void tma_stage(float* stage, unsigned long long* bar,
 template <class GEO, bool TRACK, int LOADER>
 __global__ void __launch_bounds__(GEO::NT, GEO::MINB)
 inf_forward_tiled_kernel(const __grid_constant__ TiledParams p) {
+    if (p.only_if != nullptr && *p.only_if == 0) return;
     constexpr int NT = GEO::NT, TN = GEO::TN, NOUT = GEO::NOUT, BK = GEO::BK, TILE_OUT = GEO::TILE_OUT;
     constexpr int BM = GEO::BM, BN = GEO::BN, STAGES = GEO::STAGES, STAGE_FLOATS = GEO::STAGE_FLOATS;
     constexpr int NSUB = GEO::NSUB;
@@ -804,13 +807,13 @@ static int launch_tiled(const Kernels& k, const TiledParams& p, bool track, cuda
 }
 
 int inf_forward(const float* x, const float* w, const Dims& d, float* y, int* pos,
-                void* ws, size_t ws_bytes, cudaStream_t st, const Post& post) {
+                void* ws, size_t ws_bytes, cudaStream_t st, const Post& post, const int* only_if) {
     if (!tiled_ok(x, w, d)) {
-        if (skinny_ok(d, x, w, nullptr)) return inf_forward_skinny(x, w, d, y, pos, st, post);
+        if (only_if == nullptr && skinny_ok(d, x, w, nullptr)) return inf_forward_skinny(x, w, d, y, pos, st, post);
         dim3 grid((d.R + GT - 1) / GT, (d.COg + GT - 1) / GT, d.G);
         if (grid.y > 65535u || grid.z > 65535u) return LINF_ERR_DIMS;
-        if (d.HW > 1) inf_forward_generic_kernel<true><<<grid, 256, 0, st>>>(x, w, d, y, pos, post);
-        else inf_forward_generic_kernel<false><<<grid, 256, 0, st>>>(x, w, d, y, pos, post);
+        if (d.HW > 1) inf_forward_generic_kernel<true><<<grid, 256, 0, st>>>(x, w, d, y, pos, post, only_if);
+        else inf_forward_generic_kernel<false><<<grid, 256, 0, st>>>(x, w, d, y, pos, post, only_if);
         return launch_status();
     }
     const Variant& v = cur_variant();
@@ -843,6 +846,7 @@ int inf_forward(const float* x, const float* w, const Dims& d, float* y, int* po
     p.slots_cta = 0;
     p.tile0 = 0;
     p.post = post;
+    p.only_if = only_if;
     const int slots = use->min_blocks * sm_count();
     if (plan.split) {
         const size_t tick_bytes = align256((size_t)tiles * sizeof(int));
@@ -875,6 +879,28 @@ int inf_forward(const float* x, const float* w, const Dims& d, float* y, int* po
         }
     }
     return launch_tiled(*use, p, pos != nullptr, st);
+}
+
+// The forward through lists of large entries where that may pay (inf_prune.cu), with the dense kernel behind it for the
+// calls that the device finds unsuited; without workspace, or where the query answers 0, the dense kernel alone.
+static size_t up256(size_t n) { return (n + 255) & ~(size_t)255; }
+
+size_t inf_forward_pruned_workspace(const Dims& d) {
+    const size_t lists = inf_prune_workspace(d, false);
+    return lists == 0 ? 0 : up256(lists) + inf_forward_workspace(d);
+}
+
+int inf_forward_pruned(const float* x, const float* w, const Dims& d, float* y, int* pos,
+                       void* ws, size_t ws_bytes, cudaStream_t st, const Post& post) {
+    const size_t need = inf_forward_pruned_workspace(d);
+    if (need == 0 || ws == nullptr) return inf_forward(x, w, d, y, pos, nullptr, 0, st, post);
+    if (ws_bytes < need || (reinterpret_cast<uintptr_t>(ws) & 255u)) return LINF_ERR_WORKSPACE;
+    const size_t lists = up256(inf_prune_workspace(d, false)), dense = inf_forward_workspace(d);
+    const int* only_if = nullptr;
+    const float dense_speed = tiled_ok(x, w, d) ? 1.f : 0.25f;
+    const int rc = inf_prune(x, x, w, d, y, pos, nullptr, false, ws, st, post, dense_speed, &only_if);
+    if (rc) return rc;
+    return inf_forward(x, w, d, y, pos, dense ? reinterpret_cast<char*>(ws) + lists : nullptr, dense, st, post, only_if);
 }
 
 }  // namespace linf

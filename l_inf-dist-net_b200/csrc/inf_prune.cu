@@ -1,0 +1,489 @@
+// inf-dist forward and interval bounds through lists of large entries, for dense layers (HW == 1).
+//
+// A maximum of |x_i - w_i| over thousands of i is large, and |x_i - w_i| <= |x_i| + |w_i|: with two thresholds tx, tw and
+// every entry |x_i| >= tx or |w_i| >= tw looked at, no other i can reach more than tx + tw.  So an output whose
+// maximum over the listed entries is GREATER than fl(tx + tw) is final, exactly as the full scan gives it: rounding is
+// monotonic, |fl(x - w)| <= fl(|x| + |w|) <= fl(tx + tw), so no unlisted term equals the maximum either and the lowest index
+// among equal terms is among the listed ones.  Outputs that do not pass this test are computed by a full scan
+// (`fail_kernel`); if there are too many of them, or the lists would be long, the dense kernel does the layer.
+//
+//   sample_kernel   looks at 128 rows of either side (counts of entries by magnitude) and 1024 outputs; the last CTA takes
+//                   tx + tw = the smallest sampled output and divides it so that the lists are shortest, or decides for the dense kernel
+//   list_kernel     one warp per row of x and of w writes the row's entries (value, index) of at least its threshold,
+//                   ascending, slot by slot across the rows ([slot][row]: a warp that works on 32 rows reads whole lines)
+//   gather_kernel   four rows of one side interleaved in shared memory (one 16-byte load gives an entry's four partners), the
+//                   lanes of a warp are rows of the other side and walk over their own lists.  Once for the lists of x (skipped when
+//                   they are all empty), once for the lists of w, which also merges, tests and stores.
+//   fail_kernel     one warp per output that did not pass
+// All decisions are taken on the device; the dense kernel is launched behind and returns at once unless it is wanted.
+//
+// Bound: shared-memory gathers (a random 16-byte load of a warp takes about 10 cycles for 4 x 32 terms) and the 8-byte list entries
+// from L2.  How many entries there are depends on the data.  Dout = Din = 5120, B = 512: x uniform in [0,1) or activations of a
+// distance net, w ~ N(0,1): 20-45 of 5120; x and w ~ N(0,1): 240.  A gathered term costs about as much as six terms of the dense kernel,
+// hence kGatherCost.
+#include "common.cuh"
+
+namespace linf {
+namespace {
+
+constexpr unsigned FULL = 0xffffffffu;
+constexpr int kBins = 4096, kBinShift = 19;     // bins of |v|: exponent and four bits of the mantissa
+constexpr int kSampleCtas = 128;
+constexpr int kMaxList = 256;                   // slots per row
+constexpr int kMaxK = 14000;                    // 16 bytes each in shared memory
+
+struct Head {                                   // zeroed before every call
+    int ymin_inv;                               // 0x7fffffff - bits of the smallest sampled output
+    int ticket;
+    int dense;                                  // the dense kernel is wanted
+    int any_x;                                  // some list of x is not empty
+    int n_fail;
+    float tx, tw, bound;
+    int pad[56];
+};
+
+struct PruneParams {
+    const float* xl; const float* xu;           // x (twice), or lower and upper
+    const float* w;
+    float* y0; int* pos; float* y1;             // forward: y, pos (or null); bounds: lower, -, upper
+    int R, G, K, N, CI, CO;                     // K inputs and N outputs per group
+    Head* head;
+    int* hist;                                  // [2][kBins]
+    int* cnt_x; int* cnt_w;                     // [G * R], [CO]
+    void* list_x; int2* list_w;                 // [slots][G * R] int2 or int4, [slots][CO]
+    int* fail; int fail_cap;
+    int slots;
+    int vec;                                    // y and pos take 16-byte stores at multiples of four outputs
+    float budget;                               // entries per output at which the dense kernel is as fast
+    Post post;
+};
+
+__device__ __forceinline__ float pinf() { return __int_as_float(0x7f800000); }
+__device__ __forceinline__ int signed_at(float t, int at) { return at | (t < 0.f ? (int)0x80000000 : 0); }
+
+template <bool BOUND>
+__device__ __forceinline__ float key_x(const PruneParams& p, size_t a) {
+    const float v = fabsf(__ldg(p.xl + a));
+    return BOUND ? fmaxf(v, fabsf(__ldg(p.xu + a))) : v;
+}
+
+// one term of an interval bound: U = max of the far ends, m = min (the lower bound is -m, at least 0)
+__device__ __forceinline__ void bound_term(float lo, float up, float w, float& m, float& U) {
+    const float a = w - lo, b = up - w;
+    U = max3(U, a, b);
+    m = fminf(m, fminf(a, b));
+}
+
+template <bool BOUND>
+__global__ void __launch_bounds__(256)
+sample_kernel(const PruneParams p) {
+    __shared__ int hx[kBins], hw[kBins];
+    __shared__ int s_last;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int i = tid; i < kBins; i += 256) { hx[i] = 0; hw[i] = 0; }
+    __syncthreads();
+    const int rows = p.R * p.G;
+    const int rx = (int)((long long)rows * blockIdx.x / kSampleCtas);         // row of x: r * G + g in memory
+    const int r = rx / p.G, g = rx - r * p.G;
+    const size_t xa = (size_t)r * p.CI + (size_t)g * p.K;
+    const float* wh = p.w + (size_t)((long long)p.CO * blockIdx.x / kSampleCtas) * p.K;
+    for (int k = tid; k < p.K; k += 256) {
+        atomicAdd(&hx[__float_as_int(key_x<BOUND>(p, xa + k)) >> kBinShift], 1);
+        atomicAdd(&hw[__float_as_int(fabsf(__ldg(wh + k))) >> kBinShift], 1);
+    }
+    {
+        const int o = (int)((long long)p.N * ((blockIdx.x * 8 + warp) * 37 % 1024) / 1024);
+        const float* wr = p.w + ((size_t)g * p.N + o) * p.K;
+        float v = 0.f;
+#pragma unroll 8
+        for (int k = lane; k < p.K; k += 32) {
+            const float wv = __ldg(wr + k), a = __ldg(p.xl + xa + k);
+            if (BOUND) v = max3(v, a - wv, wv - __ldg(p.xu + xa + k));
+            else v = fmaxf(v, fabsf(a - wv));
+        }
+        const int bits = __reduce_min_sync(FULL, 0x7fffffff - __float_as_int(v));       // the largest v of the lanes
+        if (lane == 0) atomicMax(&p.head->ymin_inv, bits);
+    }
+    __syncthreads();
+    for (int i = tid; i < kBins; i += 256) {
+        if (hx[i]) atomicAdd(&p.hist[i], hx[i]);
+        if (hw[i]) atomicAdd(&p.hist[kBins + i], hw[i]);
+    }
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) s_last = atomicAdd(&p.head->ticket, 1) == kSampleCtas - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+
+    // ---- the last CTA: entries at or above every bin edge, then the division of the smallest sampled output ----
+    constexpr int PER = kBins / 256;
+    __shared__ int tot[2][256];
+    __shared__ float s_cost[8]; __shared__ int s_bin[8];
+    for (int h = 0; h < 2; ++h) {
+        int* dst = h ? hw : hx;
+        int sum = 0;
+        for (int j = PER - 1; j >= 0; --j) {
+            sum += __ldcg(p.hist + h * kBins + tid * PER + j);
+            dst[tid * PER + j] = sum;
+        }
+        tot[h][tid] = sum;
+    }
+    __syncthreads();
+    for (int h = 0; h < 2; ++h) {
+        int above = 0;
+        for (int t = tid + 1; t < 256; ++t) above += tot[h][t];
+        int* dst = h ? hw : hx;
+        for (int j = 0; j < PER; ++j) dst[tid * PER + j] += above;
+    }
+    __syncthreads();
+    const float yref = __int_as_float(0x7fffffff - __ldcg(&p.head->ymin_inv));
+    float cost = 3e38f; int bin = 0;
+    for (int j = tid * PER; j < tid * PER + PER; ++j) {
+        const float tx = __int_as_float(j << kBinShift);
+        const float tw = (yref - tx) * 0.999999f;
+        if (j == 0 || !(tw > 0.f) || !(yref < 3e38f)) continue;
+        const float nx = hx[j] * (1.f / kSampleCtas), nw = hw[__float_as_int(tw) >> kBinShift] * (1.f / kSampleCtas);
+        // lists of x that are (with a bin to spare) empty spare a pass over the weights and the outputs, about a dozen entries' worth
+        const float c = nx + nw + (hx[j - 1] == 0 ? 0.f : 12.f);
+        if (nx <= 0.6f * p.slots && nw <= 0.6f * p.slots && c < cost) { cost = c; bin = j; }
+    }
+#pragma unroll
+    for (int s = 16; s; s >>= 1) {
+        const float oc = __shfl_xor_sync(FULL, cost, s); const int ob = __shfl_xor_sync(FULL, bin, s);
+        if (oc < cost || (oc == cost && ob < bin)) { cost = oc; bin = ob; }
+    }
+    if (lane == 0) { s_cost[warp] = cost; s_bin[warp] = bin; }
+    __syncthreads();
+    if (tid == 0) {
+        for (int k = 1; k < 8; ++k) if (s_cost[k] < cost) { cost = s_cost[k]; bin = s_bin[k]; }
+        const float tx = __int_as_float(bin << kBinShift), tw = (yref - tx) * 0.999999f;
+        p.head->tx = tx; p.head->tw = tw;
+        p.head->bound = __fadd_ru(tx, tw);
+        if (!(cost < p.budget)) p.head->dense = 1;
+    }
+}
+
+// Rows 0 .. R * G - 1 are rows of x, in the order g * R + r; the others rows of w.
+template <bool BOUND>
+__global__ void __launch_bounds__(256)
+list_kernel(const PruneParams p) {
+    if (p.head->dense) return;
+    const int lane = threadIdx.x & 31;
+    const int nx = p.R * p.G;
+    int row = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (row >= nx + p.CO) return;
+    const bool is_x = row < nx;
+    if (!is_x) row -= nx;
+    const float thr = is_x ? p.head->tx : p.head->tw;
+    const int stride = is_x ? nx : p.CO;
+    const int g = is_x ? row / p.R : 0;
+    const size_t at = is_x ? (size_t)(row - g * p.R) * p.CI + (size_t)g * p.K : (size_t)row * p.K;
+    const float* lo = (is_x ? p.xl : p.w) + at;
+    const float* up = is_x && BOUND ? p.xu + at : lo;
+    int n = 0;
+    bool odd = false;                            // bounds: an interval that is empty or not finite
+    constexpr int U = 8;
+    for (int k0 = 0; k0 < p.K; k0 += 32 * U) {
+        float a[U], b[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int k = k0 + 32 * u + lane;
+            a[u] = k < p.K ? __ldg(lo + k) : 0.f;
+            b[u] = BOUND && is_x ? (k < p.K ? __ldg(up + k) : 0.f) : a[u];
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int k = k0 + 32 * u + lane;
+            if (BOUND && is_x) odd |= !(a[u] <= b[u] && a[u] > -pinf() && b[u] < pinf());
+            const bool hit = k < p.K && (fabsf(a[u]) >= thr || (BOUND && fabsf(b[u]) >= thr));
+            const unsigned m = __ballot_sync(FULL, hit);
+            if (m) {
+                const int s = n + __popc(m & ((1u << lane) - 1u));
+                if (hit && s < p.slots) {
+                    const size_t e = (size_t)s * stride + row;
+                    if (!is_x) p.list_w[e] = make_int2(__float_as_int(a[u]), k);
+                    else if (BOUND) reinterpret_cast<int4*>(p.list_x)[e] = make_int4(__float_as_int(a[u]), __float_as_int(b[u]), k, 0);
+                    else reinterpret_cast<int2*>(p.list_x)[e] = make_int2(__float_as_int(a[u]), k);
+                }
+                n += __popc(m);
+            }
+        }
+    }
+    odd = __any_sync(FULL, odd);
+    if (lane == 0) {
+        (is_x ? p.cnt_x : p.cnt_w)[row] = min(n, p.slots);
+        if (n > p.slots || odd) p.head->dense = 1;
+        if (is_x && n > 0) p.head->any_x = 1;
+    }
+}
+
+// Shared rows: W_LISTS: four rows of x (bounds: two rows of lower and upper), lanes = outputs.  Otherwise: four rows of w, lanes = rows of x.
+template <bool BOUND, bool W_LISTS, bool TRACK>
+__global__ void __launch_bounds__(512, 2)
+gather_kernel(const PruneParams p, int blocks_a, int splits) {
+    extern __shared__ __align__(16) float4 rows4[];
+    const int any_x = p.head->any_x;
+    if (p.head->dense || (!W_LISTS && !any_x)) return;
+    constexpr int NA = BOUND && W_LISTS ? 2 : 4;        // rows of the shared side
+    const int tid = threadIdx.x, lane = tid & 31, nt = blockDim.x;
+    int id = blockIdx.x;
+    const int split = id % splits; id /= splits;
+    const int blk = id % blocks_a, g = id / blocks_a;
+    const int a0 = blk * NA;
+    {
+        const int last = (W_LISTS ? p.R : p.N) - 1;
+        const float* src[4];
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            if (W_LISTS && BOUND) src[a] = (a & 1 ? p.xu : p.xl) + (size_t)min(a0 + (a >> 1), last) * p.CI + (size_t)g * p.K;
+            else if (W_LISTS) src[a] = p.xl + (size_t)min(a0 + a, last) * p.CI + (size_t)g * p.K;
+            else src[a] = p.w + ((size_t)g * p.N + min(a0 + a, last)) * p.K;
+        }
+#pragma unroll 2
+        for (int k = tid; k < p.K; k += nt) rows4[k] = make_float4(__ldg(src[0] + k), __ldg(src[1] + k), __ldg(src[2] + k), __ldg(src[3] + k));
+    }
+    __syncthreads();
+    const int NL = W_LISTS ? p.N : p.R;
+    const int stride = W_LISTS ? p.CO : p.G * p.R;
+    const int* cnt = (W_LISTS ? p.cnt_w : p.cnt_x) + g * NL;
+    const int per = ((NL + splits - 1) / splits + 31) / 32 * 32;
+    const int l_end = min(NL, (split + 1) * per);
+    const float bound = p.head->bound;
+    for (int l0 = split * per + (tid & ~31); l0 < l_end; l0 += nt) {
+        const int l = l0 + lane;
+        const int n = l < l_end ? __ldg(cnt + l) : 0;
+        const int most = __reduce_max_sync(FULL, n);
+        float t[4] = {0.f, 0.f, 0.f, 0.f};              // forward: signed difference of the largest term; bounds: U
+        [[maybe_unused]] float m[4] = {0.f, 0.f, 0.f, 0.f};
+        [[maybe_unused]] int at[4] = {0, 0, 0, 0};
+        constexpr int U = 4;
+        for (int s = 0; s < most; s += U) {
+            float v[U], v2[U]; int k[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                // past the end of a list: a NaN, which no comparison takes
+                v[u] = v2[u] = __int_as_float(0x7fffffff); k[u] = 0;
+                if (s + u < n) {
+                    const size_t e = (size_t)(s + u) * stride + (size_t)g * NL + l;
+                    if (!W_LISTS && BOUND) {
+                        const int4 q = __ldg(reinterpret_cast<const int4*>(p.list_x) + e);
+                        v[u] = __int_as_float(q.x); v2[u] = __int_as_float(q.y); k[u] = q.z;
+                    } else {
+                        const int2 q = __ldg((W_LISTS ? p.list_w : reinterpret_cast<const int2*>(p.list_x)) + e);
+                        v[u] = __int_as_float(q.x); k[u] = q.y;
+                    }
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const float4 q = rows4[k[u]];
+                const float r[4] = {q.x, q.y, q.z, q.w};
+                if (BOUND) {
+#pragma unroll
+                    for (int a = 0; a < NA; ++a) {
+                        if (W_LISTS) bound_term(r[2 * (a & 1)], r[2 * (a & 1) + 1], v[u], m[a], t[a]);
+                        else bound_term(v[u], v2[u], r[a], m[a], t[a]);
+                    }
+                } else {
+#pragma unroll
+                    for (int a = 0; a < 4; ++a) {
+                        const float d = W_LISTS ? r[a] - v[u] : v[u] - r[a];
+                        if (fabsf(d) > fabsf(t[a])) { t[a] = d; if (TRACK) at[a] = k[u]; }
+                    }
+                }
+            }
+        }
+        if (l >= l_end) continue;
+        if (!W_LISTS && !BOUND && p.vec && a0 + 3 < p.N) {      // four neighbouring outputs of one row
+            const size_t e = (size_t)l * p.CO + g * p.N + a0;
+            *reinterpret_cast<float4*>(p.y0 + e) = make_float4(fabsf(t[0]), fabsf(t[1]), fabsf(t[2]), fabsf(t[3]));
+            if (TRACK) *reinterpret_cast<int4*>(p.pos + e) = make_int4(signed_at(t[0], at[0]), signed_at(t[1], at[1]), signed_at(t[2], at[2]), signed_at(t[3], at[3]));
+            continue;
+        }
+#pragma unroll
+        for (int a = 0; a < NA; ++a) {
+            const int r = W_LISTS ? a0 + a : l, o = W_LISTS ? l : a0 + a;
+            if (W_LISTS ? r >= p.R : o >= p.N) continue;
+            const int c = g * p.N + o;
+            const size_t e = (size_t)r * p.CO + c;
+            if (BOUND) {
+                float L = 0.f - m[a], U2 = t[a];
+                if (W_LISTS) {
+                    if (any_x) { L = fmaxf(L, p.y0[e]); U2 = fmaxf(U2, p.y1[e]); }
+                    if (L > bound && U2 > bound) {
+                        const float lo = post_apply(p.post, L, c), up = post_apply(p.post, U2, c);
+                        L = p.post.negate ? up : lo; U2 = p.post.negate ? lo : up;
+                    } else {
+                        const int s = atomicAdd(&p.head->n_fail, 1);
+                        if (s < p.fail_cap) p.fail[s] = (int)e;
+                    }
+                }
+                p.y0[e] = L; p.y1[e] = U2;
+            } else {
+                float best = fabsf(t[a]); int where = at[a];
+                bool neg = t[a] < 0.f;
+                if (W_LISTS) {
+                    if (any_x) {
+                        const float y = p.y0[e];
+                        const int q = TRACK ? p.pos[e] : 0;
+                        if (y > best || (TRACK && y == best && (q & 0x7fffffff) < where)) { best = y; where = q & 0x7fffffff; neg = q < 0; }
+                    }
+                    if (!(best > bound)) {
+                        const int s = atomicAdd(&p.head->n_fail, 1);
+                        if (s < p.fail_cap) p.fail[s] = (int)e;
+                    }
+                    best = post_apply(p.post, best, c);
+                }
+                p.y0[e] = best;
+                if (TRACK) p.pos[e] = where | (neg ? (int)0x80000000 : 0);
+            }
+        }
+    }
+}
+
+// The outputs that did not pass: a full scan by one warp each.
+template <bool BOUND, bool TRACK>
+__global__ void __launch_bounds__(256)
+fail_kernel(const PruneParams p) {
+    const int n = p.head->n_fail;
+    if (n > p.fail_cap) {
+        // too many: the dense kernel behind this one does the layer
+        if (blockIdx.x == 0 && threadIdx.x == 0) p.head->dense = 1;
+        return;
+    }
+    if (p.head->dense) return;
+    const int lane = threadIdx.x & 31;
+    for (int q = blockIdx.x * 8 + (threadIdx.x >> 5); q < n; q += gridDim.x * 8) {
+        const int e = p.fail[q], r = e / p.CO, c = e - r * p.CO, g = c / p.N;
+        const size_t xa = (size_t)r * p.CI + (size_t)g * p.K;
+        const float* wr = p.w + (size_t)c * p.K;
+        if (BOUND) {
+            float m = 0.f, U2 = 0.f;
+#pragma unroll 8
+            for (int k = lane; k < p.K; k += 32) bound_term(__ldg(p.xl + xa + k), __ldg(p.xu + xa + k), __ldg(wr + k), m, U2);
+#pragma unroll
+            for (int s = 16; s; s >>= 1) {
+                m = fminf(m, __shfl_xor_sync(FULL, m, s));
+                U2 = fmaxf(U2, __shfl_xor_sync(FULL, U2, s));
+            }
+            if (lane == 0) {
+                const float lo = post_apply(p.post, 0.f - m, c), up = post_apply(p.post, U2, c);
+                p.y0[e] = p.post.negate ? up : lo;
+                p.y1[e] = p.post.negate ? lo : up;
+            }
+        } else {
+            float t = 0.f; int at = 0;
+#pragma unroll 8
+            for (int k = lane; k < p.K; k += 32) {
+                const float d = __ldg(p.xl + xa + k) - __ldg(wr + k);
+                if (fabsf(d) > fabsf(t)) { t = d; at = k; }
+            }
+            // larger |t| first, then the lower index
+#pragma unroll
+            for (int s = 16; s; s >>= 1) {
+                const float ot = __shfl_xor_sync(FULL, t, s); const int oa = __shfl_xor_sync(FULL, at, s);
+                if (fabsf(ot) > fabsf(t) || (fabsf(ot) == fabsf(t) && oa < at)) { t = ot; at = oa; }
+            }
+            if (lane == 0) {
+                p.y0[e] = post_apply(p.post, fabsf(t), c);
+                if (TRACK) p.pos[e] = signed_at(t, at);
+            }
+        }
+    }
+}
+
+size_t up256(size_t n) { return (n + 255) & ~(size_t)255; }
+
+struct PruneSizes { size_t head, cnt_x, cnt_w, list_x, list_w, fail, total; int slots, fail_cap; };
+
+PruneSizes prune_sizes(const Dims& d, bool bound) {
+    PruneSizes s;
+    s.slots = kMaxList < d.CIg ? kMaxList : d.CIg;
+    const size_t nx = (size_t)d.R * d.G, outs = (size_t)d.R * d.CO;
+    s.fail_cap = (int)(outs / 128 + 1024);
+    size_t at = 0;
+    s.head = at; at += up256(sizeof(Head) + 2 * kBins * sizeof(int));
+    s.cnt_x = at; at += up256(nx * sizeof(int));
+    s.cnt_w = at; at += up256((size_t)d.CO * sizeof(int));
+    s.list_x = at; at += up256(nx * s.slots * (bound ? 16 : 8));
+    s.list_w = at; at += up256((size_t)d.CO * s.slots * 8);
+    s.fail = at; at += up256((size_t)s.fail_cap * sizeof(int));
+    s.total = at;
+    return s;
+}
+
+template <bool BOUND, bool W_LISTS, bool TRACK>
+int launch_gather(const PruneParams& p, cudaStream_t st) {
+    constexpr int NA = BOUND && W_LISTS ? 2 : 4;
+    const int na = W_LISTS ? p.R : p.N, nl = W_LISTS ? p.N : p.R;
+    const int blocks = (na + NA - 1) / NA;
+    int threads = (nl + 31) / 32 * 32;
+    if (threads > 512) threads = 512;
+    const size_t smem = (size_t)p.K * 16;
+    int per_sm = (int)(220 * 1024 / (smem + 1024));
+    if (per_sm > 1024 / threads) per_sm = 1024 / threads;
+    if (per_sm < 1) per_sm = 1;
+    // enough CTAs for four waves, as long as every warp of a CTA has a list to walk
+    const long long want = 4LL * per_sm * sm_count();
+    long long splits = (want + (long long)blocks * p.G - 1) / ((long long)blocks * p.G);
+    const int most = (nl + threads - 1) / threads;
+    if (splits > most) splits = most;
+    if (splits < 1) splits = 1;
+    auto kern = gather_kernel<BOUND, W_LISTS, TRACK>;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return LINF_ERR_LAUNCH;
+    kern<<<(unsigned)((long long)blocks * p.G * splits), threads, smem, st>>>(p, blocks, (int)splits);
+    return launch_status();
+}
+
+template <bool BOUND, bool TRACK>
+int run_pruned(const PruneParams& p, cudaStream_t st) {
+    if (cudaMemsetAsync(p.head, 0, sizeof(Head) + 2 * kBins * sizeof(int), st) != cudaSuccess) return LINF_ERR_LAUNCH;
+    sample_kernel<BOUND><<<kSampleCtas, 256, 0, st>>>(p);
+    const int rows = p.R * p.G + p.CO;
+    list_kernel<BOUND><<<(rows + 7) / 8, 256, 0, st>>>(p);
+    int rc = launch_status(2);
+    if (rc) return rc;
+    rc = launch_gather<BOUND, false, TRACK>(p, st);
+    if (rc) return rc;
+    rc = launch_gather<BOUND, true, TRACK>(p, st);
+    if (rc) return rc;
+    fail_kernel<BOUND, TRACK><<<4 * sm_count(), 256, 0, st>>>(p);
+    return launch_status();
+}
+
+}  // namespace
+
+// Which calls are worth the attempt: dense layers with long rows and enough outputs that five extra launches are small.
+bool inf_prune_ok(const Dims& d) {
+    return d.HW == 1 && d.CIg >= 256 && d.CIg <= kMaxK && d.COg >= 64 && d.R >= 64 &&
+           (double)d.R * d.CO * d.CIg >= 1.5e8 && (long long)d.R * d.G + d.CO <= 131072;
+}
+
+size_t inf_prune_workspace(const Dims& d, bool bound) { return inf_prune_ok(d) ? prune_sizes(d, bound).total : 0; }
+
+// The list pass over a workspace of inf_prune_workspace bytes.  *only_if receives the device flag under which the dense kernel must
+// run behind it.  dense_speed: terms per second of the kernel behind, relative to the tiled ones.
+int inf_prune(const float* xl, const float* xu, const float* w, const Dims& d, float* y0, int* pos, float* y1, bool bound,
+              void* ws, cudaStream_t st, const Post& post, float dense_speed, const int** only_if) {
+    const PruneSizes s = prune_sizes(d, bound);
+    char* base = reinterpret_cast<char*>(ws);
+    PruneParams p;
+    p.xl = xl; p.xu = xu; p.w = w; p.y0 = y0; p.pos = pos; p.y1 = y1;
+    p.R = d.R; p.G = d.G; p.K = d.CIg; p.N = d.COg; p.CI = d.CI; p.CO = d.CO;
+    p.head = reinterpret_cast<Head*>(base + s.head);
+    p.hist = reinterpret_cast<int*>(base + s.head + sizeof(Head));
+    p.cnt_x = reinterpret_cast<int*>(base + s.cnt_x); p.cnt_w = reinterpret_cast<int*>(base + s.cnt_w);
+    p.list_x = base + s.list_x; p.list_w = reinterpret_cast<int2*>(base + s.list_w);
+    p.fail = reinterpret_cast<int*>(base + s.fail); p.fail_cap = s.fail_cap;
+    p.slots = s.slots;
+    p.vec = (d.COg & 3) == 0 && aligned16(y0) && (pos == nullptr || aligned16(pos));
+    constexpr float kGatherCost = 6.f;
+    p.budget = 0.85f * d.CIg / (kGatherCost * dense_speed);
+    p.post = post;
+    *only_if = &p.head->dense;
+    if (bound) return run_pruned<true, false>(p, st);
+    return pos != nullptr ? run_pruned<false, true>(p, st) : run_pruned<false, false>(p, st);
+}
+
+}  // namespace linf

@@ -103,8 +103,13 @@ class DistF(torch.autograd.Function):
         with torch.cuda.device(x.device):
             if math.isinf(p):
                 pos = torch.empty(B, CO, HW, device=x.device, dtype=torch.int32)
-                need = lib.linf_inf_dist_forward_workspace_bytes(B, CO, CI, G, HW)
-                if need:
+                lists = lib.linf_inf_dist_forward_pruned_workspace_bytes(B, CO, CI, G, HW)
+                need = 0 if lists else lib.linf_inf_dist_forward_workspace_bytes(B, CO, CI, G, HW)
+                if lists:
+                    ws = torch.empty(lists, dtype=torch.uint8, device=x.device)
+                    rc = lib.linf_inf_dist_forward_pruned(xk.data_ptr(), weight.data_ptr(), B, CO, CI, G, HW, None, None, 0,
+                                                          y.data_ptr(), pos.data_ptr(), ws.data_ptr(), lists, _stream())
+                elif need:
                     ws = _workspace(x.device, need)
                     rc = lib.linf_inf_dist_forward_ws(xk.data_ptr(), weight.data_ptr(), B, CO, CI, G, HW,
                                                       y.data_ptr(), pos.data_ptr(), ws.data_ptr(),
@@ -209,6 +214,13 @@ def inf_dist_post(input, weight, group, post, tag=None):
     y = torch.empty(B, CO, HW, device=input.device, dtype=torch.float32)
     sub, add, neg = _post_args(post)
     with torch.cuda.device(input.device):
+        lists = lib.linf_inf_dist_forward_pruned_workspace_bytes(B, CO, CI, G, HW)
+        if lists:
+            ws = torch.empty(lists, dtype=torch.uint8, device=input.device)
+            rc = lib.linf_inf_dist_forward_pruned(input.data_ptr(), weight.data_ptr(), B, CO, CI, G, HW, sub, add, neg,
+                                                  y.data_ptr(), None, ws.data_ptr(), lists, _stream())
+            _lib.check(rc, "inf_dist_forward_pruned")
+            return y
         need = lib.linf_inf_dist_forward_workspace_bytes(B, CO, CI, G, HW)
         ws = _workspace(input.device, need) if need else None
         rc = lib.linf_inf_dist_forward_post(input.data_ptr(), weight.data_ptr(), B, CO, CI, G, HW, sub, add, neg,
@@ -236,11 +248,14 @@ def inf_dist_bound(input_lower, input_upper, weight, group, use_custom_cuda_func
     lo = torch.empty(B, CO, HW, device=input_lower.device, dtype=torch.float32)
     up = torch.empty_like(lo)
     with torch.cuda.device(input_lower.device):
-        if post is None:
-            rc = lib.linf_inf_dist_bound_forward(input_lower.data_ptr(), input_upper.data_ptr(), weight.data_ptr(),
-                                                 B, CO, CI, G, HW, lo.data_ptr(), up.data_ptr(), _stream())
+        sub, add, neg = _post_args(post)
+        lists = lib.linf_inf_dist_bound_pruned_workspace_bytes(B, CO, CI, G, HW)
+        if lists:
+            ws = torch.empty(lists, dtype=torch.uint8, device=lo.device)
+            rc = lib.linf_inf_dist_bound_pruned(input_lower.data_ptr(), input_upper.data_ptr(), weight.data_ptr(),
+                                                B, CO, CI, G, HW, sub, add, neg, lo.data_ptr(), up.data_ptr(),
+                                                ws.data_ptr(), lists, _stream())
         else:
-            sub, add, neg = _post_args(post)
             rc = lib.linf_inf_dist_bound_forward_post(input_lower.data_ptr(), input_upper.data_ptr(), weight.data_ptr(),
                                                       B, CO, CI, G, HW, sub, add, neg, lo.data_ptr(), up.data_ptr(), _stream())
     _lib.check(rc, "inf_dist_bound_forward")

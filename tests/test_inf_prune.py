@@ -1,0 +1,66 @@
+"""The p = inf forward and bounds through lists of large entries against the full scan: the same bits for every kind of data, whether
+the lists serve, some outputs have to be scanned again, or the dense kernel does the layer."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def make_x(kind, *shape):
+    x = torch.randn(*shape, device="cuda")
+    if kind == "uniform":
+        return torch.rand(*shape, device="cuda")
+    if kind == "narrow":
+        return 0.25 * x
+    if kind == "ties":
+        return (x * 4).round() / 4
+    if kind == "equal":
+        return torch.ones_like(x)
+    if kind == "rows":                       # rows of very different size: the smallest output says little about the others
+        return x * torch.exp(torch.randn(shape[0], 1, 1, device="cuda"))
+    if kind == "spikes":                     # more outputs fail the test than the list of them holds
+        x = 0.01 * x
+        x[:: 2, 0] = 50.0
+        return x
+    if kind == "special":
+        x[3, 5] = x[9] = float("nan")
+        x[11, 7] = float("inf")
+        x[12] = 0.0
+    return x
+
+
+@pytest.mark.parametrize("kind", ["normal", "uniform", "narrow", "ties", "equal", "rows", "spikes", "special"])
+@pytest.mark.parametrize("B,CI,CO,G", [(203, 1027, 1333, 1), (512, 784, 516, 1), (130, 2100, 700, 1), (257, 2048, 2056, 2), (3000, 576, 128, 1)])
+def test_same_bits_as_the_full_scan(cuda, lib, B, CI, CO, G, kind):
+    torch.manual_seed(B)
+    x, w = make_x(kind, B, CI, 1), torch.randn(CO, CI // G, device="cuda")
+    if kind == "ties":
+        w = (w * 4).round() / 4
+    if kind == "special":
+        w[5, 3], w[6, 2] = float("inf"), float("nan")
+    s = torch.cuda.current_stream().cuda_stream
+    clean = lambda t: torch.nan_to_num(t, nan=7.0, posinf=8.0, neginf=9.0)
+    new = lambda dtype=torch.float32: torch.full((B, CO, 1), -7, dtype=dtype, device="cuda")
+
+    y, pos, y2, pos2, y3 = new(), new(torch.int32), new(), new(torch.int32), new()
+    sub, add = torch.randn(CO, device="cuda"), torch.randn(CO, device="cuda")
+    n = lib.linf_inf_dist_forward_pruned_workspace_bytes(B, CO, CI, G, 1)
+    assert n > 0
+    ws = torch.empty(n, dtype=torch.uint8, device="cuda")
+    sizes = (B, CO, CI, G, 1)
+    assert lib.linf_inf_dist_forward_pruned(x.data_ptr(), w.data_ptr(), *sizes, None, None, 0, y.data_ptr(), pos.data_ptr(), ws.data_ptr(), n, s) == 0
+    assert lib.linf_inf_dist_forward(x.data_ptr(), w.data_ptr(), *sizes, y2.data_ptr(), pos2.data_ptr(), s) == 0
+    assert torch.equal(clean(y), clean(y2)) and torch.equal(pos, pos2)
+    assert lib.linf_inf_dist_forward_pruned(x.data_ptr(), w.data_ptr(), *sizes, sub.data_ptr(), add.data_ptr(), 1, y3.data_ptr(), None, ws.data_ptr(), n, s) == 0
+    assert torch.equal(clean(y3), clean(-((y2 - sub.view(1, -1, 1)) + add.view(1, -1, 1))))
+
+    lo, up = x - 0.03, x + 0.03
+    if kind == "special":
+        lo[2, 4] = up[2, 4] + 1.0            # an empty interval
+    n = lib.linf_inf_dist_bound_pruned_workspace_bytes(B, CO, CI, G, 1)
+    ws = torch.empty(n, dtype=torch.uint8, device="cuda")
+    a = [new() for _ in range(4)]
+    for post in ((None, None, 0), (sub.data_ptr(), add.data_ptr(), 1)):
+        assert lib.linf_inf_dist_bound_pruned(lo.data_ptr(), up.data_ptr(), w.data_ptr(), *sizes, *post, a[0].data_ptr(), a[1].data_ptr(), ws.data_ptr(), n, s) == 0
+        assert lib.linf_inf_dist_bound_forward_post(lo.data_ptr(), up.data_ptr(), w.data_ptr(), *sizes, *post, a[2].data_ptr(), a[3].data_ptr(), s) == 0
+        assert torch.equal(clean(a[0]), clean(a[2])) and torch.equal(clean(a[1]), clean(a[3]))
