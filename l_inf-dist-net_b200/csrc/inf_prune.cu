@@ -61,12 +61,6 @@ struct PruneParams {
 __device__ __forceinline__ float pinf() { return __int_as_float(0x7f800000); }
 __device__ __forceinline__ int signed_at(float t, int at) { return at | (t < 0.f ? (int)0x80000000 : 0); }
 
-template <bool BOUND>
-__device__ __forceinline__ float key_x(const PruneParams& p, size_t a) {
-    const float v = fabsf(__ldg(p.xl + a));
-    return BOUND ? fmaxf(v, fabsf(__ldg(p.xu + a))) : v;
-}
-
 // one term of an interval bound: U = max of the far ends, m = min (the lower bound is -m, at least 0)
 __device__ __forceinline__ void bound_term(float lo, float up, float w, float& m, float& U) {
     const float a = w - lo, b = up - w;
@@ -77,8 +71,8 @@ __device__ __forceinline__ void bound_term(float lo, float up, float w, float& m
 template <bool BOUND>
 __global__ void __launch_bounds__(256)
 sample_kernel(const PruneParams p) {
-    __shared__ int hx[kBins], hw[kBins];
-    __shared__ int s_last;
+    __shared__ __align__(16) int hx[kBins], hw[kBins];
+    __shared__ int s_last, s_out[8][8];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (int i = tid; i < kBins; i += 256) { hx[i] = 0; hw[i] = 0; }
     __syncthreads();
@@ -86,23 +80,37 @@ sample_kernel(const PruneParams p) {
     const int rx = (int)((long long)rows * blockIdx.x / kSampleCtas);         // row of x: r * G + g in memory
     const int r = rx / p.G, g = rx - r * p.G;
     const size_t xa = (size_t)r * p.CI + (size_t)g * p.K;
-    const float* wh = p.w + (size_t)((long long)p.CO * blockIdx.x / kSampleCtas) * p.K;
-    for (int k = tid; k < p.K; k += 256) {
-        atomicAdd(&hx[__float_as_int(key_x<BOUND>(p, xa + k)) >> kBinShift], 1);
-        atomicAdd(&hw[__float_as_int(fabsf(__ldg(wh + k))) >> kBinShift], 1);
+    // eight outputs of this row of x, every thread on all eight: 9 loads in flight per step
+    const float* wr[8];
+    float v[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const int o = (int)((long long)p.N * ((blockIdx.x * 8 + q) * 37 % 1024) / 1024);
+        wr[q] = p.w + ((size_t)g * p.N + o) * p.K;
+        v[q] = 0.f;
     }
-    {
-        const int o = (int)((long long)p.N * ((blockIdx.x * 8 + warp) * 37 % 1024) / 1024);
-        const float* wr = p.w + ((size_t)g * p.N + o) * p.K;
-        float v = 0.f;
-#pragma unroll 8
-        for (int k = lane; k < p.K; k += 32) {
-            const float wv = __ldg(wr + k), a = __ldg(p.xl + xa + k);
-            if (BOUND) v = max3(v, a - wv, wv - __ldg(p.xu + xa + k));
-            else v = fmaxf(v, fabsf(a - wv));
-        }
-        const int bits = __reduce_min_sync(FULL, 0x7fffffff - __float_as_int(v));       // the largest v of the lanes
-        if (lane == 0) atomicMax(&p.head->ymin_inv, bits);
+#pragma unroll 2
+    for (int k = tid; k < p.K; k += 256) {
+        const float a = __ldg(p.xl + xa + k), b = BOUND ? __ldg(p.xu + xa + k) : a;
+        float wv[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) wv[q] = __ldg(wr[q] + k);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = BOUND ? max3(v[q], a - wv[q], wv[q] - b) : fmaxf(v[q], fabsf(a - wv[q]));
+        atomicAdd(&hx[__float_as_int(BOUND ? fmaxf(fabsf(a), fabsf(b)) : fabsf(a)) >> kBinShift], 1);
+        atomicAdd(&hw[__float_as_int(fabsf(wv[0])) >> kBinShift], 1);
+    }
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const int bits = __reduce_min_sync(FULL, 0x7fffffff - __float_as_int(v[q]));    // the largest v of the lanes
+        if (lane == 0) s_out[q][warp] = bits;
+    }
+    __syncthreads();
+    if (tid < 8) {
+        int bits = s_out[tid][0];
+#pragma unroll
+        for (int k = 1; k < 8; ++k) bits = min(bits, s_out[tid][k]);
+        atomicMax(&p.head->ymin_inv, bits);
     }
     __syncthreads();
     for (int i = tid; i < kBins; i += 256) {
@@ -117,24 +125,37 @@ sample_kernel(const PruneParams p) {
     __threadfence();
 
     // ---- the last CTA: entries at or above every bin edge, then the division of the smallest sampled output ----
-    constexpr int PER = kBins / 256;
-    __shared__ int tot[2][256];
+    constexpr int PER = kBins / 256;                // 16: four 16-byte loads
+    __shared__ int tot[2][8];
     __shared__ float s_cost[8]; __shared__ int s_bin[8];
+    int above[2];
+#pragma unroll
     for (int h = 0; h < 2; ++h) {
-        int* dst = h ? hw : hx;
-        int sum = 0;
-        for (int j = PER - 1; j >= 0; --j) {
-            sum += __ldcg(p.hist + h * kBins + tid * PER + j);
-            dst[tid * PER + j] = sum;
+        int c[PER], sum = 0;
+#pragma unroll
+        for (int j = 0; j < PER; j += 4) {
+            const int4 q = __ldcg(reinterpret_cast<const int4*>(p.hist + h * kBins + tid * PER + j));
+            c[j] = q.x; c[j + 1] = q.y; c[j + 2] = q.z; c[j + 3] = q.w;
         }
-        tot[h][tid] = sum;
+        int* dst = h ? hw : hx;
+#pragma unroll
+        for (int j = PER - 1; j >= 0; --j) { sum += c[j]; dst[tid * PER + j] = sum; }
+        int incl = sum;                             // of this lane and the lanes above
+#pragma unroll
+        for (int s = 1; s < 32; s <<= 1) {
+            const int t = __shfl_down_sync(FULL, incl, s);
+            if (lane + s < 32) incl += t;
+        }
+        if (lane == 0) tot[h][warp] = incl;
+        above[h] = incl - sum;
     }
     __syncthreads();
+#pragma unroll
     for (int h = 0; h < 2; ++h) {
-        int above = 0;
-        for (int t = tid + 1; t < 256; ++t) above += tot[h][t];
+        for (int k = warp + 1; k < 8; ++k) above[h] += tot[h][k];
         int* dst = h ? hw : hx;
-        for (int j = 0; j < PER; ++j) dst[tid * PER + j] += above;
+#pragma unroll
+        for (int j = 0; j < PER; ++j) dst[tid * PER + j] += above[h];
     }
     __syncthreads();
     const float yref = __int_as_float(0x7fffffff - __ldcg(&p.head->ymin_inv));
@@ -164,8 +185,67 @@ sample_kernel(const PruneParams p) {
     }
 }
 
+// One row's entries of at least `thr`, ascending, written by a warp: (value, index), or (lower, upper, index, -) for PAIR.  Returns how
+// many there are; `odd`: an interval that is empty or not finite.  VEC: K is a multiple of four and the row 16-byte aligned.
+template <bool PAIR, bool VEC>
+__device__ __forceinline__ int list_row(const float* __restrict__ lo, const float* __restrict__ up, int K, float thr, int slots,
+                                        void* list, int stride, int row, int lane, bool& odd) {
+    constexpr int W = VEC ? 4 : 1, U = VEC ? (PAIR ? 2 : 4) : 8;
+    const unsigned below = (1u << lane) - 1u;
+    int n = 0;
+    for (int k0 = 0; k0 < K; k0 += 32 * U * W) {
+        float a[U][W], b[U][W];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int k = k0 + (32 * u + lane) * W;
+            if (VEC) {
+                const float4 q = k < K ? __ldg(reinterpret_cast<const float4*>(lo + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                a[u][0] = q.x; a[u][W > 1] = q.y; a[u][W > 1 ? 2 : 0] = q.z; a[u][W > 1 ? 3 : 0] = q.w;
+                if (PAIR) {
+                    const float4 t = k < K ? __ldg(reinterpret_cast<const float4*>(up + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    b[u][0] = t.x; b[u][W > 1] = t.y; b[u][W > 1 ? 2 : 0] = t.z; b[u][W > 1 ? 3 : 0] = t.w;
+                }
+            } else {
+                a[u][0] = k < K ? __ldg(lo + k) : 0.f;
+                if (PAIR) b[u][0] = k < K ? __ldg(up + k) : 0.f;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int k = k0 + (32 * u + lane) * W;
+            bool hit[W];
+            bool any = false;
+#pragma unroll
+            for (int c = 0; c < W; ++c) {
+                if (PAIR) odd |= !(a[u][c] <= b[u][c] && a[u][c] > -pinf() && b[u][c] < pinf());
+                hit[c] = k < K && (fabsf(a[u][c]) >= thr || (PAIR && fabsf(b[u][c]) >= thr));
+                any |= hit[c];
+            }
+            if (__ballot_sync(FULL, any) == 0) continue;
+            int s = n;
+#pragma unroll
+            for (int c = 0; c < W; ++c) {
+                const unsigned m = __ballot_sync(FULL, hit[c]);
+                s += __popc(m & below);
+                n += __popc(m);
+            }
+#pragma unroll
+            for (int c = 0; c < W; ++c)
+                if (hit[c]) {
+                    if (s < slots) {
+                        const size_t e = (size_t)s * stride + row;
+                        if (PAIR) reinterpret_cast<int4*>(list)[e] = make_int4(__float_as_int(a[u][c]), __float_as_int(b[u][c]), k + c, 0);
+                        else reinterpret_cast<int2*>(list)[e] = make_int2(__float_as_int(a[u][c]), k + c);
+                    }
+                    ++s;
+                }
+        }
+    }
+    return n;
+}
+
 // Rows 0 .. R * G - 1 are rows of x, in the order g * R + r; the others rows of w.
-template <bool BOUND>
+template <bool BOUND, bool VEC>
 __global__ void __launch_bounds__(256)
 list_kernel(const PruneParams p) {
     if (p.head->dense) return;
@@ -173,59 +253,39 @@ list_kernel(const PruneParams p) {
     const int nx = p.R * p.G;
     int row = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (row >= nx + p.CO) return;
-    const bool is_x = row < nx;
-    if (!is_x) row -= nx;
-    const float thr = is_x ? p.head->tx : p.head->tw;
-    const int stride = is_x ? nx : p.CO;
-    const int g = is_x ? row / p.R : 0;
-    const size_t at = is_x ? (size_t)(row - g * p.R) * p.CI + (size_t)g * p.K : (size_t)row * p.K;
-    const float* lo = (is_x ? p.xl : p.w) + at;
-    const float* up = is_x && BOUND ? p.xu + at : lo;
-    int n = 0;
-    bool odd = false;                            // bounds: an interval that is empty or not finite
-    constexpr int U = 8;
-    for (int k0 = 0; k0 < p.K; k0 += 32 * U) {
-        float a[U], b[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int k = k0 + 32 * u + lane;
-            a[u] = k < p.K ? __ldg(lo + k) : 0.f;
-            b[u] = BOUND && is_x ? (k < p.K ? __ldg(up + k) : 0.f) : a[u];
+    bool odd = false;
+    if (row < nx) {
+        const int g = row / p.R;
+        const size_t at = (size_t)(row - g * p.R) * p.CI + (size_t)g * p.K;
+        const int n = list_row<BOUND, VEC>(p.xl + at, p.xu + at, p.K, p.head->tx, p.slots, p.list_x, nx, row, lane, odd);
+        odd = __any_sync(FULL, odd);
+        if (lane == 0) {
+            p.cnt_x[row] = min(n, p.slots);
+            if (n > p.slots || odd) p.head->dense = 1;
+            if (n > 0) p.head->any_x = 1;
         }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int k = k0 + 32 * u + lane;
-            if (BOUND && is_x) odd |= !(a[u] <= b[u] && a[u] > -pinf() && b[u] < pinf());
-            const bool hit = k < p.K && (fabsf(a[u]) >= thr || (BOUND && fabsf(b[u]) >= thr));
-            const unsigned m = __ballot_sync(FULL, hit);
-            if (m) {
-                const int s = n + __popc(m & ((1u << lane) - 1u));
-                if (hit && s < p.slots) {
-                    const size_t e = (size_t)s * stride + row;
-                    if (!is_x) p.list_w[e] = make_int2(__float_as_int(a[u]), k);
-                    else if (BOUND) reinterpret_cast<int4*>(p.list_x)[e] = make_int4(__float_as_int(a[u]), __float_as_int(b[u]), k, 0);
-                    else reinterpret_cast<int2*>(p.list_x)[e] = make_int2(__float_as_int(a[u]), k);
-                }
-                n += __popc(m);
-            }
+    } else {
+        row -= nx;
+        const float* w = p.w + (size_t)row * p.K;
+        const int n = list_row<false, VEC>(w, w, p.K, p.head->tw, p.slots, p.list_w, p.CO, row, lane, odd);
+        if (lane == 0) {
+            p.cnt_w[row] = min(n, p.slots);
+            if (n > p.slots) p.head->dense = 1;
         }
-    }
-    odd = __any_sync(FULL, odd);
-    if (lane == 0) {
-        (is_x ? p.cnt_x : p.cnt_w)[row] = min(n, p.slots);
-        if (n > p.slots || odd) p.head->dense = 1;
-        if (is_x && n > 0) p.head->any_x = 1;
     }
 }
 
-// Shared rows: W_LISTS: four rows of x (bounds: two rows of lower and upper), lanes = outputs.  Otherwise: four rows of w, lanes = rows of x.
-template <bool BOUND, bool W_LISTS, bool TRACK>
-__global__ void __launch_bounds__(512, 2)
+// Shared rows, 4 * NQ of them in NQ arrays of float4 [K] (one array of twice the width would use half the bank groups per load).  W_LISTS:
+// rows of x (bounds: lower and upper of half as many rows), lanes = outputs.  Otherwise: rows of w, lanes = rows of x.  NQ = 2 halves the
+// list entries read from L2; NQ = 1 is for rows too long for two arrays and for layers with too few blocks of rows to fill the GPU.
+template <bool BOUND, bool W_LISTS, bool TRACK, int NQ>
+__global__ void __launch_bounds__(1024, 1)
 gather_kernel(const PruneParams p, int blocks_a, int splits) {
     extern __shared__ __align__(16) float4 rows4[];
     const int any_x = p.head->any_x;
     if (p.head->dense || (!W_LISTS && !any_x)) return;
-    constexpr int NA = BOUND && W_LISTS ? 2 : 4;        // rows of the shared side
+    constexpr bool PAIRS = BOUND && W_LISTS;
+    constexpr int NA = PAIRS ? 2 * NQ : 4 * NQ;         // rows of the shared side
     const int tid = threadIdx.x, lane = tid & 31, nt = blockDim.x;
     int id = blockIdx.x;
     const int split = id % splits; id /= splits;
@@ -233,15 +293,19 @@ gather_kernel(const PruneParams p, int blocks_a, int splits) {
     const int a0 = blk * NA;
     {
         const int last = (W_LISTS ? p.R : p.N) - 1;
-        const float* src[4];
 #pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            if (W_LISTS && BOUND) src[a] = (a & 1 ? p.xu : p.xl) + (size_t)min(a0 + (a >> 1), last) * p.CI + (size_t)g * p.K;
-            else if (W_LISTS) src[a] = p.xl + (size_t)min(a0 + a, last) * p.CI + (size_t)g * p.K;
-            else src[a] = p.w + ((size_t)g * p.N + min(a0 + a, last)) * p.K;
+        for (int q = 0; q < NQ; ++q) {
+            const float* src[4];
+#pragma unroll
+            for (int a = 0; a < 4; ++a) {
+                if (PAIRS) src[a] = (a & 1 ? p.xu : p.xl) + (size_t)min(a0 + 2 * q + (a >> 1), last) * p.CI + (size_t)g * p.K;
+                else if (W_LISTS) src[a] = p.xl + (size_t)min(a0 + 4 * q + a, last) * p.CI + (size_t)g * p.K;
+                else src[a] = p.w + ((size_t)g * p.N + min(a0 + 4 * q + a, last)) * p.K;
+            }
+#pragma unroll 4
+            for (int k = tid; k < p.K; k += nt)
+                rows4[q * p.K + k] = make_float4(__ldg(src[0] + k), __ldg(src[1] + k), __ldg(src[2] + k), __ldg(src[3] + k));
         }
-#pragma unroll 2
-        for (int k = tid; k < p.K; k += nt) rows4[k] = make_float4(__ldg(src[0] + k), __ldg(src[1] + k), __ldg(src[2] + k), __ldg(src[3] + k));
     }
     __syncthreads();
     const int NL = W_LISTS ? p.N : p.R;
@@ -254,15 +318,17 @@ gather_kernel(const PruneParams p, int blocks_a, int splits) {
         const int l = l0 + lane;
         const int n = l < l_end ? __ldg(cnt + l) : 0;
         const int most = __reduce_max_sync(FULL, n);
-        float t[4] = {0.f, 0.f, 0.f, 0.f};              // forward: signed difference of the largest term; bounds: U
-        [[maybe_unused]] float m[4] = {0.f, 0.f, 0.f, 0.f};
-        [[maybe_unused]] int at[4] = {0, 0, 0, 0};
+        float t[NA];                                    // forward: signed difference of the largest term; bounds: U
+        [[maybe_unused]] float m[BOUND ? NA : 1];
+        [[maybe_unused]] int at[TRACK ? NA : 1];
+#pragma unroll
+        for (int a = 0; a < NA; ++a) { t[a] = 0.f; if (BOUND) m[a] = 0.f; if (TRACK) at[a] = 0; }
         constexpr int U = 4;
-        for (int s = 0; s < most; s += U) {
-            float v[U], v2[U]; int k[U];
+        float v[U], v2[U]; int k[U];
+        // past the end of a list: a NaN, which no comparison takes
+        auto fetch = [&](int s) {
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                // past the end of a list: a NaN, which no comparison takes
                 v[u] = v2[u] = __int_as_float(0x7fffffff); k[u] = 0;
                 if (s + u < n) {
                     const size_t e = (size_t)(s + u) * stride + (size_t)g * NL + l;
@@ -275,30 +341,46 @@ gather_kernel(const PruneParams p, int blocks_a, int splits) {
                     }
                 }
             }
+        };
+        fetch(0);
+        for (int s = 0; s < most; s += U) {
+            float c[U], c2[U]; int kk[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) { c[u] = v[u]; c2[u] = v2[u]; kk[u] = k[u]; }
+            fetch(s + U);                               // the next entries are on their way while these are looked up
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                const float4 q = rows4[k[u]];
-                const float r[4] = {q.x, q.y, q.z, q.w};
-                if (BOUND) {
 #pragma unroll
-                    for (int a = 0; a < NA; ++a) {
-                        if (W_LISTS) bound_term(r[2 * (a & 1)], r[2 * (a & 1) + 1], v[u], m[a], t[a]);
-                        else bound_term(v[u], v2[u], r[a], m[a], t[a]);
-                    }
-                } else {
+                for (int q = 0; q < NQ; ++q) {
+                    const float4 f = rows4[q * p.K + kk[u]];
+                    const float r[4] = {f.x, f.y, f.z, f.w};
+                    if (PAIRS) {
 #pragma unroll
-                    for (int a = 0; a < 4; ++a) {
-                        const float d = W_LISTS ? r[a] - v[u] : v[u] - r[a];
-                        if (fabsf(d) > fabsf(t[a])) { t[a] = d; if (TRACK) at[a] = k[u]; }
+                        for (int a = 0; a < 2; ++a) bound_term(r[2 * a], r[2 * a + 1], c[u], m[2 * q + a], t[2 * q + a]);
+                    } else if (BOUND) {
+#pragma unroll
+                        for (int a = 0; a < 4; ++a) bound_term(c[u], c2[u], r[a], m[(BOUND ? 4 * q + a : 0)], t[(4 * q + a) % NA]);
+                    } else {
+#pragma unroll
+                        for (int a = 0; a < 4; ++a) {
+                            const float d = W_LISTS ? r[a] - c[u] : c[u] - r[a];
+                            const int i = (4 * q + a) % NA;
+                            if (fabsf(d) > fabsf(t[i])) { t[i] = d; if (TRACK) at[i] = kk[u]; }
+                        }
                     }
                 }
             }
         }
         if (l >= l_end) continue;
-        if (!W_LISTS && !BOUND && p.vec && a0 + 3 < p.N) {      // four neighbouring outputs of one row
+        if (!W_LISTS && !BOUND && p.vec && a0 + NA <= p.N) {    // neighbouring outputs of one row, four at a time
             const size_t e = (size_t)l * p.CO + g * p.N + a0;
-            *reinterpret_cast<float4*>(p.y0 + e) = make_float4(fabsf(t[0]), fabsf(t[1]), fabsf(t[2]), fabsf(t[3]));
-            if (TRACK) *reinterpret_cast<int4*>(p.pos + e) = make_int4(signed_at(t[0], at[0]), signed_at(t[1], at[1]), signed_at(t[2], at[2]), signed_at(t[3], at[3]));
+#pragma unroll
+            for (int a = 0; a < NA; a += 4) {
+                *reinterpret_cast<float4*>(p.y0 + e + a) = make_float4(fabsf(t[a]), fabsf(t[(a + 1) % NA]), fabsf(t[(a + 2) % NA]), fabsf(t[(a + 3) % NA]));
+                if constexpr (TRACK)
+                    *reinterpret_cast<int4*>(p.pos + e + a) = make_int4(signed_at(t[a], at[a]), signed_at(t[(a + 1) % NA], at[(a + 1) % NA]),
+                                                                        signed_at(t[(a + 2) % NA], at[(a + 2) % NA]), signed_at(t[(a + 3) % NA], at[(a + 3) % NA]));
+            }
             continue;
         }
 #pragma unroll
@@ -307,7 +389,7 @@ gather_kernel(const PruneParams p, int blocks_a, int splits) {
             if (W_LISTS ? r >= p.R : o >= p.N) continue;
             const int c = g * p.N + o;
             const size_t e = (size_t)r * p.CO + c;
-            if (BOUND) {
+            if constexpr (BOUND) {
                 float L = 0.f - m[a], U2 = t[a];
                 if (W_LISTS) {
                     if (any_x) { L = fmaxf(L, p.y0[e]); U2 = fmaxf(U2, p.y1[e]); }
@@ -321,7 +403,7 @@ gather_kernel(const PruneParams p, int blocks_a, int splits) {
                 }
                 p.y0[e] = L; p.y1[e] = U2;
             } else {
-                float best = fabsf(t[a]); int where = at[a];
+                float best = fabsf(t[a]); int where = TRACK ? at[TRACK ? a : 0] : 0;
                 bool neg = t[a] < 0.f;
                 if (W_LISTS) {
                     if (any_x) {
@@ -342,10 +424,13 @@ gather_kernel(const PruneParams p, int blocks_a, int splits) {
     }
 }
 
-// The outputs that did not pass: a full scan by one warp each.
+// The outputs that did not pass: a full scan by a CTA of four warps each (by one warp, the 160 dependent loads of a row of 5120 made
+// this the longest kernel of a layer with a few hundred such outputs: 40 us).
 template <bool BOUND, bool TRACK>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(128)
 fail_kernel(const PruneParams p) {
+    __shared__ float s_t[4], s_u[4];
+    __shared__ int s_i[4];
     const int n = p.head->n_fail;
     if (n > p.fail_cap) {
         // too many: the dense kernel behind this one does the layer
@@ -353,39 +438,42 @@ fail_kernel(const PruneParams p) {
         return;
     }
     if (p.head->dense) return;
-    const int lane = threadIdx.x & 31;
-    for (int q = blockIdx.x * 8 + (threadIdx.x >> 5); q < n; q += gridDim.x * 8) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int q = blockIdx.x; q < n; q += gridDim.x) {
         const int e = p.fail[q], r = e / p.CO, c = e - r * p.CO, g = c / p.N;
         const size_t xa = (size_t)r * p.CI + (size_t)g * p.K;
         const float* wr = p.w + (size_t)c * p.K;
-        if (BOUND) {
-            float m = 0.f, U2 = 0.f;
+        float t = 0.f, u = 0.f; int at = 0;             // forward: signed difference, index; bounds: -lower, upper
 #pragma unroll 8
-            for (int k = lane; k < p.K; k += 32) bound_term(__ldg(p.xl + xa + k), __ldg(p.xu + xa + k), __ldg(wr + k), m, U2);
-#pragma unroll
-            for (int s = 16; s; s >>= 1) {
-                m = fminf(m, __shfl_xor_sync(FULL, m, s));
-                U2 = fmaxf(U2, __shfl_xor_sync(FULL, U2, s));
-            }
-            if (lane == 0) {
-                const float lo = post_apply(p.post, 0.f - m, c), up = post_apply(p.post, U2, c);
-                p.y0[e] = p.post.negate ? up : lo;
-                p.y1[e] = p.post.negate ? lo : up;
-            }
-        } else {
-            float t = 0.f; int at = 0;
-#pragma unroll 8
-            for (int k = lane; k < p.K; k += 32) {
+        for (int k = tid; k < p.K; k += 128) {
+            if (BOUND) {
+                bound_term(__ldg(p.xl + xa + k), __ldg(p.xu + xa + k), __ldg(wr + k), t, u);
+            } else {
                 const float d = __ldg(p.xl + xa + k) - __ldg(wr + k);
                 if (fabsf(d) > fabsf(t)) { t = d; at = k; }
             }
-            // larger |t| first, then the lower index
+        }
+        // larger |t| first, then the lower index
+        auto merge = [&](float ot, float ou, int oa) {
+            if (BOUND) { t = fminf(t, ot); u = fmaxf(u, ou); }
+            else if (fabsf(ot) > fabsf(t) || (fabsf(ot) == fabsf(t) && oa < at)) { t = ot; at = oa; }
+        };
 #pragma unroll
-            for (int s = 16; s; s >>= 1) {
-                const float ot = __shfl_xor_sync(FULL, t, s); const int oa = __shfl_xor_sync(FULL, at, s);
-                if (fabsf(ot) > fabsf(t) || (fabsf(ot) == fabsf(t) && oa < at)) { t = ot; at = oa; }
-            }
-            if (lane == 0) {
+        for (int s = 16; s; s >>= 1) {
+            const float ot = __shfl_xor_sync(FULL, t, s), ou = __shfl_xor_sync(FULL, u, s);
+            const int oa = __shfl_xor_sync(FULL, at, s);
+            merge(ot, ou, oa);
+        }
+        __syncthreads();                                // the previous output's values have been read
+        if (lane == 0) { s_t[warp] = t; s_u[warp] = u; s_i[warp] = at; }
+        __syncthreads();
+        if (tid == 0) {
+            for (int k = 1; k < 4; ++k) merge(s_t[k], s_u[k], s_i[k]);
+            if (BOUND) {
+                const float lo = post_apply(p.post, 0.f - t, c), up = post_apply(p.post, u, c);
+                p.y0[e] = p.post.negate ? up : lo;
+                p.y1[e] = p.post.negate ? lo : up;
+            } else {
                 p.y0[e] = post_apply(p.post, fabsf(t), c);
                 if (TRACK) p.pos[e] = signed_at(t, at);
             }
@@ -413,42 +501,52 @@ PruneSizes prune_sizes(const Dims& d, bool bound) {
     return s;
 }
 
-template <bool BOUND, bool W_LISTS, bool TRACK>
-int launch_gather(const PruneParams& p, cudaStream_t st) {
-    constexpr int NA = BOUND && W_LISTS ? 2 : 4;
+template <bool BOUND, bool W_LISTS, bool TRACK, int NQ>
+int launch_gather_as(const PruneParams& p, cudaStream_t st) {
+    constexpr int NA = (BOUND && W_LISTS ? 2 : 4) * NQ;
     const int na = W_LISTS ? p.R : p.N, nl = W_LISTS ? p.N : p.R;
     const int blocks = (na + NA - 1) / NA;
-    int threads = (nl + 31) / 32 * 32;
-    if (threads > 512) threads = 512;
-    const size_t smem = (size_t)p.K * 16;
+    const size_t smem = (size_t)p.K * 16 * NQ;
     int per_sm = (int)(220 * 1024 / (smem + 1024));
-    if (per_sm > 1024 / threads) per_sm = 1024 / threads;
+    if (per_sm > 4) per_sm = 4;
     if (per_sm < 1) per_sm = 1;
+    // 32 warps on an SM (64 registers a thread); no more threads than lanes of work, but enough to fill the shared rows
+    int threads = 1024 / per_sm;
+    const int lanes = (nl + 31) / 32 * 32;
+    if (threads > lanes) threads = lanes < 256 ? 256 : lanes;
     // enough CTAs for four waves, as long as every warp of a CTA has a list to walk
     const long long want = 4LL * per_sm * sm_count();
     long long splits = (want + (long long)blocks * p.G - 1) / ((long long)blocks * p.G);
     const int most = (nl + threads - 1) / threads;
     if (splits > most) splits = most;
     if (splits < 1) splits = 1;
-    auto kern = gather_kernel<BOUND, W_LISTS, TRACK>;
+    auto kern = gather_kernel<BOUND, W_LISTS, TRACK, NQ>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return LINF_ERR_LAUNCH;
     kern<<<(unsigned)((long long)blocks * p.G * splits), threads, smem, st>>>(p, blocks, (int)splits);
     return launch_status();
 }
 
+template <bool BOUND, bool W_LISTS, bool TRACK>
+int launch_gather(const PruneParams& p, cudaStream_t st) {
+    const long long rows = (long long)(W_LISTS ? p.R * (BOUND ? 2 : 1) : p.N) * p.G;
+    const bool two = p.K <= kMaxK / 2 && rows * ((W_LISTS ? p.N : p.R) + 511) / 512 >= 8LL * 4 * sm_count();
+    return two ? launch_gather_as<BOUND, W_LISTS, TRACK, 2>(p, st) : launch_gather_as<BOUND, W_LISTS, TRACK, 1>(p, st);
+}
+
 template <bool BOUND, bool TRACK>
-int run_pruned(const PruneParams& p, cudaStream_t st) {
+int run_pruned(const PruneParams& p, bool vec, cudaStream_t st) {
     if (cudaMemsetAsync(p.head, 0, sizeof(Head) + 2 * kBins * sizeof(int), st) != cudaSuccess) return LINF_ERR_LAUNCH;
     sample_kernel<BOUND><<<kSampleCtas, 256, 0, st>>>(p);
-    const int rows = p.R * p.G + p.CO;
-    list_kernel<BOUND><<<(rows + 7) / 8, 256, 0, st>>>(p);
+    const int blocks = (p.R * p.G + p.CO + 7) / 8;
+    if (vec) list_kernel<BOUND, true><<<blocks, 256, 0, st>>>(p);
+    else list_kernel<BOUND, false><<<blocks, 256, 0, st>>>(p);
     int rc = launch_status(2);
     if (rc) return rc;
     rc = launch_gather<BOUND, false, TRACK>(p, st);
     if (rc) return rc;
     rc = launch_gather<BOUND, true, TRACK>(p, st);
     if (rc) return rc;
-    fail_kernel<BOUND, TRACK><<<4 * sm_count(), 256, 0, st>>>(p);
+    fail_kernel<BOUND, TRACK><<<8 * sm_count(), 128, 0, st>>>(p);
     return launch_status();
 }
 
@@ -482,8 +580,9 @@ int inf_prune(const float* xl, const float* xu, const float* w, const Dims& d, f
     p.budget = 0.85f * d.CIg / (kGatherCost * dense_speed);
     p.post = post;
     *only_if = &p.head->dense;
-    if (bound) return run_pruned<true, false>(p, st);
-    return pos != nullptr ? run_pruned<false, true>(p, st) : run_pruned<false, false>(p, st);
+    const bool vec = (d.CIg & 3) == 0 && aligned16(xl) && aligned16(xu) && aligned16(w);
+    if (bound) return run_pruned<true, false>(p, vec, st);
+    return pos != nullptr ? run_pruned<false, true>(p, vec, st) : run_pruned<false, false>(p, vec, st);
 }
 
 }  // namespace linf

@@ -44,38 +44,56 @@ __device__ __forceinline__ float ex2_approx(float a) { float r; asm("ex2.approx.
 
 struct PowQ { int m; float f; };       // p - 2 = m + f
 
-template <int E>
-__device__ __forceinline__ u64 pow2_ct(u64 a) {       // a^E, E >= 1
-    if constexpr (E == 1) return a;
-    else if constexpr (E % 2 == 0) { const u64 h = pow2_ct<E / 2>(a); return mul2(h, h); }
-    else if constexpr (E % 4 == 3) { const u64 h = pow2_ct<(E - 1) / 2>(a); return mul2(mul2(h, a), h); }   // (h * a) * h
-    else return mul2(pow2_ct<E - 1>(a), a);
-}
-
-// s * |s|^(p-2) for a pair.  IP > 0: p is that even integer (the sign comes with the odd power).  IP <= 0: p - 2 = q.m + q.f at run time,
-// q.m < 2^-IP; the bit tests are uniform over the grid.
-template <int IP>
-__device__ __forceinline__ u64 factor2(u64 s, const PowQ q) {
-    if constexpr (IP > 0) {
-        return pow2_ct<IP - 1>(s);
+// s <- s * |s|^(p-2) for N pairs.  IP > 0: p is that even integer (the sign comes with the odd power p - 1: 7 and 15 as
+// (a^n * a) * a^n, 63 along the chain 2 3 6 12 15 30 60 63).  IP <= 0: p - 2 = q.m + q.f at run time, q.m < 2^-IP; the bit tests are
+// uniform over the grid, and one test serves all N pairs: a branch per pair kept the pairs' chains from overlapping
+// (B = 512, Din = Dout = 5120, p = 23.7: RUNTIME_BEFORE -> RUNTIME_AFTER us).
+template <int IP, int N>
+__device__ __forceinline__ void factors(u64 (&s)[N], const PowQ q) {
+    if constexpr (IP == 8 || IP == 16) {
+#pragma unroll
+        for (int e = 0; e < N; ++e) {
+            const u64 a = s[e], a3 = mul2(mul2(a, a), a), a7 = mul2(mul2(a3, a), a3);
+            if constexpr (IP == 8) s[e] = a7;
+            else s[e] = mul2(mul2(a7, a), a7);
+        }
+    } else if constexpr (IP == 64) {
+#pragma unroll
+        for (int e = 0; e < N; ++e) {
+            const u64 a = s[e], a3 = mul2(mul2(a, a), a), a6 = mul2(a3, a3), a15 = mul2(mul2(a6, a6), a3), a30 = mul2(a15, a15);
+            s[e] = mul2(mul2(a30, a30), a3);
+        }
     } else {
         constexpr int NB = -IP;
-        u64 v = s;
-        if (q.m & 1) v = mul2(v, abs2(s));
-        u64 b = s;
+        u64 b[N], v[N];
+#pragma unroll
+        for (int e = 0; e < N; ++e) { b[e] = s[e]; v[e] = s[e]; }
+        if (q.m & 1) {
+#pragma unroll
+            for (int e = 0; e < N; ++e) v[e] = mul2(v[e], abs2(s[e]));
+        }
 #pragma unroll
         for (int k = 1; k < NB; ++k) {
             if ((q.m >> k) == 0) break;
-            b = mul2(b, b);
-            if ((q.m >> k) & 1) v = mul2(v, b);
+#pragma unroll
+            for (int e = 0; e < N; ++e) b[e] = mul2(b[e], b[e]);
+            if ((q.m >> k) & 1) {
+#pragma unroll
+                for (int e = 0; e < N; ++e) v[e] = mul2(v[e], b[e]);
+            }
         }
         if (q.f != 0.f) {
-            float s0, s1;
-            unpack_f32x2(s, s0, s1);
-            // s = 0: exp2(-inf) = 0
-            v = mul2(v, pack2(ex2_approx(q.f * lg2_approx(fabsf(s0))), ex2_approx(q.f * lg2_approx(fabsf(s1)))));
+            const u64 ff = pack2(q.f, q.f);
+#pragma unroll
+            for (int e = 0; e < N; ++e) {
+                float a0, a1;
+                unpack_f32x2(s[e], a0, a1);
+                unpack_f32x2(mul2(pack2(lg2_approx(fabsf(a0)), lg2_approx(fabsf(a1))), ff), a0, a1);
+                v[e] = mul2(v[e], pack2(ex2_approx(a0), ex2_approx(a1)));       // s = 0: exp2(-inf) = 0
+            }
         }
-        return v;
+#pragma unroll
+        for (int e = 0; e < N; ++e) s[e] = v[e];
     }
 }
 
@@ -211,16 +229,29 @@ __device__ __forceinline__ void both_body(const BothParams& p, float* smem) {
                     const ulonglong2 hv = *reinterpret_cast<const ulonglong2*>(hs + o * BT + 2 * k);
                     ulonglong2 rv;
                     if (SCALED) rv = *reinterpret_cast<const ulonglong2*>(rs + o * BT + 2 * k);
+                    if constexpr (IP > 0) {
 #pragma unroll
-                    for (int e = 0; e < 2; ++e)
+                        for (int e = 0; e < 2; ++e)
 #pragma unroll
-                        for (int c = 0; c < 2; ++c) {
-                            u64 s = sub_f32x2(xp[k + e][c], w2[c]);
-                            if (SCALED) s = mul2(s, e ? rv.y : rv.x);
-                            const u64 f = factor2<IP>(s, p.q);
-                            if (DOX) acc[k + e][c] = fma2(e ? hv.y : hv.x, f, acc[k + e][c]);
-                            if (DOW) sum[c] = fma2(e ? hv.y : hv.x, f, sum[c]);
+                            for (int c = 0; c < 2; ++c) {
+                                u64 f[1] = {sub_f32x2(xp[k + e][c], w2[c])};
+                                if (SCALED) f[0] = mul2(f[0], e ? rv.y : rv.x);
+                                factors<IP>(f, p.q);
+                                if (DOX) acc[k + e][c] = fma2(e ? hv.y : hv.x, f[0], acc[k + e][c]);
+                                if (DOW) sum[c] = fma2(e ? hv.y : hv.x, f[0], sum[c]);
+                            }
+                    } else {
+                        u64 f[4];
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) f[e] = mul2(sub_f32x2(xp[k + (e >> 1)][e & 1], w2[e & 1]), e >> 1 ? rv.y : rv.x);
+                        factors<IP>(f, p.q);
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const u64 h2 = e >> 1 ? hv.y : hv.x;
+                            if (DOX) acc[k + (e >> 1)][e & 1] = fma2(h2, f[e], acc[k + (e >> 1)][e & 1]);
+                            if (DOW) sum[e & 1] = fma2(h2, f[e], sum[e & 1]);
                         }
+                    }
                 }
                 if (DOW) {
                     float a0, a1, b0, b1;
@@ -269,13 +300,13 @@ lp_backward_both_kernel(const BothParams p) {
     both_body<IP, WARPS, DOX, DOW, AL, true>(p, smem);
 }
 
-// grad_output and 1 / y (0 where y is not positive) transposed to [CO][Bp] (rows past the batch: zero), and for
+// 1 / y (0 where y is not positive) and grad_output, less the rounding of 1 / y, transposed to [CO][Bp] (rows past the batch: zero), and for
 // p = 8 / 16 the factor h = g / y^(p-1) with the look at the range of y.  With y in [2^-8, 2^8] (p = 8) or [2^-3, 2^4] (p = 16)
 // y^(p-1) and its reciprocal stay within 2^+-60, and a difference whose power underflows is below 2^-70 of its row's y^(p-1).
 template <int IP>
 __global__ void __launch_bounds__(256)
 lp_backward_prepare_kernel(const float* __restrict__ g, const float* __restrict__ y, int B, int Bp, int CO,
-                           float* __restrict__ gt, float* __restrict__ rt, float* __restrict__ ht, int* __restrict__ flag) {
+                           float* __restrict__ gt, float* __restrict__ rt, float* __restrict__ ht, int* __restrict__ flag, float pm1) {
     __shared__ float gs[32][33], ys[32][33];
     const int o0 = blockIdx.x * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     constexpr float LO = IP == 8 ? 0x1p-8f : 0x1p-3f, HI = IP == 8 ? 0x1p8f : 0x1p4f;
@@ -295,8 +326,11 @@ lp_backward_prepare_kernel(const float* __restrict__ g, const float* __restrict_
             if (o < CO) {
                 const float gv = gs[tx][ty + k], yv = ys[tx][ty + k];
                 const size_t a = (size_t)o * Bp + b;
-                gt[a] = gv;
-                rt[a] = yv > 0.f ? 1.f / yv : 0.f;
+                // r = fl(1 / y) enters every term as r^(p-1): its rounding, r * y - 1 (exact as one fma), is taken back out of g
+                const float rv = yv > 0.f ? 1.f / yv : 0.f;
+                const float off = pm1 * fmaf(rv, yv, -1.f);
+                rt[a] = rv;
+                gt[a] = fabsf(off) < 0.01f ? fmaf(gv, -off, gv) : gv;
                 if (IP == 8 || IP == 16) {
                     bad |= b < B && !(yv >= LO && yv <= HI);
                     float pw = yv, sq = yv;                   // y^(2^k - 1): 7 or 15
@@ -449,13 +483,14 @@ int lp_backward_both(const float* g, const float* x, const float* w, const float
     const dim3 pg((d.CO + 31) / 32, (unsigned)min((pl.Bp + 31) / 32, 64));
     const bool plain = p == 8.f || p == 16.f;
     if (plain && cudaMemsetAsync(flag, 0, sizeof(int), st) != cudaSuccess) return LINF_ERR_LAUNCH;
-    if (p == 8.f) lp_backward_prepare_kernel<8><<<pg, 256, 0, st>>>(g, y, d.R, pl.Bp, d.CO, gt, rt, ht, flag);
-    else if (p == 16.f) lp_backward_prepare_kernel<16><<<pg, 256, 0, st>>>(g, y, d.R, pl.Bp, d.CO, gt, rt, ht, flag);
-    else lp_backward_prepare_kernel<0><<<pg, 256, 0, st>>>(g, y, d.R, pl.Bp, d.CO, gt, rt, ht, flag);
+    if (p == 8.f) lp_backward_prepare_kernel<8><<<pg, 256, 0, st>>>(g, y, d.R, pl.Bp, d.CO, gt, rt, ht, flag, p - 1.f);
+    else if (p == 16.f) lp_backward_prepare_kernel<16><<<pg, 256, 0, st>>>(g, y, d.R, pl.Bp, d.CO, gt, rt, ht, flag, p - 1.f);
+    else lp_backward_prepare_kernel<0><<<pg, 256, 0, st>>>(g, y, d.R, pl.Bp, d.CO, gt, rt, ht, flag, p - 1.f);
     int rc = launch_status();
     if (rc) return rc;
     if (p == 8.f) rc = launch_ip<8>(P, (int)grid, pl.warps, al, dox, dow, st);
     else if (p == 16.f) rc = launch_ip<16>(P, (int)grid, pl.warps, al, dox, dow, st);
+    else if (p == 64.f) rc = launch_ip<64>(P, (int)grid, pl.warps, al, dox, dow, st);
     else if (P.q.m < 32) rc = launch_ip<-5>(P, (int)grid, pl.warps, al, dox, dow, st);
     else rc = launch_ip<-10>(P, (int)grid, pl.warps, al, dox, dow, st);
     if (rc) return rc;

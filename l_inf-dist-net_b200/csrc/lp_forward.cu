@@ -8,9 +8,10 @@
 // not needed:
 //   p = 8, 16          no scale at all.  Sums in [2^-64, 2^120] are kept: nothing overflowed, and a
 //                      difference whose power underflows is below 2^-60 of the sum.
-//   other p <= 80      one scale per output, from the largest of its first 32 (p > 32: 64) differences times 1.5, which is about where the
-//                      maximum of a long row lies (the closer to it, the smaller the exponents and their rounding).  Kept by the same rule:
-//                      the maximum of the row may be 5 times the sample's at p = 64, 4 times at 80, 20 times at 32.
+//   other p <= 80      one scale per output: the largest difference of the first eighth of its row (at least 64 terms) times 1.125, which is
+//                      about where the maximum of the whole row lies (the closer to it, the smaller the logarithms and their rounding: with
+//                      32 terms the distance itself was 1.3 times less exact).  Kept by the same rule: the maximum of the row may be 4 times
+//                      the sample's at p = 64, 3 times at 80, 15 times at 32.
 //   p > 80, or a sum outside the range (also: NaN, infinities, a row of zeros)
 //                      the literal rule: M = max_i |x - w| first, then sum (|x - w| / M)^p, y = M * sum^(1/p).  p > 80 gets M
 //                      from the value-only inf-dist kernel, a tile with a sum outside the range works it out itself.
@@ -39,8 +40,8 @@ __device__ __forceinline__ u64 pack2(float a, float b) { u64 r; asm("mov.b64 %0,
 __device__ __forceinline__ float lg2_approx(float a) { float r; asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a)); return r; }
 __device__ __forceinline__ float ex2_approx(float a) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a)); return r; }
 
-// 2^e for a pair on the FP32 pipe: e = n + f with the nearest integer n (the usual addition of 1.5 * 2^23), 2^f by the degree-5
-// interpolation of 2^f at the Chebyshev nodes of [-1/2, 1/2] (relative error in fp32 at most 2.2e-7, as ex2.approx), n added to the
+// 2^e for a pair on the FP32 pipe: e = n + f with the nearest integer n (the usual addition of 1.5 * 2^23), 2^f by the degree-6
+// interpolation of 2^f at the Chebyshev nodes of [-1/2, 1/2] (relative error in fp32 at most 8e-8; degree 5: 2.2e-7), n added to the
 // exponent.  e is held within [-125, 127] (a NaN stays one): below, the term is lost against a sum of at least 2^-64; above, the sum
 // ends outside the accepted range.
 __device__ __forceinline__ float clamp_exp(float e) {
@@ -55,12 +56,13 @@ __device__ __forceinline__ u64 ex2_poly2(u64 e) {
     const u64 c = pack2(clamp_exp(e0), clamp_exp(e1));
     const u64 z = add2(c, pack2(12582912.f, 12582912.f));
     const u64 f = sub_f32x2(c, sub_f32x2(z, pack2(12582912.f, 12582912.f)));
-    u64 r = pack2(1.339086331e-03f, 1.339086331e-03f);
-    r = fma2(r, f, pack2(9.676031768e-03f, 9.676031768e-03f));
-    r = fma2(r, f, pack2(5.550356954e-02f, 5.550356954e-02f));
-    r = fma2(r, f, pack2(2.402210683e-01f, 2.402210683e-01f));
+    u64 r = pack2(1.546144485e-04f, 1.546144485e-04f);
+    r = fma2(r, f, pack2(1.340042800e-03f, 1.340042800e-03f));
+    r = fma2(r, f, pack2(9.618056938e-03f, 9.618056938e-03f));
+    r = fma2(r, f, pack2(5.550327152e-02f, 5.550327152e-02f));
+    r = fma2(r, f, pack2(2.402265072e-01f, 2.402265072e-01f));
     r = fma2(r, f, pack2(6.931471825e-01f, 6.931471825e-01f));
-    r = fma2(r, f, pack2(1.000000119e+00f, 1.000000119e+00f));
+    r = fma2(r, f, pack2(1.f, 1.f));
     float r0, r1, z0, z1;
     unpack_f32x2(r, r0, r1);
     unpack_f32x2(z, z0, z1);
@@ -86,7 +88,7 @@ __device__ __forceinline__ float pow_ct(float a) {
 constexpr int TM = 64, NT = 128, BK = 16, LDK = BK + 4, STAGES = 3;
 constexpr float kSumLow = 0x1p-64f, kSumHigh = 0x1p120f;
 constexpr float kSampledP = 80.f;
-constexpr float kLower = 2.f / 3.f;
+constexpr float kLower = 1.f / 1.125f;
 
 struct FwdParams {
     const float* x; const float* w; float* y;
@@ -298,7 +300,7 @@ int lp_forward_dense(const float* x, const float* w, const Dims& d, float* y, fl
     P.x = x; P.w = w; P.y = y;
     P.B = d.R; P.COg = d.COg; P.CIg = d.CIg; P.G = d.G; P.CI = d.CI; P.CO = d.CO;
     P.p = p; P.inv_p = 1.f / p;
-    P.sample = p > 32.f ? 4 : 2;
+    P.sample = max(4, (d.CIg + 8 * BK - 1) / (8 * BK));
     P.have_max = lp_forward_wants_max(p) ? 1 : 0;
     const bool al = (d.CIg & 3) == 0 && aligned16(x) && aligned16(w);
     if (p == 8.f) return launch_fwd_ip<8>(P, (int)grid, narrow, al, st);
