@@ -129,7 +129,7 @@ int inf_forward(const float* x, const float* w, const Dims& d, float* y, int* po
                 const int* only_if = nullptr);
 size_t inf_forward_workspace(const Dims& d);
 // lists of large entries (inf_prune.cu) with the dense kernels behind
-bool inf_prune_ok(const Dims& d);
+bool inf_prune_ok(const Dims& d, bool bound);
 size_t inf_prune_workspace(const Dims& d, bool bound);
 int inf_prune(const float* xl, const float* xu, const float* w, const Dims& d, float* y0, int* pos, float* y1, bool bound,
               void* ws, cudaStream_t st, const Post& post, float dense_speed, const int** only_if);

@@ -19,8 +19,8 @@
 //
 // Bound: shared-memory gathers (a random 16-byte load of a warp takes about 10 cycles for 4 x 32 terms) and the 8-byte list entries
 // from L2.  How many entries there are depends on the data.  Dout = Din = 5120, B = 512: x uniform in [0,1) or activations of a
-// distance net, w ~ N(0,1): 20-45 of 5120; x and w ~ N(0,1): 240.  A gathered term costs about as much as six terms of the dense kernel,
-// hence kGatherCost.
+// distance net, w ~ N(0,1): 20-45 of 5120; x and w ~ N(0,1): 240.  A gathered term costs as much as eight terms of the
+// dense kernel (bounds: five), which sets `budget`.
 #include "common.cuh"
 
 namespace linf {
@@ -552,13 +552,17 @@ int run_pruned(const PruneParams& p, bool vec, cudaStream_t st) {
 
 }  // namespace
 
-// Which calls are worth the attempt: dense layers with long rows and enough outputs that five extra launches are small.
-bool inf_prune_ok(const Dims& d) {
+// Which calls are worth the attempt: dense layers with long rows, and enough work that the sample, the lists and five launches (about
+// 30 us) are small against the full scan.  Measured, us, full scan / lists, B = 512, x = 0.25 * normal: 1024 x 1024 forward 63 / 60, bounds 122 / 77;
+// 784 x 5120 (x uniform) forward 176 / 107.  Data that turn out not to suit cost 25 us on top of the scan.  The kernels for rows that are no
+// multiple of four floats are three times slower, so that the line lies lower there (203 x 1027 x 1333, normal: 153 / 67).
+bool inf_prune_ok(const Dims& d, bool bound) {
+    const double least = (d.CIg & 3) != 0 ? 1.5e8 : bound ? 5e8 : 1.5e9;
     return d.HW == 1 && d.CIg >= 256 && d.CIg <= kMaxK && d.COg >= 64 && d.R >= 64 &&
-           (double)d.R * d.CO * d.CIg >= 1.5e8 && (long long)d.R * d.G + d.CO <= 131072;
+           (double)d.R * d.CO * d.CIg >= least && (long long)d.R * d.G + d.CO <= 131072;
 }
 
-size_t inf_prune_workspace(const Dims& d, bool bound) { return inf_prune_ok(d) ? prune_sizes(d, bound).total : 0; }
+size_t inf_prune_workspace(const Dims& d, bool bound) { return inf_prune_ok(d, bound) ? prune_sizes(d, bound).total : 0; }
 
 // The list pass over a workspace of inf_prune_workspace bytes.  *only_if receives the device flag under which the dense kernel must
 // run behind it.  dense_speed: terms per second of the kernel behind, relative to the tiled ones.
@@ -576,8 +580,9 @@ int inf_prune(const float* xl, const float* xu, const float* w, const Dims& d, f
     p.fail = reinterpret_cast<int*>(base + s.fail); p.fail_cap = s.fail_cap;
     p.slots = s.slots;
     p.vec = (d.COg & 3) == 0 && aligned16(y0) && (pos == nullptr || aligned16(pos));
-    constexpr float kGatherCost = 6.f;
-    p.budget = 0.85f * d.CIg / (kGatherCost * dense_speed);
+    // time of a gathered term against one of the tiled kernels (B = 512, Din = Dout = 5120: 1.6 / 0.18 us per entry and input, bounds 2.2 / 0.45)
+    const float gather_cost = bound ? 5.f : 8.5f;
+    p.budget = 0.9f * d.CIg / (gather_cost * dense_speed);
     p.post = post;
     *only_if = &p.head->dense;
     const bool vec = (d.CIg & 3) == 0 && aligned16(xl) && aligned16(xu) && aligned16(w);

@@ -5,16 +5,16 @@
 //
 // A term needs a scale only so that its power stays within the range of a float, and any scale does: the sum is divided
 // by the same factor in the end.  So the maximum max_i |x - w|, which costs a pass of its own over all terms, is
-// not needed:
+// not needed for an integer p whose powers are products:
 //   p = 8, 16          no scale at all.  Sums in [2^-64, 2^120] are kept: nothing overflowed, and a
 //                      difference whose power underflows is below 2^-60 of the sum.
-//   other p <= 80      one scale per output: the largest difference of the first eighth of its row (at least 64 terms) times 1.125, which is
-//                      about where the maximum of the whole row lies (the closer to it, the smaller the logarithms and their rounding: with
-//                      32 terms the distance itself was 1.3 times less exact).  Kept by the same rule: the maximum of the row may be 4 times
-//                      the sample's at p = 64, 3 times at 80, 15 times at 32.
-//   p > 80, or a sum outside the range (also: NaN, infinities, a row of zeros)
-//                      the literal rule: M = max_i |x - w| first, then sum (|x - w| / M)^p, y = M * sum^(1/p).  p > 80 gets M
-//                      from the value-only inf-dist kernel, a tile with a sum outside the range works it out itself.
+//   p = 64             one scale per output: the largest difference of the first eighth of its row (at least 64 terms) times 1.125.
+//                      Kept by the same rule: the maximum of the row may be 4 times the sample's.
+//   other p, or a sum outside the range (also: NaN, infinities, a row of zeros)
+//                      the literal rule: M = max_i |x - w| first, then sum (|x - w| / M)^p, y = M * sum^(1/p).  With powers taken through
+//                      log2 the largest terms then enter exactly (their logarithm is 0); with a sampled scale y was 1.2 to 1.5 times
+//                      less exact.  A run-time p gets M from the value-only inf-dist kernel, a tile with a sum outside the range
+//                      works it out itself.
 // 64 x 64 (or 64 x 48) output tile per CTA of 128 threads, 8 x 4 (8 x 3) outputs per thread, operand tiles through a ring of
 // three cp.async stages; two neighbouring terms of an output sit in one register pair, so subtraction,
 // scale and squarings are packed (f32x2).
@@ -23,7 +23,7 @@
 // Run-time p: half of the exp2 run as a polynomial on the FP32 pipe (4 lg2 + 2 ex2 of the special-function unit for 4 terms =
 // 12 cycles per term and scheduler; all on the unit: 16).
 // Measured on one B200, us, maximum pass + literal rule -> here: B = 512, Din = Dout = 5120: p = 8: 3069 -> 1870,
-// 16: 3466 -> 2254, 64: 4230 -> 3468, 23.7: 7129 -> 5279; B = 203, Din = 1027, Dout = 1333 (generic kernels before), p = 8: 683 -> 117.
+// 16: 3466 -> 2254, 64: 4230 -> 3570, 23.7: 7129 -> RT; B = 203, Din = 1027, Dout = 1333 (generic kernels before), p = 8: 683 -> 117.
 #include <math.h>
 
 #include "common.cuh"
@@ -42,12 +42,10 @@ __device__ __forceinline__ float ex2_approx(float a) { float r; asm("ex2.approx.
 
 // 2^e for a pair on the FP32 pipe: e = n + f with the nearest integer n (the usual addition of 1.5 * 2^23), 2^f by the degree-6
 // interpolation of 2^f at the Chebyshev nodes of [-1/2, 1/2] (relative error in fp32 at most 8e-8; degree 5: 2.2e-7), n added to the
-// exponent.  e is held within [-125, 127] (a NaN stays one): below, the term is lost against a sum of at least 2^-64; above, the sum
-// ends outside the accepted range.
+// exponent.  e <= 0 up to rounding; below -125 the term is lost against a sum of at least 1 and e is held there (a NaN stays one).
 __device__ __forceinline__ float clamp_exp(float e) {
     float r;
     asm("max.NaN.f32 %0, %1, 0fC2FA0000;" : "=f"(r) : "f"(e));      // -125
-    asm("min.NaN.f32 %0, %1, 0f42FE0000;" : "=f"(r) : "f"(r));      // 127
     return r;
 }
 __device__ __forceinline__ u64 ex2_poly2(u64 e) {
@@ -66,8 +64,8 @@ __device__ __forceinline__ u64 ex2_poly2(u64 e) {
     float r0, r1, z0, z1;
     unpack_f32x2(r, r0, r1);
     unpack_f32x2(z, z0, z1);
-    // A NaN ends as the canonical NaN 0x7fffffff in r and z; the addition below then gives 0x7f7fffff, the largest float,
-    // and the sum leaves the accepted range: the literal rule answers.
+    // A NaN ends as the canonical NaN 0x7fffffff in r and z; the addition below then gives 0x7f7fffff, the largest float, which
+    // no sum of terms <= 1 reaches: the caller takes such a sum for a NaN.
     const float s0 = __int_as_float(__float_as_int(r0) + (__float_as_int(z0) << 23));
     const float s1 = __int_as_float(__float_as_int(r1) + (__float_as_int(z1) << 23));
     return pack2(s0, s1);
@@ -87,7 +85,6 @@ __device__ __forceinline__ float pow_ct(float a) {
 
 constexpr int TM = 64, NT = 128, BK = 16, LDK = BK + 4, STAGES = 3;
 constexpr float kSumLow = 0x1p-64f, kSumHigh = 0x1p120f;
-constexpr float kSampledP = 80.f;
 constexpr float kLower = 1.f / 1.125f;
 
 struct FwdParams {
@@ -95,7 +92,6 @@ struct FwdParams {
     int B, COg, CIg, G, CI, CO;
     float p, inv_p;
     int sample;                 // k-tiles the scale is taken from
-    int have_max;               // y holds max_i |x - w|
 };
 
 template <int ROWS, bool AL>
@@ -117,7 +113,7 @@ __device__ __forceinline__ void load_rows(float* dst, const float* __restrict__ 
     }
 }
 
-// IP: 8, 16, 64 at compile time (8 and 16 without a scale), 0: p at run time.  TJ: output columns per thread.
+// IP: 8, 16, 64 at compile time (8 and 16 without a scale), 0: p at run time, and y holds max_i |x - w| on entry.  TJ: output columns per thread.
 template <int IP, int TJ, bool AL>
 __global__ void __launch_bounds__(NT, 3)
 lp_forward_kernel(const FwdParams p) {
@@ -153,7 +149,7 @@ lp_forward_kernel(const FwdParams p) {
             const float* As = smem + rd * STAGE + row_off * LDK;
             const float* Bs = smem + rd * STAGE + (TM + col_off) * LDK;
             // two of the four k4 steps per trip (one where a term is long): the fully unrolled body runs into instruction fetch stalls
-#pragma unroll (IP == 8 ? 2 : 1)
+#pragma unroll (IP == 8 || IP == 16 ? 2 : 1)
             for (int k4 = 0; k4 < BK / 4; ++k4) {
                 ulonglong2 bf[TJ];
 #pragma unroll
@@ -174,7 +170,7 @@ lp_forward_kernel(const FwdParams p) {
     auto inside = [&](int e) { return m0 + row_off + 4 * (e / TJ) < p.B && n0 + col_off + 8 * (e % TJ) < p.COg; };
 
     float S[NO];
-    if (!p.have_max) {
+    if constexpr (IP > 0) {
         [[maybe_unused]] float r[PLAIN ? 1 : NO];
 #pragma unroll
         for (int e = 0; e < NO; ++e) S[e] = 0.f;
@@ -194,26 +190,13 @@ lp_forward_kernel(const FwdParams p) {
             });
 #pragma unroll
             for (int e = 0; e < NO; ++e) { r[e] = S[e] > 0.f ? kLower / S[e] : 0.f; S[e] = 0.f; }
-            const u64 pp = pack2(p.p, p.p);
             sweep(KT, [&](int e, u64 t01, u64 t23) {
                 const u64 rr = pack2(r[e], r[e]);
-                const u64 u01 = mul2(t01, rr), u23 = mul2(t23, rr);
                 float a, b;
-                if constexpr (IP > 0) {
-                    unpack_f32x2(pow2_ct<IP / 2>(u01), a, b);
-                    S[e] = fmaf(a, a, S[e]); S[e] = fmaf(b, b, S[e]);
-                    unpack_f32x2(pow2_ct<IP / 2>(u23), a, b);
-                    S[e] = fmaf(a, a, S[e]); S[e] = fmaf(b, b, S[e]);
-                } else {
-                    unpack_f32x2(u01, a, b);
-                    const u64 e01 = mul2(pack2(lg2_approx(fabsf(a)), lg2_approx(fabsf(b))), pp);
-                    unpack_f32x2(u23, a, b);
-                    const u64 e23 = mul2(pack2(lg2_approx(fabsf(a)), lg2_approx(fabsf(b))), pp);
-                    unpack_f32x2(e01, a, b);
-                    S[e] += ex2_approx(a); S[e] += ex2_approx(b);
-                    unpack_f32x2(ex2_poly2(e23), a, b);
-                    S[e] += a; S[e] += b;
-                }
+                unpack_f32x2(pow2_ct<(IP > 0 ? IP / 2 : 1)>(mul2(t01, rr)), a, b);
+                S[e] = fmaf(a, a, S[e]); S[e] = fmaf(b, b, S[e]);
+                unpack_f32x2(pow2_ct<(IP > 0 ? IP / 2 : 1)>(mul2(t23, rr)), a, b);
+                S[e] = fmaf(a, a, S[e]); S[e] = fmaf(b, b, S[e]);
             });
         }
         bool bad = false;
@@ -243,14 +226,25 @@ lp_forward_kernel(const FwdParams p) {
         rM[e] = M > 0.f ? 1.f / M : 0.f;
         S[e] = 0.f;
     }
+    [[maybe_unused]] const u64 pp = pack2(p.p, p.p);
     sweep(KT, [&](int e, u64 t01, u64 t23) {
-        float t[4];
-        unpack_f32x2(t01, t[0], t[1]); unpack_f32x2(t23, t[2], t[3]);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const float u = fabsf(t[q]) * rM[e];
-            if constexpr (IP > 0) { const float h = pow_ct<IP / 2>(u); S[e] = fmaf(h, h, S[e]); }
-            else S[e] += ex2_approx(p.p * lg2_approx(u));
+        const u64 rr = pack2(rM[e], rM[e]);
+        const u64 u01 = mul2(t01, rr), u23 = mul2(t23, rr);
+        float a, b;
+        if constexpr (IP > 0) {
+            unpack_f32x2(pow2_ct<IP / 2>(u01), a, b);
+            S[e] = fmaf(a, a, S[e]); S[e] = fmaf(b, b, S[e]);
+            unpack_f32x2(pow2_ct<IP / 2>(u23), a, b);
+            S[e] = fmaf(a, a, S[e]); S[e] = fmaf(b, b, S[e]);
+        } else {
+            unpack_f32x2(u01, a, b);
+            const u64 e01 = mul2(pack2(lg2_approx(fabsf(a)), lg2_approx(fabsf(b))), pp);
+            unpack_f32x2(u23, a, b);
+            const u64 e23 = mul2(pack2(lg2_approx(fabsf(a)), lg2_approx(fabsf(b))), pp);
+            unpack_f32x2(e01, a, b);
+            S[e] += ex2_approx(a); S[e] += ex2_approx(b);
+            unpack_f32x2(ex2_poly2(e23), a, b);
+            S[e] += a; S[e] += b;
         }
     });
 #pragma unroll
@@ -258,6 +252,7 @@ lp_forward_kernel(const FwdParams p) {
         if (inside(e)) {
             float* yo = out(e);
             const float M = *yo;
+            if (IP == 0 && S[e] > 1e30f) S[e] = __int_as_float(0x7fffffff);
             *yo = M > 0.f ? powf(S[e], p.inv_p) * M : 0.f;
         }
 }
@@ -279,7 +274,7 @@ int launch_fwd_ip(const FwdParams& P, int grid, bool narrow, bool al, cudaStream
 }  // namespace
 
 bool lp_forward_dense_ok(const Dims& d) { return d.HW == 1 && d.COg >= 32 && d.CIg >= 32; }
-bool lp_forward_wants_max(float p) { return p > kSampledP; }
+bool lp_forward_wants_max(float p) { return p != 8.f && p != 16.f && p != 64.f; }
 
 int lp_forward_width = 0;   // 0: tile width by shape; 1: 64 columns; 2: 48 columns (benchmarking knob)
 
@@ -301,7 +296,6 @@ int lp_forward_dense(const float* x, const float* w, const Dims& d, float* y, fl
     P.B = d.R; P.COg = d.COg; P.CIg = d.CIg; P.G = d.G; P.CI = d.CI; P.CO = d.CO;
     P.p = p; P.inv_p = 1.f / p;
     P.sample = max(4, (d.CIg + 8 * BK - 1) / (8 * BK));
-    P.have_max = lp_forward_wants_max(p) ? 1 : 0;
     const bool al = (d.CIg & 3) == 0 && aligned16(x) && aligned16(w);
     if (p == 8.f) return launch_fwd_ip<8>(P, (int)grid, narrow, al, st);
     if (p == 16.f) return launch_fwd_ip<16>(P, (int)grid, narrow, al, st);
