@@ -6,7 +6,7 @@ import subprocess
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "liblinfdist.so")
 CSRC = os.path.join(_HERE, "csrc")
-SOURCES = ["adamw.cu", "api.cu", "epilogue.cu", "sparse_exchange.cu", "inf_forward.cu", "inf_prune.cu", "inf_bound.cu", "inf_backward.cu", "inf_backward_accum.cu", "inf_backward_direct.cu", "lp.cu", "lp_tiled.cu", "lp_forward.cu", "lp_backward.cu", "no_alloc.cu", "skinny.cu"]
+SOURCES = ["adamw.cu", "api.cu", "epilogue.cu", "sparse_exchange.cu", "inf_forward.cu", "inf_prune.cu", "inf_bound.cu", "inf_backward.cu", "inf_backward_accum.cu", "inf_backward_direct.cu", "lp.cu", "lp_tiled.cu", "lp_forward.cu", "lp_backward.cu", "no_alloc.cu", "skinny.cu", "few_rows.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
               "--shared", "-Xcompiler", "-fPIC"]
 

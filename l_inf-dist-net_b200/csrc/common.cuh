@@ -170,6 +170,9 @@ int inf_backward_input_direct(const float* g, const int* pos, const Dims& d, flo
 extern int inf_backward_path;
 int inf_backward_ordered_both(const float* g, const int* pos, const Dims& d, float* gx, float* gw,
                               cudaStream_t st);
+// a handful of input rows (few_rows.cu)
+bool inf_few_rows_ok(const Dims& d);
+int inf_forward_few_rows(const float* x, const float* w, const Dims& d, float* y, int* pos, cudaStream_t st, const Post& post);
 // few output channels per group (skinny.cu)
 bool skinny_ok(const Dims& d, const void* a, const void* b, const void* c);
 int inf_forward_skinny(const float* x, const float* w, const Dims& d, float* y, int* pos, cudaStream_t st,

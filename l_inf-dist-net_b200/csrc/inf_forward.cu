@@ -670,6 +670,7 @@ int inf_forward_tma_gave_up() {
 int inf_forward_variant = 0;   // index into kVariants (benchmarking knob)
 int inf_forward_tail = 1;      // 1: a partial last wave runs as half-width tiles; 0: never
 int inf_forward_split = 0;     // 0: k-splitting by the rule of make_plan; 1: whenever scratch is given; 2: never
+int inf_forward_rows = 0;      // 0: a handful of input rows take few_rows.cu; 1: never (benchmarking knob)
 int inf_forward_windows = 0;   // 0: 16-term tracking windows for long rows; 1: 8-term windows always (benchmarking knob)
 int inf_forward_width = 0;     // 0: tile width by the rule of make_plan; 1: 64 columns always; 2: 48 wherever they exist
 
@@ -808,6 +809,7 @@ static int launch_tiled(const Kernels& k, const TiledParams& p, bool track, cuda
 
 int inf_forward(const float* x, const float* w, const Dims& d, float* y, int* pos,
                 void* ws, size_t ws_bytes, cudaStream_t st, const Post& post, const int* only_if) {
+    if (inf_few_rows_ok(d) && inf_forward_rows != 1) return inf_forward_few_rows(x, w, d, y, pos, st, post);
     if (!tiled_ok(x, w, d)) {
         if (only_if == nullptr && skinny_ok(d, x, w, nullptr)) return inf_forward_skinny(x, w, d, y, pos, st, post);
         dim3 grid((d.R + GT - 1) / GT, (d.COg + GT - 1) / GT, d.G);

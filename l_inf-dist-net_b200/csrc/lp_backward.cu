@@ -42,13 +42,6 @@ __device__ __forceinline__ u64 abs2(u64 a) { return a & 0x7fffffff7fffffffULL; }
 __device__ __forceinline__ float lg2_approx(float a) { float r; asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a)); return r; }
 __device__ __forceinline__ float ex2_approx(float a) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a)); return r; }
 
-__device__ __forceinline__ float clamp_unit(float a) {       // [-1, 1]; a NaN stays one
-    float r;
-    asm("max.NaN.f32 %0, %1, 0fBF800000;" : "=f"(r) : "f"(a));
-    asm("min.NaN.f32 %0, %1, 0f3F800000;" : "=f"(r) : "f"(r));
-    return r;
-}
-
 struct PowQ { int m; float f; };       // p - 2 = m + f
 
 // s <- s * |s|^(p-2) for N pairs.  IP > 0: p is that even integer (the sign comes with the odd power p - 1: 7 and 15 as
@@ -72,16 +65,6 @@ __device__ __forceinline__ void factors(u64 (&s)[N], const PowQ q) {
         }
     } else {
         constexpr int NB = -IP;
-        if (NB > 5) {
-            // |t| <= y, but fl(t * fl(1 / y)) may come out above 1; held at 1, the terms that make up a sum at a large p are exact
-            // (their powers otherwise carry hundreds of roundings)
-#pragma unroll
-            for (int e = 0; e < N; ++e) {
-                float a0, a1;
-                unpack_f32x2(s[e], a0, a1);
-                s[e] = pack2(clamp_unit(a0), clamp_unit(a1));
-            }
-        }
         u64 b[N], v[N];
 #pragma unroll
         for (int e = 0; e < N; ++e) { b[e] = s[e]; v[e] = s[e]; }
@@ -344,7 +327,6 @@ lp_backward_prepare_kernel(const float* __restrict__ g, const float* __restrict_
                 const float gv = gs[tx][ty + k], yv = ys[tx][ty + k];
                 const size_t a = (size_t)o * Bp + b;
                 // r = fl(1 / y) enters every term as r^(p-1): its rounding, r * y - 1 (exact as one fma), is taken back out of g
-                // (pm1 = p - 1, or 0 where the terms are held at 1)
                 const float rv = yv > 0.f ? 1.f / yv : 0.f;
                 const float off = pm1 * fmaf(rv, yv, -1.f);
                 rt[a] = rv;
@@ -503,7 +485,7 @@ int lp_backward_both(const float* g, const float* x, const float* w, const float
     if (plain && cudaMemsetAsync(flag, 0, sizeof(int), st) != cudaSuccess) return LINF_ERR_LAUNCH;
     if (p == 8.f) lp_backward_prepare_kernel<8><<<pg, 256, 0, st>>>(g, y, d.R, pl.Bp, d.CO, gt, rt, ht, flag, p - 1.f);
     else if (p == 16.f) lp_backward_prepare_kernel<16><<<pg, 256, 0, st>>>(g, y, d.R, pl.Bp, d.CO, gt, rt, ht, flag, p - 1.f);
-    else lp_backward_prepare_kernel<0><<<pg, 256, 0, st>>>(g, y, d.R, pl.Bp, d.CO, gt, rt, ht, flag, P.q.m < 32 || p == 64.f ? p - 1.f : 0.f);
+    else lp_backward_prepare_kernel<0><<<pg, 256, 0, st>>>(g, y, d.R, pl.Bp, d.CO, gt, rt, ht, flag, p - 1.f);
     int rc = launch_status();
     if (rc) return rc;
     if (p == 8.f) rc = launch_ip<8>(P, (int)grid, pl.warps, al, dox, dow, st);

@@ -23,7 +23,7 @@
 // Run-time p: half of the exp2 run as a polynomial on the FP32 pipe (4 lg2 + 2 ex2 of the special-function unit for 4 terms =
 // 12 cycles per term and scheduler; all on the unit: 16).
 // Measured on one B200, us, maximum pass + literal rule -> here: B = 512, Din = Dout = 5120: p = 8: 3069 -> 1870,
-// 16: 3466 -> 2254, 64: 4230 -> 3570, 23.7: 7129 -> RT; B = 203, Din = 1027, Dout = 1333 (generic kernels before), p = 8: 683 -> 117.
+// 16: 3466 -> 2254, 64: 4230 -> 3550, 23.7: 7129 -> 5980; B = 203, Din = 1027, Dout = 1333 (generic kernels before), p = 8: 683 -> 117.
 #include <math.h>
 
 #include "common.cuh"

@@ -46,7 +46,25 @@ def _require(t, name, dtype=torch.float32):
 
 
 def _stream():
-    return torch.cuda.current_stream().cuda_stream
+    """Raw handle of torch's current stream on the current device."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
+class _NoGuard:
+    def __enter__(self):
+        pass
+
+    def __exit__(self, *exc):
+        pass
+
+
+_no_guard = _NoGuard()
+
+
+def _on(device):
+    """torch.cuda.device(device), or nothing where that is the current device already (the usual case: a guard costs
+    about as much host time as a launch)."""
+    return _no_guard if device.index == torch._C._cuda_getDevice() else torch.cuda.device(device)
 
 
 def _workspace(device, nbytes):
@@ -100,7 +118,7 @@ class DistF(torch.autograd.Function):
         xk = _rows_view(x) if ctx.rows else x
         B, CO, CI, G, HW = _shape5(xk, weight, group)
         y = torch.empty(B, CO, HW, device=x.device, dtype=torch.float32)
-        with torch.cuda.device(x.device):
+        with _on(x.device):
             if math.isinf(p):
                 pos = torch.empty(B, CO, HW, device=x.device, dtype=torch.int32)
                 lists = lib.linf_inf_dist_forward_pruned_workspace_bytes(B, CO, CI, G, HW)
@@ -134,7 +152,7 @@ class DistF(torch.autograd.Function):
         _require(grad_output, "grad_output")
         need_x, need_w = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
         gx = gw = None
-        with torch.cuda.device(grad_output.device):
+        with _on(grad_output.device):
             if math.isinf(ctx.p):
                 x, weight, y, pos = ctx.saved_tensors
                 B, CO, CI, G, HW = _shape5(x, weight, ctx.group)
@@ -202,31 +220,35 @@ def _post_args(post):
     return (sub.data_ptr() if sub is not None else None, add.data_ptr() if add is not None else None, 1 if negate else 0)
 
 
+def _inf_post_values(x, weight, shape, sizes, post):
+    """Launches the value-only forward with its epilogue; sizes = (B, CO, CI, group, HW)."""
+    lib = _lib.load()
+    _require(x, "input"); _require(weight, "weight")
+    sub, add, neg = _post_args(post)
+    y = torch.empty(shape, device=x.device, dtype=torch.float32)
+    with _on(x.device):
+        lists = lib.linf_inf_dist_forward_pruned_workspace_bytes(*sizes)
+        if lists:
+            ws = torch.empty(lists, dtype=torch.uint8, device=x.device)
+            rc = lib.linf_inf_dist_forward_pruned(x.data_ptr(), weight.data_ptr(), *sizes, sub, add, neg,
+                                                  y.data_ptr(), None, ws.data_ptr(), lists, _stream())
+        else:
+            need = lib.linf_inf_dist_forward_workspace_bytes(*sizes)
+            ws = _workspace(x.device, need) if need else None
+            rc = lib.linf_inf_dist_forward_post(x.data_ptr(), weight.data_ptr(), *sizes, sub, add, neg,
+                                                y.data_ptr(), ws.data_ptr() if need else None, ws.numel() if need else 0, _stream())
+    _lib.check(rc, "inf_dist_forward_post")
+    return y
+
+
 @torch.no_grad()
 def inf_dist_post(input, weight, group, post, tag=None):
     """Value of an inf-dist layer with the per-channel epilogue (sub, add, negate) folded into the
     kernel's store: ((y - sub[c]) + add[c]), negated if asked.  No arg-max is kept, so there is no
     gradient: the inference / certification path.  input [B, CI, HW], weight [CO, CI/group]."""
-    lib = _lib.load()
-    _require(input, "input"); _require(weight, "weight")
     assert weight.size(1) * group == input.size(1)
     B, CO, CI, G, HW = _shape5(input, weight, group)
-    y = torch.empty(B, CO, HW, device=input.device, dtype=torch.float32)
-    sub, add, neg = _post_args(post)
-    with torch.cuda.device(input.device):
-        lists = lib.linf_inf_dist_forward_pruned_workspace_bytes(B, CO, CI, G, HW)
-        if lists:
-            ws = torch.empty(lists, dtype=torch.uint8, device=input.device)
-            rc = lib.linf_inf_dist_forward_pruned(input.data_ptr(), weight.data_ptr(), B, CO, CI, G, HW, sub, add, neg,
-                                                  y.data_ptr(), None, ws.data_ptr(), lists, _stream())
-            _lib.check(rc, "inf_dist_forward_pruned")
-            return y
-        need = lib.linf_inf_dist_forward_workspace_bytes(B, CO, CI, G, HW)
-        ws = _workspace(input.device, need) if need else None
-        rc = lib.linf_inf_dist_forward_post(input.data_ptr(), weight.data_ptr(), B, CO, CI, G, HW, sub, add, neg,
-                                            y.data_ptr(), ws.data_ptr() if need else None, ws.numel() if need else 0, _stream())
-    _lib.check(rc, "inf_dist_forward_post")
-    return y
+    return _inf_post_values(input, weight, (B, CO, HW), (B, CO, CI, G, HW), post)
 
 
 def inf_dist_bound(input_lower, input_upper, weight, group, use_custom_cuda_func=True, tag=None, post=None):
@@ -247,7 +269,7 @@ def inf_dist_bound(input_lower, input_upper, weight, group, use_custom_cuda_func
     B, CO, CI, G, HW = _shape5(input_lower, weight, group)
     lo = torch.empty(B, CO, HW, device=input_lower.device, dtype=torch.float32)
     up = torch.empty_like(lo)
-    with torch.cuda.device(input_lower.device):
+    with _on(input_lower.device):
         sub, add, neg = _post_args(post)
         lists = lib.linf_inf_dist_bound_pruned_workspace_bytes(B, CO, CI, G, HW)
         if lists:
@@ -273,7 +295,7 @@ class MeanShiftF(torch.autograd.Function):
         lib = _lib.load()
         _require(x, "input")
         out = torch.empty_like(x)
-        with torch.cuda.device(x.device):
+        with _on(x.device):
             rc = lib.linf_mean_shift(x.data_ptr(), x.size(0), x.size(1),
                                      running_mean.data_ptr() if running_mean is not None else None,
                                      float(momentum), out.data_ptr(), None, _stream())
@@ -285,7 +307,7 @@ class MeanShiftF(torch.autograd.Function):
         lib = _lib.load()
         g = grad_output.contiguous()
         out = torch.empty_like(g)
-        with torch.cuda.device(g.device):
+        with _on(g.device):
             rc = lib.linf_mean_shift(g.data_ptr(), g.size(0), g.size(1), None, 0.0, out.data_ptr(), None, _stream())
         _lib.check(rc, "mean_shift backward")
         return out, None, None
@@ -455,6 +477,14 @@ class NormDist(NormDistConv):
                          identity_init=identity_init)
 
     def forward(self, x, lower=None, upper=None, negate=False):
+        if (lower is None or upper is None) and x.dim() == 2:
+            post = self._fused_post(negate)
+            if post is not None and not (torch.is_grad_enabled() and (x.requires_grad or self.weight.requires_grad)):
+                # inference: the same call as below without its views (they cost more host time than the launch)
+                B, CI = x.shape
+                CO = self.weight.size(0)
+                assert self.weight.size(1) * self.group == CI
+                return _inf_post_values(x.contiguous(), self.weight.detach(), (B, CO), (B, CO, CI, self.group, 1), post), None, None
         as4d = lambda t: None if t is None else t.reshape(t.size(0), t.size(1), 1, 1)
         y, lo, up = super().forward(as4d(x), as4d(lower), as4d(upper), negate=negate)
         flat = lambda t: None if t is None else t.reshape(t.size(0), t.size(1))
