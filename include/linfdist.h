@@ -274,6 +274,16 @@ int linf_inf_dist_bound_pruned(const float* input_lower, const float* input_uppe
                                float* output_lower, float* output_upper,
                                void* workspace, size_t workspace_bytes, void* stream);
 
+/*
+ * Patches of a k x k convolution over input [B, C, H, W] as rows [B * Ho * Wo, C * k * k] of a dense layer (channel-major, zero
+ * outside the image; the column order of the reference's unfold, model/norm_dist.py:126-131), and the adjoint: grad_input [B, C, H, W],
+ * fully overwritten, every cell summed over the output rows, then columns, ascending.
+ */
+int linf_unfold_rows(const float* input, int B, int C, int H, int W, int kernel_size, int dilation, int padding, int stride,
+                     float* rows, void* stream);
+int linf_fold_rows(const float* rows, int B, int C, int H, int W, int kernel_size, int dilation, int padding, int stride,
+                   float* grad_input, void* stream);
+
 /* ---------------------------------------------------------------------------------
  * optimiser step (next to the distance neuron on the training path)
  * --------------------------------------------------------------------------------- */

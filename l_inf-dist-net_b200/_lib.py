@@ -6,7 +6,7 @@ import subprocess
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "liblinfdist.so")
 CSRC = os.path.join(_HERE, "csrc")
-SOURCES = ["adamw.cu", "api.cu", "epilogue.cu", "sparse_exchange.cu", "inf_forward.cu", "inf_prune.cu", "inf_bound.cu", "inf_backward.cu", "inf_backward_accum.cu", "inf_backward_direct.cu", "lp.cu", "lp_tiled.cu", "lp_forward.cu", "lp_backward.cu", "no_alloc.cu", "skinny.cu", "few_rows.cu"]
+SOURCES = ["adamw.cu", "api.cu", "epilogue.cu", "sparse_exchange.cu", "inf_forward.cu", "inf_prune.cu", "inf_bound.cu", "inf_backward.cu", "inf_backward_accum.cu", "inf_backward_direct.cu", "lp.cu", "lp_tiled.cu", "lp_forward.cu", "lp_backward.cu", "no_alloc.cu", "skinny.cu", "few_rows.cu", "patches.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
               "--shared", "-Xcompiler", "-fPIC"]
 
@@ -40,6 +40,8 @@ _PROTOS = {
     "linf_norm_dist_forward": [_F, _F, _INT, _INT, _INT, _INT, _INT, _F, ctypes.c_float, _F],
     "linf_norm_dist_backward_input": [_F, _F, _F, _F, _INT, _INT, _INT, _INT, _INT, _F, ctypes.c_float, _F],
     "linf_norm_dist_backward_weight": [_F, _F, _F, _F, _INT, _INT, _INT, _INT, _INT, _F, ctypes.c_float, _F],
+    "linf_unfold_rows": [_F, _INT, _INT, _INT, _INT, _INT, _INT, _INT, _INT, _F, _F],
+    "linf_fold_rows": [_F, _INT, _INT, _INT, _INT, _INT, _INT, _INT, _INT, _F, _F],
     "linf_inf_dist_forward_pruned_workspace_bytes": [_INT, _INT, _INT, _INT, _INT],
     "linf_inf_dist_forward_pruned": [_F, _F, _INT, _INT, _INT, _INT, _INT, _F, _F, _INT, _F, _F, _F, ctypes.c_size_t, _F],
     "linf_inf_dist_bound_pruned_workspace_bytes": [_INT, _INT, _INT, _INT, _INT],

@@ -8,7 +8,7 @@ import torch
 from torch.optim import Optimizer
 
 from . import _lib
-from .norm_dist import get_p_norm
+from .norm_dist import _on, _stream, get_p_norm
 
 
 class AdamW(Optimizer):
@@ -86,11 +86,11 @@ class AdamW(Optimizer):
         if not (p.is_cuda and p.dtype == torch.float32 and p.is_contiguous() and grad_rows.is_contiguous()
                 and grad_rows.dtype == torch.float32 and cols <= 51200):
             raise RuntimeError("step_rows needs a contiguous fp32 CUDA parameter with rows of at most 51200 entries")
-        with torch.cuda.device(p.device):
+        with _on(p.device):
             rc = _lib.load().linf_adamw_step(
                 p.data_ptr() + row0 * cols * 4, grad_rows.data_ptr(), st["exp_avg"].data_ptr(), st["exp_avg_sq"].data_ptr(),
                 nrows, cols, -1.0 if p_norm is None else float(p_norm), group["lr"], beta1, beta2,
-                group["eps"], group["weight_decay"], st["step"], torch.cuda.current_stream().cuda_stream)
+                group["eps"], group["weight_decay"], st["step"], _stream())
         _lib.check(rc, "adamw_step")
 
     def _update(self, p, group):
@@ -107,11 +107,11 @@ class AdamW(Optimizer):
         if self._fused_ok(p):
             # CUDA tensors: one fused launch per tensor (csrc/adamw.cu)
             rows = p.size(0)
-            with torch.cuda.device(p.device):
+            with _on(p.device):
                 rc = _lib.load().linf_adamw_step(
                     p.data_ptr(), p.grad.data_ptr(), state["exp_avg"].data_ptr(), state["exp_avg_sq"].data_ptr(),
                     rows, p.numel() // rows, -1.0 if p_norm is None else float(p_norm), group["lr"], beta1, beta2,
-                    group["eps"], group["weight_decay"], state["step"], torch.cuda.current_stream().cuda_stream)
+                    group["eps"], group["weight_decay"], state["step"], _stream())
             _lib.check(rc, "adamw_step")
             return
         self._decay(p, p_norm, group["lr"] * group["weight_decay"], group["eps"])

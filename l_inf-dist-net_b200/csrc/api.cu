@@ -348,4 +348,16 @@ int linf_inf_dist_bound_pruned(const float* input_lower, const float* input_uppe
                             as_stream(stream), post);
 }
 
+int linf_unfold_rows(const float* input, int B, int C, int H, int W, int kernel_size, int dilation, int padding, int stride,
+                     float* rows, void* stream) {
+    if (!input || !rows) return LINF_ERR_NULL;
+    return unfold_rows(input, B, C, H, W, kernel_size, dilation, padding, stride, rows, as_stream(stream));
+}
+
+int linf_fold_rows(const float* rows, int B, int C, int H, int W, int kernel_size, int dilation, int padding, int stride,
+                   float* grad_input, void* stream) {
+    if (!rows || !grad_input) return LINF_ERR_NULL;
+    return fold_rows(rows, B, C, H, W, kernel_size, dilation, padding, stride, grad_input, as_stream(stream));
+}
+
 }  // extern "C"

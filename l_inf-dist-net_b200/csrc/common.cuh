@@ -170,6 +170,9 @@ int inf_backward_input_direct(const float* g, const int* pos, const Dims& d, flo
 extern int inf_backward_path;
 int inf_backward_ordered_both(const float* g, const int* pos, const Dims& d, float* gx, float* gw,
                               cudaStream_t st);
+// patches of a convolution-shaped layer as rows, and back (patches.cu)
+int unfold_rows(const float* x, int B, int C, int H, int W, int k, int dil, int pad, int stride, float* rows, cudaStream_t st);
+int fold_rows(const float* rows, int B, int C, int H, int W, int k, int dil, int pad, int stride, float* gx, cudaStream_t st);
 // a handful of input rows (few_rows.cu)
 bool inf_few_rows_ok(const Dims& d);
 int inf_forward_few_rows(const float* x, const float* w, const Dims& d, float* y, int* pos, cudaStream_t st, const Post& post);

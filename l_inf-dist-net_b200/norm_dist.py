@@ -286,6 +286,35 @@ def inf_dist_bound(input_lower, input_upper, weight, group, use_custom_cuda_func
     return lo, up
 
 
+class PatchRowsF(torch.autograd.Function):
+    """Patches of x [B, C, H, W] as rows [B * L, C * k * k, 1] of a dense layer, in one launch (csrc/patches.cu); the backward adds
+    them up again.  Same values as F.unfold and a permuting copy."""
+
+    @staticmethod
+    def forward(ctx, x, k, dilation, padding, stride, L):
+        lib = _lib.load()
+        x = x.contiguous()
+        _require(x, "input")
+        B, C, H, W = x.shape
+        ctx.geometry = (B, C, H, W, k, dilation, padding, stride)
+        rows = torch.empty(B * L, C * k * k, 1, device=x.device, dtype=torch.float32)
+        with _on(x.device):
+            rc = lib.linf_unfold_rows(x.data_ptr(), *ctx.geometry, rows.data_ptr(), _stream())
+        _lib.check(rc, "unfold_rows")
+        return rows
+
+    @staticmethod
+    def backward(ctx, grad_rows):
+        lib = _lib.load()
+        g = grad_rows.contiguous()
+        _require(g, "grad_rows")
+        gx = torch.empty(ctx.geometry[:4], device=g.device, dtype=torch.float32)
+        with _on(g.device):
+            rc = lib.linf_fold_rows(g.data_ptr(), *ctx.geometry, gx.data_ptr(), _stream())
+        _lib.check(rc, "fold_rows")
+        return gx, None, None, None, None, None
+
+
 class MeanShiftF(torch.autograd.Function):
     """x[B, C] -> x - column mean(x), with the exponential running mean updated in the same launch
     (csrc/epilogue.cu).  The backward is the same map applied to the gradient."""
@@ -402,6 +431,13 @@ class NormDistConv(nn.Module):
             return t.reshape(t.size(0), t.size(1), -1)      # a dense layer needs no unfold copy
         return F.unfold(t, self.kernel_size, self.dilation, self.padding, self.stride)
 
+    def _rows_from_patches(self, x, ho, wo):
+        """Whether DistF would run this call as a dense layer over the patches (`_dense_route`), and x is what the unfold kernel takes."""
+        return (x.is_cuda and x.dtype == torch.float32 and x.dim() == 4 and x.numel() > 0 and ho > 0 and wo > 0 and ho * wo > 1
+                and not (self.kernel_size == 1 and self.stride == 1 and self.padding == 0)
+                and self.weight[0].numel() % 4 == 0 and self.weight.size(0) // self.group >= 32
+                and x.size(0) * ho * wo * x.size(1) * self.kernel_size ** 2 < 2 ** 31)
+
     def _post(self, t):
         if self.normalize is not None:
             t = self.normalize(t)
@@ -426,6 +462,12 @@ class NormDistConv(nn.Module):
         ho = (h + 2 * self.padding - self.dilation * (self.kernel_size - 1) - 1) // self.stride + 1
         wo = (w + 2 * self.padding - self.dilation * (self.kernel_size - 1) - 1) // self.stride + 1
         weight = self.weight.view(self.weight.size(0), -1)
+        if (lower is None or upper is None) and self._rows_from_patches(x, ho, wo):
+            # the patches go straight into the rows of a dense layer (DistF would copy them there)
+            rows = PatchRowsF.apply(x, self.kernel_size, self.dilation, self.padding, self.stride, ho * wo)
+            y = norm_dist(rows, weight, self.group, p=self.p, tag=self.tag)
+            y = self._post(y.view(x.size(0), ho, wo, -1).permute(0, 3, 1, 2).contiguous())
+            return (-y if negate else y), None, None
         cols = self._patches(x)
         post = self._fused_post(negate)
         if post is not None and _dense_route(cols, weight, self.group):
