@@ -29,7 +29,7 @@ namespace {
 constexpr unsigned FULL = 0xffffffffu;
 constexpr int kBins = 4096, kBinShift = 19;     // bins of |v|: exponent and four bits of the mantissa
 constexpr int kSampleCtas = 128;
-constexpr int kMaxList = 256;                   // slots per row
+constexpr int kMaxList = 512;                   // slots per row (the thresholds aim at 0.6 of them at most)
 constexpr int kMaxK = 14000;                    // 16 bytes each in shared memory
 
 struct Head {                                   // zeroed before every call
