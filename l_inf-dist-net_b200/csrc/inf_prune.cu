@@ -61,6 +61,8 @@ struct PruneParams {
 __device__ __forceinline__ float pinf() { return __int_as_float(0x7f800000); }
 __device__ __forceinline__ int signed_at(float t, int at) { return at | (t < 0.f ? (int)0x80000000 : 0); }
 
+__device__ __forceinline__ float4 ld4(const float* a) { return __ldg(reinterpret_cast<const float4*>(a)); }
+
 // one term of an interval bound: U = max of the far ends, m = min (the lower bound is -m, at least 0)
 __device__ __forceinline__ void bound_term(float lo, float up, float w, float& m, float& U) {
     const float a = w - lo, b = up - w;
@@ -68,7 +70,7 @@ __device__ __forceinline__ void bound_term(float lo, float up, float w, float& m
     m = fminf(m, fminf(a, b));
 }
 
-template <bool BOUND>
+template <bool BOUND, bool VEC>
 __global__ void __launch_bounds__(256)
 sample_kernel(const PruneParams p) {
     __shared__ __align__(16) int hx[kBins], hw[kBins];
@@ -89,16 +91,35 @@ sample_kernel(const PruneParams p) {
         wr[q] = p.w + ((size_t)g * p.N + o) * p.K;
         v[q] = 0.f;
     }
-#pragma unroll 2
-    for (int k = tid; k < p.K; k += 256) {
-        const float a = __ldg(p.xl + xa + k), b = BOUND ? __ldg(p.xu + xa + k) : a;
-        float wv[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) wv[q] = __ldg(wr[q] + k);
+    auto look = [&](float a, float b, const float (&wv)[8]) {
 #pragma unroll
         for (int q = 0; q < 8; ++q) v[q] = BOUND ? max3(v[q], a - wv[q], wv[q] - b) : fmaxf(v[q], fabsf(a - wv[q]));
         atomicAdd(&hx[__float_as_int(BOUND ? fmaxf(fabsf(a), fabsf(b)) : fabsf(a)) >> kBinShift], 1);
         atomicAdd(&hw[__float_as_int(fabsf(wv[0])) >> kBinShift], 1);
+    };
+    if (VEC) {
+        for (int k = 4 * tid; k < p.K; k += 1024) {
+            const float4 a = ld4(p.xl + xa + k), b = BOUND ? ld4(p.xu + xa + k) : a;
+            float4 f[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) f[q] = ld4(wr[q] + k);
+            float wv[8];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+#pragma unroll
+                for (int q = 0; q < 8; ++q) wv[q] = c == 0 ? f[q].x : c == 1 ? f[q].y : c == 2 ? f[q].z : f[q].w;
+                look(c == 0 ? a.x : c == 1 ? a.y : c == 2 ? a.z : a.w, c == 0 ? b.x : c == 1 ? b.y : c == 2 ? b.z : b.w, wv);
+            }
+        }
+    } else {
+#pragma unroll 2
+        for (int k = tid; k < p.K; k += 256) {
+            const float a = __ldg(p.xl + xa + k), b = BOUND ? __ldg(p.xu + xa + k) : a;
+            float wv[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) wv[q] = __ldg(wr[q] + k);
+            look(a, b, wv);
+        }
     }
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
@@ -426,7 +447,7 @@ gather_kernel(const PruneParams p, int blocks_a, int splits) {
 
 // The outputs that did not pass: a full scan by a CTA of four warps each (by one warp, the 160 dependent loads of a row of 5120 made
 // this the longest kernel of a layer with a few hundred such outputs: 40 us).
-template <bool BOUND, bool TRACK>
+template <bool BOUND, bool TRACK, bool VEC>
 __global__ void __launch_bounds__(128)
 fail_kernel(const PruneParams p) {
     __shared__ float s_t[4], s_u[4];
@@ -444,13 +465,25 @@ fail_kernel(const PruneParams p) {
         const size_t xa = (size_t)r * p.CI + (size_t)g * p.K;
         const float* wr = p.w + (size_t)c * p.K;
         float t = 0.f, u = 0.f; int at = 0;             // forward: signed difference, index; bounds: -lower, upper
-#pragma unroll 8
-        for (int k = tid; k < p.K; k += 128) {
+        auto take = [&](float lo, float up, float w, int k) {
             if (BOUND) {
-                bound_term(__ldg(p.xl + xa + k), __ldg(p.xu + xa + k), __ldg(wr + k), t, u);
+                bound_term(lo, up, w, t, u);
             } else {
-                const float d = __ldg(p.xl + xa + k) - __ldg(wr + k);
+                const float d = lo - w;
                 if (fabsf(d) > fabsf(t)) { t = d; at = k; }
+            }
+        };
+        if (VEC) {
+#pragma unroll 4
+            for (int k = 4 * tid; k < p.K; k += 512) {
+                const float4 a = ld4(p.xl + xa + k), b = BOUND ? ld4(p.xu + xa + k) : a, w = ld4(wr + k);
+                take(a.x, b.x, w.x, k); take(a.y, b.y, w.y, k + 1); take(a.z, b.z, w.z, k + 2); take(a.w, b.w, w.w, k + 3);
+            }
+        } else {
+#pragma unroll 8
+            for (int k = tid; k < p.K; k += 128) {
+                const float a = __ldg(p.xl + xa + k);
+                take(a, BOUND ? __ldg(p.xu + xa + k) : a, __ldg(wr + k), k);
             }
         }
         // larger |t| first, then the lower index
@@ -521,7 +554,7 @@ int launch_gather_as(const PruneParams& p, cudaStream_t st) {
     if (splits > most) splits = most;
     if (splits < 1) splits = 1;
     auto kern = gather_kernel<BOUND, W_LISTS, TRACK, NQ>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return LINF_ERR_LAUNCH;
+    if (smem > 40 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return LINF_ERR_LAUNCH;
     kern<<<(unsigned)((long long)blocks * p.G * splits), threads, smem, st>>>(p, blocks, (int)splits);
     return launch_status();
 }
@@ -529,24 +562,31 @@ int launch_gather_as(const PruneParams& p, cudaStream_t st) {
 template <bool BOUND, bool W_LISTS, bool TRACK>
 int launch_gather(const PruneParams& p, cudaStream_t st) {
     const long long rows = (long long)(W_LISTS ? p.R * (BOUND ? 2 : 1) : p.N) * p.G;
-    const bool two = p.K <= kMaxK / 2 && rows * ((W_LISTS ? p.N : p.R) + 511) / 512 >= 8LL * 4 * sm_count();
+    // with at most 512 lanes a CTA cannot hold more than 16 warps: two CTAs of one array each then
+    const int nl = W_LISTS ? p.N : p.R;
+    const bool two = p.K <= kMaxK / 2 && (nl > 512 || p.K <= kMaxK / 4) && rows * ((W_LISTS ? p.N : p.R) + 511) / 512 >= 8LL * 4 * sm_count();
     return two ? launch_gather_as<BOUND, W_LISTS, TRACK, 2>(p, st) : launch_gather_as<BOUND, W_LISTS, TRACK, 1>(p, st);
 }
 
 template <bool BOUND, bool TRACK>
 int run_pruned(const PruneParams& p, bool vec, cudaStream_t st) {
     if (cudaMemsetAsync(p.head, 0, sizeof(Head) + 2 * kBins * sizeof(int), st) != cudaSuccess) return LINF_ERR_LAUNCH;
-    sample_kernel<BOUND><<<kSampleCtas, 256, 0, st>>>(p);
     const int blocks = (p.R * p.G + p.CO + 7) / 8;
-    if (vec) list_kernel<BOUND, true><<<blocks, 256, 0, st>>>(p);
-    else list_kernel<BOUND, false><<<blocks, 256, 0, st>>>(p);
+    if (vec) {
+        sample_kernel<BOUND, true><<<kSampleCtas, 256, 0, st>>>(p);
+        list_kernel<BOUND, true><<<blocks, 256, 0, st>>>(p);
+    } else {
+        sample_kernel<BOUND, false><<<kSampleCtas, 256, 0, st>>>(p);
+        list_kernel<BOUND, false><<<blocks, 256, 0, st>>>(p);
+    }
     int rc = launch_status(2);
     if (rc) return rc;
     rc = launch_gather<BOUND, false, TRACK>(p, st);
     if (rc) return rc;
     rc = launch_gather<BOUND, true, TRACK>(p, st);
     if (rc) return rc;
-    fail_kernel<BOUND, TRACK><<<8 * sm_count(), 128, 0, st>>>(p);
+    if (vec) fail_kernel<BOUND, TRACK, true><<<8 * sm_count(), 128, 0, st>>>(p);
+    else fail_kernel<BOUND, TRACK, false><<<8 * sm_count(), 128, 0, st>>>(p);
     return launch_status();
 }
 

@@ -15,6 +15,28 @@ from .nets import MLP, MLPFeature, Model
 from .norm_dist import NormDistConv, get_p_norm, set_p_norm
 
 
+def _current_stream():
+    """torch.cuda.current_stream() without its look-up of the device (which costs more host time than the launch that follows;
+    a step asks some 25 times)."""
+    sid, index, kind = torch._C._cuda_getCurrentStream(torch._C._cuda_getDevice())
+    return torch.cuda.Stream(stream_id=sid, device_index=index, device_type=kind)
+
+
+class _use_stream:
+    """torch.cuda.stream(side) for a stream of the current device."""
+
+    def __init__(self, side):
+        self.side = side
+
+    def __enter__(self):
+        self.before = torch._C._cuda_getCurrentStream(self.side.device_index)
+        torch._C._cuda_setStream(stream_id=self.side.stream_id, device_index=self.side.device_index, device_type=self.side.device_type)
+
+    def __exit__(self, *exc):
+        sid, index, kind = self.before
+        torch._C._cuda_setStream(stream_id=sid, device_index=index, device_type=kind)
+
+
 def hinge(mix=0.75):
     """mix * mean_b max_j relu(m_bj) + (1 - mix) * mean_bj relu(m_bj) on margin vectors m."""
     def fn(margins, targets):
@@ -124,7 +146,7 @@ class DataParallelStep:
 
     def _make_wait(self, own):
         def wait(module, inputs):
-            cur = torch.cuda.current_stream()
+            cur = _current_stream()
             marks = None
             if self.trace is not None:
                 marks = (torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True))
@@ -152,9 +174,9 @@ class DataParallelStep:
             group = self.urgent if (p is self.first and self.urgent is not None) else None
             work = self.dist.all_reduce(p.grad, op=self.avg, group=group, async_op=True)
         else:
-            side.wait_stream(torch.cuda.current_stream())
+            side.wait_stream(_current_stream())
         p.grad.record_stream(side)
-        with torch.cuda.stream(side):
+        with _use_stream(side):
             if work is not None:
                 work.wait()                       # stream-side wait: the host does not block
             self.opt.step_params([p])
@@ -193,7 +215,7 @@ class DataParallelStep:
         if self.flat_buffers is not None and self.net.training:
             if self.cuda:
                 # the collective runs on the communicator's stream: it must see this forward's updates
-                self.flat_buffers.record_stream(torch.cuda.current_stream())
+                self.flat_buffers.record_stream(_current_stream())
             self.buffer_work = self.dist.broadcast(self.flat_buffers, src=0, async_op=self.cuda)
         return out
 
@@ -207,8 +229,8 @@ class DataParallelStep:
     def synchronize(self):
         """Makes the current stream wait for every update issued so far."""
         if self.cuda:
-            torch.cuda.current_stream().wait_stream(self.side)
-            torch.cuda.current_stream().wait_stream(self.side_first)
+            _current_stream().wait_stream(self.side)
+            _current_stream().wait_stream(self.side_first)
 
     def close(self):
         """Takes the hooks off the network (the hooks hold this object, the object holds the network)."""
@@ -313,12 +335,12 @@ class SparseRowsStep(DataParallelStep):
         rows, cols, cap, W = p.size(0), p.numel() // p.size(0), st["cap"], self.world
         par, lib = self.step_no & 1, self.lib
         side = self.side_first if p is self.first else self.side
-        side.wait_stream(torch.cuda.current_stream())
+        side.wait_stream(_current_stream())
         grad = p.grad
         if not grad.is_contiguous():
             return super()._issue(p)
         grad.record_stream(side)
-        with torch.cuda.stream(side):
+        with _use_stream(side):
             s, err = side.cuda_stream, self.err.data_ptr()
             mine_c, mine_e = st["cnt"].view(2, rows)[par], st["ent"].view(2, rows * cap * 2)[par]
             _lib.check(lib.linf_grad_rows_compact(grad.data_ptr(), rows, cols, cap, mine_c.data_ptr(),
@@ -358,7 +380,7 @@ class SparseRowsStep(DataParallelStep):
 
     def synchronize(self):
         super().synchronize()
-        torch.cuda.current_stream().synchronize()
+        _current_stream().synchronize()
         self._check(wait=True)
 
 
@@ -476,7 +498,7 @@ def bench_train_step(device, world, rank, steps=8, warmup=3, batch=None, p=float
     def step():
         x, t, ev = nxt["x"], nxt["t"], nxt["ev"]
         if ev is not None:
-            cur = torch.cuda.current_stream()
+            cur = _current_stream()
             cur.wait_event(ev)
             x.record_stream(cur); t.record_stream(cur)
         fetch()
