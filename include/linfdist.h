@@ -244,6 +244,13 @@ int linf_norm_dist_backward_weight(const float* grad_output, const float* input,
                                    float* grad_weight, float p, void* stream);
 
 /*
+ * linf_norm_dist_forward with scratch for the maximum pass of a run-time p (same rules for the workspace as below; same result).
+ */
+size_t linf_norm_dist_forward_workspace_bytes(int B, int CO, int CI, int G, int HW, float p);
+int linf_norm_dist_forward_ws(const float* input, const float* weight, int B, int CO, int CI, int G, int HW,
+                              float* output, float p, void* workspace, size_t workspace_bytes, void* stream);
+
+/*
  * One or both of the two gradients above (either pointer may be NULL, not both) in one pass over the terms.
  * The workspace (256-byte aligned, contents irrelevant, free again when the call's work on the stream is done) has
  * the size the query answers for the same arguments; 0, or a NULL workspace, means the separate kernels are used.

@@ -46,6 +46,8 @@ _PROTOS = {
     "linf_inf_dist_forward_pruned": [_F, _F, _INT, _INT, _INT, _INT, _INT, _F, _F, _INT, _F, _F, _F, ctypes.c_size_t, _F],
     "linf_inf_dist_bound_pruned_workspace_bytes": [_INT, _INT, _INT, _INT, _INT],
     "linf_inf_dist_bound_pruned": [_F, _F, _F, _INT, _INT, _INT, _INT, _INT, _F, _F, _INT, _F, _F, _F, ctypes.c_size_t, _F],
+    "linf_norm_dist_forward_workspace_bytes": [_INT, _INT, _INT, _INT, _INT, ctypes.c_float],
+    "linf_norm_dist_forward_ws": [_F, _F, _INT, _INT, _INT, _INT, _INT, _F, ctypes.c_float, _F, ctypes.c_size_t, _F],
     "linf_norm_dist_backward_workspace_bytes": [_INT, _INT, _INT, _INT, _INT, ctypes.c_float, _INT, _INT],
     "linf_norm_dist_backward": [_F, _F, _F, _F, _INT, _INT, _INT, _INT, _INT, _F, _F, ctypes.c_float, _F, ctypes.c_size_t, _F],
 }
@@ -53,6 +55,7 @@ _RESTYPE = {
     "linf_error_string": ctypes.c_char_p,
     "linf_launch_count": ctypes.c_ulonglong,
     "linf_inf_dist_forward_workspace_bytes": ctypes.c_size_t,
+    "linf_norm_dist_forward_workspace_bytes": ctypes.c_size_t,
     "linf_norm_dist_backward_workspace_bytes": ctypes.c_size_t,
     "linf_inf_dist_forward_pruned_workspace_bytes": ctypes.c_size_t,
     "linf_inf_dist_bound_pruned_workspace_bytes": ctypes.c_size_t,

@@ -88,6 +88,7 @@ extern int inf_forward_split;
 extern int inf_forward_width;
 extern int inf_forward_windows;
 extern int inf_forward_rows;
+void inf_prune_set(int);
 extern int lp_forward_width;
 int inf_forward_tma_gave_up();
 
@@ -132,6 +133,7 @@ int linf_tune_set(int key, int value) {
     if (key == 6 && value >= 0 && value <= 2) { lp_forward_width = value; return LINF_OK; }
     if (key == 7 && value >= 0 && value <= 1) { inf_forward_windows = value; return LINF_OK; }
     if (key == 8 && value >= 0 && value <= 1) { inf_forward_rows = value; return LINF_OK; }
+    if (key == 9) { inf_prune_set(value); return LINF_OK; }
     if (key == 2) return inf_forward_tma_gave_up();   // 1 = a bounded wait of the TMA loader ran out since the library was loaded
     return LINF_ERR_DIMS;
 }
@@ -292,6 +294,22 @@ int linf_norm_dist_backward_weight(const float* grad_output, const float* input,
     int rc = make_dims(B, CO, CI, G, HW, &d);
     if (rc) return rc;
     return lp_backward_weight(grad_output, input, weight, output, d, grad_weight, p, as_stream(stream));
+}
+
+size_t linf_norm_dist_forward_workspace_bytes(int B, int CO, int CI, int G, int HW, float p) {
+    Dims d;
+    if (bad_p(p) || make_dims(B, CO, CI, G, HW, &d)) return 0;
+    return lp_forward_workspace(d, p);
+}
+
+int linf_norm_dist_forward_ws(const float* input, const float* weight, int B, int CO, int CI, int G, int HW,
+                              float* output, float p, void* workspace, size_t workspace_bytes, void* stream) {
+    if (!input || !weight || !output) return LINF_ERR_NULL;
+    if (bad_p(p)) return LINF_ERR_P;
+    Dims d;
+    int rc = make_dims(B, CO, CI, G, HW, &d);
+    if (rc) return rc;
+    return lp_forward(input, weight, d, output, p, as_stream(stream), lp_forward_workspace(d, p) ? workspace : nullptr, workspace_bytes);
 }
 
 size_t linf_norm_dist_backward_workspace_bytes(int B, int CO, int CI, int G, int HW, float p, int want_input, int want_weight) {

@@ -190,7 +190,8 @@ int lp_forward_dense(const float* x, const float* w, const Dims& d, float* y, fl
 bool lp_tiled_ok(const Dims& d, const void* a, const void* b, const void* c, const void* e, const void* f);
 int lp_backward_tiled(const float* g, const float* x, const float* w, const float* y, const Dims& d,
                       float* out, float p, bool wrt_weight, cudaStream_t st);
-int lp_forward(const float* x, const float* w, const Dims& d, float* y, float p, cudaStream_t st);
+size_t lp_forward_workspace(const Dims& d, float p);
+int lp_forward(const float* x, const float* w, const Dims& d, float* y, float p, cudaStream_t st, void* ws = nullptr, size_t ws_bytes = 0);
 int lp_backward_input(const float* g, const float* x, const float* w, const float* y,
                       const Dims& d, float* gx, float p, cudaStream_t st);
 int lp_backward_weight(const float* g, const float* x, const float* w, const float* y,

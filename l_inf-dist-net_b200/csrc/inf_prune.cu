@@ -296,47 +296,46 @@ list_kernel(const PruneParams p) {
     }
 }
 
-// Shared rows, 4 * NQ of them in NQ arrays of float4 [K] (one array of twice the width would use half the bank groups per load).  W_LISTS:
-// rows of x (bounds: lower and upper of half as many rows), lanes = outputs.  Otherwise: rows of w, lanes = rows of x.  NQ = 2 halves the
-// list entries read from L2; NQ = 1 is for rows too long for two arrays and for layers with too few blocks of rows to fill the GPU.
-template <bool BOUND, bool W_LISTS, bool TRACK, int NQ>
+// Shared rows, 4 * LG of them as [K][4 * LG] floats.  W_LISTS: rows of x (bounds: lower and upper of half as many rows), lanes = outputs.
+// Otherwise: rows of w, lanes = rows of x.  LG neighbouring lanes walk the list of one row together, each with its own four of the shared
+// rows: a gather then reads 16 * LG contiguous bytes per entry, which meets fewer bank conflicts (expected cycles of a warp's 16-byte load:
+// 10.4 / 8.5 / 6 / 4 for LG = 1 / 2 / 4 / 8), and the warp's lists differ less in length.  LG is as large as the shared memory holds.
+template <bool BOUND, bool W_LISTS, bool TRACK, int LG>
 __global__ void __launch_bounds__(1024, 1)
 gather_kernel(const PruneParams p, int blocks_a, int splits) {
     extern __shared__ __align__(16) float4 rows4[];
     const int any_x = p.head->any_x;
     if (p.head->dense || (!W_LISTS && !any_x)) return;
     constexpr bool PAIRS = BOUND && W_LISTS;
-    constexpr int NA = PAIRS ? 2 * NQ : 4 * NQ;         // rows of the shared side
-    const int tid = threadIdx.x, lane = tid & 31, nt = blockDim.x;
+    constexpr int NA = PAIRS ? 2 : 4;                   // outputs of a lane per list row
+    constexpr int RW = 32 / LG;                         // list rows of a warp
+    const int tid = threadIdx.x, lane = tid & 31, nt = blockDim.x, quad = tid % LG;
     int id = blockIdx.x;
     const int split = id % splits; id /= splits;
     const int blk = id % blocks_a, g = id / blocks_a;
-    const int a0 = blk * NA;
+    const int a0 = blk * (NA * LG) + NA * quad;         // first of this lane's shared rows
     {
         const int last = (W_LISTS ? p.R : p.N) - 1;
+        const float* src[4];
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-            const float* src[4];
-#pragma unroll
-            for (int a = 0; a < 4; ++a) {
-                if (PAIRS) src[a] = (a & 1 ? p.xu : p.xl) + (size_t)min(a0 + 2 * q + (a >> 1), last) * p.CI + (size_t)g * p.K;
-                else if (W_LISTS) src[a] = p.xl + (size_t)min(a0 + 4 * q + a, last) * p.CI + (size_t)g * p.K;
-                else src[a] = p.w + ((size_t)g * p.N + min(a0 + 4 * q + a, last)) * p.K;
-            }
-#pragma unroll 4
-            for (int k = tid; k < p.K; k += nt)
-                rows4[q * p.K + k] = make_float4(__ldg(src[0] + k), __ldg(src[1] + k), __ldg(src[2] + k), __ldg(src[3] + k));
+        for (int a = 0; a < 4; ++a) {
+            if (PAIRS) src[a] = (a & 1 ? p.xu : p.xl) + (size_t)min(a0 + (a >> 1), last) * p.CI + (size_t)g * p.K;
+            else if (W_LISTS) src[a] = p.xl + (size_t)min(a0 + a, last) * p.CI + (size_t)g * p.K;
+            else src[a] = p.w + ((size_t)g * p.N + min(a0 + a, last)) * p.K;
         }
+#pragma unroll 4
+        for (int k = tid / LG; k < p.K; k += nt / LG)
+            rows4[k * LG + quad] = make_float4(__ldg(src[0] + k), __ldg(src[1] + k), __ldg(src[2] + k), __ldg(src[3] + k));
     }
     __syncthreads();
     const int NL = W_LISTS ? p.N : p.R;
     const int stride = W_LISTS ? p.CO : p.G * p.R;
     const int* cnt = (W_LISTS ? p.cnt_w : p.cnt_x) + g * NL;
-    const int per = ((NL + splits - 1) / splits + 31) / 32 * 32;
+    const int per = ((NL + splits - 1) / splits + RW - 1) / RW * RW;
     const int l_end = min(NL, (split + 1) * per);
     const float bound = p.head->bound;
-    for (int l0 = split * per + (tid & ~31); l0 < l_end; l0 += nt) {
-        const int l = l0 + lane;
+    for (int l0 = split * per + (tid >> 5) * RW; l0 < l_end; l0 += (nt >> 5) * RW) {
+        const int l = l0 + lane / LG;
         const int n = l < l_end ? __ldg(cnt + l) : 0;
         const int most = __reduce_max_sync(FULL, n);
         float t[NA];                                    // forward: signed difference of the largest term; bounds: U
@@ -371,38 +370,28 @@ gather_kernel(const PruneParams p, int blocks_a, int splits) {
             fetch(s + U);                               // the next entries are on their way while these are looked up
 #pragma unroll
             for (int u = 0; u < U; ++u) {
+                const float4 f = rows4[kk[u] * LG + quad];
+                const float r[4] = {f.x, f.y, f.z, f.w};
 #pragma unroll
-                for (int q = 0; q < NQ; ++q) {
-                    const float4 f = rows4[q * p.K + kk[u]];
-                    const float r[4] = {f.x, f.y, f.z, f.w};
-                    if (PAIRS) {
-#pragma unroll
-                        for (int a = 0; a < 2; ++a) bound_term(r[2 * a], r[2 * a + 1], c[u], m[2 * q + a], t[2 * q + a]);
-                    } else if (BOUND) {
-#pragma unroll
-                        for (int a = 0; a < 4; ++a) bound_term(c[u], c2[u], r[a], m[(BOUND ? 4 * q + a : 0)], t[(4 * q + a) % NA]);
-                    } else {
-#pragma unroll
-                        for (int a = 0; a < 4; ++a) {
-                            const float d = W_LISTS ? r[a] - c[u] : c[u] - r[a];
-                            const int i = (4 * q + a) % NA;
-                            if (fabsf(d) > fabsf(t[i])) { t[i] = d; if (TRACK) at[i] = kk[u]; }
-                        }
+                for (int a = 0; a < NA; ++a) {
+                    if constexpr (PAIRS) bound_term(r[2 * a], r[2 * a + 1], c[u], m[a], t[a]);
+                    else if constexpr (BOUND) bound_term(c[u], c2[u], r[a], m[a], t[a]);
+                    else {
+                        const float d = W_LISTS ? r[a] - c[u] : c[u] - r[a];
+                        if (fabsf(d) > fabsf(t[a])) { t[a] = d; if constexpr (TRACK) at[a] = kk[u]; }
                     }
                 }
             }
         }
         if (l >= l_end) continue;
-        if (!W_LISTS && !BOUND && p.vec && a0 + NA <= p.N) {    // neighbouring outputs of one row, four at a time
-            const size_t e = (size_t)l * p.CO + g * p.N + a0;
-#pragma unroll
-            for (int a = 0; a < NA; a += 4) {
-                *reinterpret_cast<float4*>(p.y0 + e + a) = make_float4(fabsf(t[a]), fabsf(t[(a + 1) % NA]), fabsf(t[(a + 2) % NA]), fabsf(t[(a + 3) % NA]));
+        if constexpr (!W_LISTS && !BOUND) {
+            if (p.vec && a0 + 3 < p.N) {                // four neighbouring outputs of one row
+                const size_t e = (size_t)l * p.CO + g * p.N + a0;
+                *reinterpret_cast<float4*>(p.y0 + e) = make_float4(fabsf(t[0]), fabsf(t[1]), fabsf(t[2]), fabsf(t[3]));
                 if constexpr (TRACK)
-                    *reinterpret_cast<int4*>(p.pos + e + a) = make_int4(signed_at(t[a], at[a]), signed_at(t[(a + 1) % NA], at[(a + 1) % NA]),
-                                                                        signed_at(t[(a + 2) % NA], at[(a + 2) % NA]), signed_at(t[(a + 3) % NA], at[(a + 3) % NA]));
+                    *reinterpret_cast<int4*>(p.pos + e) = make_int4(signed_at(t[0], at[0]), signed_at(t[1], at[1]), signed_at(t[2], at[2]), signed_at(t[3], at[3]));
+                continue;
             }
-            continue;
         }
 #pragma unroll
         for (int a = 0; a < NA; ++a) {
@@ -534,38 +523,41 @@ PruneSizes prune_sizes(const Dims& d, bool bound) {
     return s;
 }
 
-template <bool BOUND, bool W_LISTS, bool TRACK, int NQ>
+template <bool BOUND, bool W_LISTS, bool TRACK, int LG>
 int launch_gather_as(const PruneParams& p, cudaStream_t st) {
-    constexpr int NA = (BOUND && W_LISTS ? 2 : 4) * NQ;
+    constexpr int NA = (BOUND && W_LISTS ? 2 : 4) * LG;
     const int na = W_LISTS ? p.R : p.N, nl = W_LISTS ? p.N : p.R;
     const int blocks = (na + NA - 1) / NA;
-    const size_t smem = (size_t)p.K * 16 * NQ;
+    const size_t smem = (size_t)p.K * 16 * LG;
     int per_sm = (int)(220 * 1024 / (smem + 1024));
     if (per_sm > 4) per_sm = 4;
     if (per_sm < 1) per_sm = 1;
     // 32 warps on an SM (64 registers a thread); no more threads than lanes of work, but enough to fill the shared rows
     int threads = 1024 / per_sm;
-    const int lanes = (nl + 31) / 32 * 32;
+    const int lanes = (nl * LG + 31) / 32 * 32;
     if (threads > lanes) threads = lanes < 256 ? 256 : lanes;
-    // enough CTAs for four waves, as long as every warp of a CTA has a list to walk
-    const long long want = 4LL * per_sm * sm_count();
+    // enough CTAs for two waves, as long as every warp of a CTA has a list to walk
+    const long long want = 2LL * per_sm * sm_count();
     long long splits = (want + (long long)blocks * p.G - 1) / ((long long)blocks * p.G);
-    const int most = (nl + threads - 1) / threads;
+    const int most = (int)(((long long)nl * LG + threads - 1) / threads);
     if (splits > most) splits = most;
     if (splits < 1) splits = 1;
-    auto kern = gather_kernel<BOUND, W_LISTS, TRACK, NQ>;
+    auto kern = gather_kernel<BOUND, W_LISTS, TRACK, LG>;
     if (smem > 40 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return LINF_ERR_LAUNCH;
     kern<<<(unsigned)((long long)blocks * p.G * splits), threads, smem, st>>>(p, blocks, (int)splits);
     return launch_status();
 }
 
+int inf_prune_lanes = 0;      // probe
+
 template <bool BOUND, bool W_LISTS, bool TRACK>
 int launch_gather(const PruneParams& p, cudaStream_t st) {
-    const long long rows = (long long)(W_LISTS ? p.R * (BOUND ? 2 : 1) : p.N) * p.G;
-    // with at most 512 lanes a CTA cannot hold more than 16 warps: two CTAs of one array each then
-    const int nl = W_LISTS ? p.N : p.R;
-    const bool two = p.K <= kMaxK / 2 && (nl > 512 || p.K <= kMaxK / 4) && rows * ((W_LISTS ? p.N : p.R) + 511) / 512 >= 8LL * 4 * sm_count();
-    return two ? launch_gather_as<BOUND, W_LISTS, TRACK, 2>(p, st) : launch_gather_as<BOUND, W_LISTS, TRACK, 1>(p, st);
+    int lg = p.K <= kMaxK / 8 ? 8 : p.K <= kMaxK / 4 ? 4 : p.K <= kMaxK / 2 ? 2 : 1;
+    if (inf_prune_lanes && lg > inf_prune_lanes) lg = inf_prune_lanes;
+    if (lg == 8) return launch_gather_as<BOUND, W_LISTS, TRACK, 8>(p, st);
+    if (lg == 4) return launch_gather_as<BOUND, W_LISTS, TRACK, 4>(p, st);
+    if (lg == 2) return launch_gather_as<BOUND, W_LISTS, TRACK, 2>(p, st);
+    return launch_gather_as<BOUND, W_LISTS, TRACK, 1>(p, st);
 }
 
 template <bool BOUND, bool TRACK>
@@ -592,6 +584,7 @@ int run_pruned(const PruneParams& p, bool vec, cudaStream_t st) {
 
 }  // namespace
 
+void inf_prune_set(int v) { inf_prune_lanes = v; }
 // Which calls are worth the attempt: dense layers with long rows, and enough work that the sample, the lists and five launches (about
 // 30 us) are small against the full scan.  Measured, us, full scan / lists, B = 512, x = 0.25 * normal: 1024 x 1024 forward 63 / 60, bounds 122 / 77;
 // 784 x 5120 (x uniform) forward 176 / 107.  Data that turn out not to suit cost 25 us on top of the scan.  The kernels for rows that are no

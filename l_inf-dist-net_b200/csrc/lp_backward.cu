@@ -65,7 +65,18 @@ __device__ __forceinline__ void factors(u64 (&s)[N], const PowQ q) {
         }
     } else {
         constexpr int NB = -IP;
-        u64 b[N], v[N];
+        // the fractional part first: the special-function unit works on it while the FP32 pipe squares
+        u64 b[N], v[N], r[N];
+        if (q.f != 0.f) {
+            const u64 ff = pack2(q.f, q.f);
+#pragma unroll
+            for (int e = 0; e < N; ++e) {
+                float a0, a1;
+                unpack_f32x2(s[e], a0, a1);
+                unpack_f32x2(mul2(pack2(lg2_approx(fabsf(a0)), lg2_approx(fabsf(a1))), ff), a0, a1);
+                r[e] = pack2(ex2_approx(a0), ex2_approx(a1));       // s = 0: exp2(-inf) = 0
+            }
+        }
 #pragma unroll
         for (int e = 0; e < N; ++e) { b[e] = s[e]; v[e] = s[e]; }
         if (q.m & 1) {
@@ -83,14 +94,8 @@ __device__ __forceinline__ void factors(u64 (&s)[N], const PowQ q) {
             }
         }
         if (q.f != 0.f) {
-            const u64 ff = pack2(q.f, q.f);
 #pragma unroll
-            for (int e = 0; e < N; ++e) {
-                float a0, a1;
-                unpack_f32x2(s[e], a0, a1);
-                unpack_f32x2(mul2(pack2(lg2_approx(fabsf(a0)), lg2_approx(fabsf(a1))), ff), a0, a1);
-                v[e] = mul2(v[e], pack2(ex2_approx(a0), ex2_approx(a1)));       // s = 0: exp2(-inf) = 0
-            }
+            for (int e = 0; e < N; ++e) v[e] = mul2(v[e], r[e]);
         }
 #pragma unroll
         for (int e = 0; e < N; ++e) s[e] = v[e];

@@ -138,8 +138,10 @@ class DistF(torch.autograd.Function):
                 _lib.check(rc, "inf_dist_forward")
                 ctx.save_for_backward(xk, weight, y, pos)
             else:
-                rc = lib.linf_norm_dist_forward(xk.data_ptr(), weight.data_ptr(), B, CO, CI, G, HW,
-                                                y.data_ptr(), float(p), _stream())
+                need = lib.linf_norm_dist_forward_workspace_bytes(B, CO, CI, G, HW, float(p))
+                ws = torch.empty(need, dtype=torch.uint8, device=x.device) if need else None
+                rc = lib.linf_norm_dist_forward_ws(xk.data_ptr(), weight.data_ptr(), B, CO, CI, G, HW,
+                                                   y.data_ptr(), float(p), ws.data_ptr() if need else None, need, _stream())
                 _lib.check(rc, "norm_dist_forward")
                 ctx.save_for_backward(xk, weight, y)
         ctx.group, ctx.p, ctx.tag = group, p, tag
