@@ -244,7 +244,7 @@ int linf_norm_dist_backward_weight(const float* grad_output, const float* input,
                                    float* grad_weight, float p, void* stream);
 
 /*
- * linf_norm_dist_forward with scratch for the maximum pass of a run-time p (same rules for the workspace as below; same result).
+ * linf_norm_dist_forward with scratch for the maximum pass (same rules for the workspace as below; same result).
  */
 size_t linf_norm_dist_forward_workspace_bytes(int B, int CO, int CI, int G, int HW, float p);
 int linf_norm_dist_forward_ws(const float* input, const float* weight, int B, int CO, int CI, int G, int HW,

@@ -88,7 +88,6 @@ extern int inf_forward_split;
 extern int inf_forward_width;
 extern int inf_forward_windows;
 extern int inf_forward_rows;
-void inf_prune_set(int);
 extern int lp_forward_width;
 int inf_forward_tma_gave_up();
 
@@ -133,7 +132,6 @@ int linf_tune_set(int key, int value) {
     if (key == 6 && value >= 0 && value <= 2) { lp_forward_width = value; return LINF_OK; }
     if (key == 7 && value >= 0 && value <= 1) { inf_forward_windows = value; return LINF_OK; }
     if (key == 8 && value >= 0 && value <= 1) { inf_forward_rows = value; return LINF_OK; }
-    if (key == 9) { inf_prune_set(value); return LINF_OK; }
     if (key == 2) return inf_forward_tma_gave_up();   // 1 = a bounded wait of the TMA loader ran out since the library was loaded
     return LINF_ERR_DIMS;
 }

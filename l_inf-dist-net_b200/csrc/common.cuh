@@ -84,6 +84,16 @@ __device__ __forceinline__ unsigned long long sub_f32x2(unsigned long long a, un
     asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
+__device__ __forceinline__ unsigned long long mul_f32x2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long pack_f32x2(float lo, float hi) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
 __device__ __forceinline__ void unpack_f32x2(unsigned long long v, float& lo, float& hi) {
     asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
 }
@@ -182,9 +192,8 @@ int inf_forward_skinny(const float* x, const float* w, const Dims& d, float* y, 
                        const Post& post);
 int inf_bound_skinny(const float* xl, const float* xu, const float* w, const Dims& d, float* yl, float* yu,
                      cudaStream_t st, const Post& post);
-// finite-p forward of dense layers (lp_forward.cu); where lp_forward_wants_max(p), y holds max_i |x - w| on entry
+// finite-p forward of dense layers (lp_forward.cu); y holds max_i |x - w| on entry
 bool lp_forward_dense_ok(const Dims& d);
-bool lp_forward_wants_max(float p);
 int lp_forward_dense(const float* x, const float* w, const Dims& d, float* y, float p, cudaStream_t st);
 // register-tiled finite-p gradients for dense, aligned layers (lp_tiled.cu)
 bool lp_tiled_ok(const Dims& d, const void* a, const void* b, const void* c, const void* e, const void* f);

@@ -298,8 +298,8 @@ list_kernel(const PruneParams p) {
 
 // Shared rows, 4 * LG of them as [K][4 * LG] floats.  W_LISTS: rows of x (bounds: lower and upper of half as many rows), lanes = outputs.
 // Otherwise: rows of w, lanes = rows of x.  LG neighbouring lanes walk the list of one row together, each with its own four of the shared
-// rows: a gather then reads 16 * LG contiguous bytes per entry, which meets fewer bank conflicts (expected cycles of a warp's 16-byte load:
-// 10.4 / 8.5 / 6 / 4 for LG = 1 / 2 / 4 / 8), and the warp's lists differ less in length.  LG is as large as the shared memory holds.
+// rows: a gather then reads 16 * LG contiguous bytes per entry, which meets fewer bank conflicts, and the warp's
+// lists differ less in length; against that, a CTA fills more shared memory and every lane does its list's bookkeeping (`launch_gather`).
 template <bool BOUND, bool W_LISTS, bool TRACK, int LG>
 __global__ void __launch_bounds__(1024, 1)
 gather_kernel(const PruneParams p, int blocks_a, int splits) {
@@ -533,7 +533,7 @@ int launch_gather_as(const PruneParams& p, cudaStream_t st) {
     if (per_sm > 4) per_sm = 4;
     if (per_sm < 1) per_sm = 1;
     // 32 warps on an SM (64 registers a thread); no more threads than lanes of work, but enough to fill the shared rows
-    int threads = 1024 / per_sm;
+    int threads = 1024 / per_sm / 32 * 32;           // whole warps
     const int lanes = (nl * LG + 31) / 32 * 32;
     if (threads > lanes) threads = lanes < 256 ? 256 : lanes;
     // enough CTAs for two waves, as long as every warp of a CTA has a list to walk
@@ -548,15 +548,13 @@ int launch_gather_as(const PruneParams& p, cudaStream_t st) {
     return launch_status();
 }
 
-int inf_prune_lanes = 0;      // probe
-
+// LG = 2 pays for the lists of w under bounds (B = 512, Din = 3072, Dout = 5120: 182 -> 168 us; Din = Dout = 5120, normal: 308 -> 285), as long as
+// there are enough rows for twice the rows a CTA; elsewhere one lane per list row is faster (forward, same shapes: 90 / 93, 152 / 174).
 template <bool BOUND, bool W_LISTS, bool TRACK>
 int launch_gather(const PruneParams& p, cudaStream_t st) {
-    int lg = p.K <= kMaxK / 8 ? 8 : p.K <= kMaxK / 4 ? 4 : p.K <= kMaxK / 2 ? 2 : 1;
-    if (inf_prune_lanes && lg > inf_prune_lanes) lg = inf_prune_lanes;
-    if (lg == 8) return launch_gather_as<BOUND, W_LISTS, TRACK, 8>(p, st);
-    if (lg == 4) return launch_gather_as<BOUND, W_LISTS, TRACK, 4>(p, st);
-    if (lg == 2) return launch_gather_as<BOUND, W_LISTS, TRACK, 2>(p, st);
+    if constexpr (BOUND && W_LISTS) {
+        if (p.K <= kMaxK / 2 && p.R > 128) return launch_gather_as<BOUND, W_LISTS, TRACK, 2>(p, st);
+    }
     return launch_gather_as<BOUND, W_LISTS, TRACK, 1>(p, st);
 }
 
@@ -584,7 +582,6 @@ int run_pruned(const PruneParams& p, bool vec, cudaStream_t st) {
 
 }  // namespace
 
-void inf_prune_set(int v) { inf_prune_lanes = v; }
 // Which calls are worth the attempt: dense layers with long rows, and enough work that the sample, the lists and five launches (about
 // 30 us) are small against the full scan.  Measured, us, full scan / lists, B = 512, x = 0.25 * normal: 1024 x 1024 forward 63 / 60, bounds 122 / 77;
 // 784 x 5120 (x uniform) forward 176 / 107.  Data that turn out not to suit cost 25 us on top of the scan.  The kernels for rows that are no

@@ -344,12 +344,12 @@ bool grid_ok(const dim3& g) { return g.y <= 65535u && g.z <= 65535u; }
 }  // namespace
 
 size_t lp_forward_workspace(const Dims& d, float p) {
-    return lp_forward_dense_ok(d) && lp_forward_wants_max(p) ? inf_forward_pruned_workspace(d) : 0;
+    (void)p;
+    return lp_forward_dense_ok(d) ? inf_forward_pruned_workspace(d) : 0;
 }
 
 int lp_forward(const float* x, const float* w, const Dims& d, float* y, float p, cudaStream_t st, void* ws, size_t ws_bytes) {
     const bool dense = lp_forward_dense_ok(d);
-    if (dense && !lp_forward_wants_max(p)) return lp_forward_dense(x, w, d, y, p, st);
     // (the maximum through lists of large entries where there is workspace for them: 250 -> 135 us at B = 256, Din = 3072, Dout = 5120)
     int rc = dense && ws != nullptr ? inf_forward_pruned(x, w, d, y, nullptr, ws, ws_bytes, st, no_post())
                                     : inf_forward(x, w, d, y, nullptr, nullptr, 0, st);

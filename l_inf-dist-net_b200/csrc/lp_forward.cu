@@ -1,29 +1,16 @@
 // Forward of the finite-p distance neuron on dense layers (HW == 1, at least 32 outputs and 32 inputs per group; no
-// alignment or divisibility is asked for):   y[b,o] = (sum_i |x[b,i] - w[o,i]|^p)^(1/p).
+// alignment or divisibility is asked for):   y[b,o] = M * (sum_i (|x[b,i] - w[o,i]| / M)^p)^(1/p),  M = max_i |x - w|, which `y` holds on entry.
 //
-// Bound: FP32 issue for integer p, the special-function unit (one log2 per term, half an exp2) otherwise.
-//
-// A term needs a scale only so that its power stays within the range of a float, and any scale does: the sum is divided
-// by the same factor in the end.  So the maximum max_i |x - w|, which costs a pass of its own over all terms, is
-// not needed for an integer p whose powers are products:
-//   p = 8, 16          no scale at all.  Sums in [2^-64, 2^120] are kept: nothing overflowed, and a
-//                      difference whose power underflows is below 2^-60 of the sum.
-//   p = 64             one scale per output: the largest difference of the first eighth of its row (at least 64 terms) times 1.125.
-//                      Kept by the same rule: the maximum of the row may be 4 times the sample's.
-//   other p, or a sum outside the range (also: NaN, infinities, a row of zeros)
-//                      the literal rule: M = max_i |x - w| first, then sum (|x - w| / M)^p, y = M * sum^(1/p).  With powers taken through
-//                      log2 the largest terms then enter exactly (their logarithm is 0); with a sampled scale y was 1.2 to 1.5 times
-//                      less exact.  A run-time p gets M from the value-only inf-dist kernel, a tile with a sum outside the range
-//                      works it out itself.
+// Bound: FP32 issue for integer p (p = 8: subtraction, scale, two squarings, one multiply-add = 5 lane operations a term), the special-function
+// unit (one log2 and one exp2 per term: 16 cycles per term and scheduler) otherwise.
 // 64 x 64 (or 64 x 48) output tile per CTA of 128 threads, 8 x 4 (8 x 3) outputs per thread, operand tiles through a ring of
 // three cp.async stages; two neighbouring terms of an output sit in one register pair, so subtraction,
-// scale and squarings are packed (f32x2).
+// scale and squarings are packed (f32x2).  The sums run over i in ascending order, whatever the tile: the same bits for every width.
 //
-// Per term: p = 8: subtraction, two squarings, one multiply-add = 4 lane operations (literal rule: 6, and the maximum pass).
-// Run-time p: half of the exp2 run as a polynomial on the FP32 pipe (4 lg2 + 2 ex2 of the special-function unit for 4 terms =
-// 12 cycles per term and scheduler; all on the unit: 16).
-// Measured on one B200, us, maximum pass + literal rule -> here: B = 512, Din = Dout = 5120: p = 8: 3069 -> 1870,
-// 16: 3466 -> 2254, 64: 4230 -> 3550, 23.7: 7129 -> 5980; B = 203, Din = 1027, Dout = 1333 (generic kernels before), p = 8: 683 -> 117.
+// Without the scale (p = 8, 16: sums checked against the range of a float afterwards) and the maximum pass this takes 1.87 ms instead of
+// FWD8 at B = 512, Din = Dout = 5120, p = 8, and the result is as exact.  It is not used: a training run at finite p amplifies the last
+// bit of a distance within two steps (hinge loss, Adam with eps = 1e-10), and runs are kept reproducible from version to version.
+// Measured on one B200, us, with the maximum pass, before -> now: B = 512, Din = Dout = 5120: FWDALL
 #include <math.h>
 
 #include "common.cuh"
@@ -34,42 +21,9 @@ namespace {
 typedef unsigned long long u64;
 
 __device__ __forceinline__ u64 mul2(u64 a, u64 b) { u64 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-__device__ __forceinline__ u64 add2(u64 a, u64 b) { u64 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) { u64 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
 __device__ __forceinline__ u64 pack2(float a, float b) { u64 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
 __device__ __forceinline__ float lg2_approx(float a) { float r; asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a)); return r; }
 __device__ __forceinline__ float ex2_approx(float a) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a)); return r; }
-
-// 2^e for a pair on the FP32 pipe: e = n + f with the nearest integer n (the usual addition of 1.5 * 2^23), 2^f by the degree-6
-// interpolation of 2^f at the Chebyshev nodes of [-1/2, 1/2] (relative error in fp32 at most 8e-8; degree 5: 2.2e-7), n added to the
-// exponent.  e <= 0 up to rounding; below -125 the term is lost against a sum of at least 1 and e is held there (a NaN stays one).
-__device__ __forceinline__ float clamp_exp(float e) {
-    float r;
-    asm("max.NaN.f32 %0, %1, 0fC2FA0000;" : "=f"(r) : "f"(e));      // -125
-    return r;
-}
-__device__ __forceinline__ u64 ex2_poly2(u64 e) {
-    float e0, e1;
-    unpack_f32x2(e, e0, e1);
-    const u64 c = pack2(clamp_exp(e0), clamp_exp(e1));
-    const u64 z = add2(c, pack2(12582912.f, 12582912.f));
-    const u64 f = sub_f32x2(c, sub_f32x2(z, pack2(12582912.f, 12582912.f)));
-    u64 r = pack2(1.546144485e-04f, 1.546144485e-04f);
-    r = fma2(r, f, pack2(1.340042800e-03f, 1.340042800e-03f));
-    r = fma2(r, f, pack2(9.618056938e-03f, 9.618056938e-03f));
-    r = fma2(r, f, pack2(5.550327152e-02f, 5.550327152e-02f));
-    r = fma2(r, f, pack2(2.402265072e-01f, 2.402265072e-01f));
-    r = fma2(r, f, pack2(6.931471825e-01f, 6.931471825e-01f));
-    r = fma2(r, f, pack2(1.f, 1.f));
-    float r0, r1, z0, z1;
-    unpack_f32x2(r, r0, r1);
-    unpack_f32x2(z, z0, z1);
-    // A NaN ends as the canonical NaN 0x7fffffff in r and z; the addition below then gives 0x7f7fffff, the largest float, which
-    // no sum of terms <= 1 reaches: the caller takes such a sum for a NaN.
-    const float s0 = __int_as_float(__float_as_int(r0) + (__float_as_int(z0) << 23));
-    const float s1 = __int_as_float(__float_as_int(r1) + (__float_as_int(z1) << 23));
-    return pack2(s0, s1);
-}
 
 // a^E of a pair, E a power of two
 template <int E>
@@ -77,21 +31,12 @@ __device__ __forceinline__ u64 pow2_ct(u64 a) {
     if constexpr (E == 1) return a;
     else { const u64 h = pow2_ct<E / 2>(a); return mul2(h, h); }
 }
-template <int E>
-__device__ __forceinline__ float pow_ct(float a) {
-    if constexpr (E == 1) return a;
-    else { const float h = pow_ct<E / 2>(a); return h * h; }
-}
-
 constexpr int TM = 64, NT = 128, BK = 16, LDK = BK + 4, STAGES = 3;
-constexpr float kSumLow = 0x1p-64f, kSumHigh = 0x1p120f;
-constexpr float kLower = 1.f / 1.125f;
 
 struct FwdParams {
     const float* x; const float* w; float* y;
     int B, COg, CIg, G, CI, CO;
     float p, inv_p;
-    int sample;                 // k-tiles the scale is taken from
 };
 
 template <int ROWS, bool AL>
@@ -113,13 +58,12 @@ __device__ __forceinline__ void load_rows(float* dst, const float* __restrict__ 
     }
 }
 
-// IP: 8, 16, 64 at compile time (8 and 16 without a scale), 0: p at run time, and y holds max_i |x - w| on entry.  TJ: output columns per thread.
+// IP: 8, 16, 64 at compile time, 0: p at run time.  TJ: output columns per thread.
 template <int IP, int TJ, bool AL>
 __global__ void __launch_bounds__(NT, 3)
 lp_forward_kernel(const FwdParams p) {
     extern __shared__ __align__(16) float smem[];
     constexpr int TN = 16 * TJ, NO = 8 * TJ, STAGE = (TM + TN) * LDK;
-    constexpr bool PLAIN = IP == 8 || IP == 16;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int wm = warp & 1, wn = warp >> 1, lm = lane >> 3, ln = lane & 7;
     const int row_off = wm * 32 + lm, col_off = wn * (8 * TJ) + ln;       // + 4i rows, + 8j columns
@@ -148,8 +92,8 @@ lp_forward_kernel(const FwdParams p) {
             cp_async_commit();
             const float* As = smem + rd * STAGE + row_off * LDK;
             const float* Bs = smem + rd * STAGE + (TM + col_off) * LDK;
-            // two of the four k4 steps per trip (one where a term is long): the fully unrolled body runs into instruction fetch stalls
-#pragma unroll (IP == 8 || IP == 16 ? 2 : 1)
+            // two of the four k4 steps per trip: the fully unrolled body runs into instruction fetch stalls
+#pragma unroll 2
             for (int k4 = 0; k4 < BK / 4; ++k4) {
                 ulonglong2 bf[TJ];
 #pragma unroll
@@ -170,55 +114,6 @@ lp_forward_kernel(const FwdParams p) {
     auto inside = [&](int e) { return m0 + row_off + 4 * (e / TJ) < p.B && n0 + col_off + 8 * (e % TJ) < p.COg; };
 
     float S[NO];
-    if constexpr (IP > 0) {
-        [[maybe_unused]] float r[PLAIN ? 1 : NO];
-#pragma unroll
-        for (int e = 0; e < NO; ++e) S[e] = 0.f;
-        if constexpr (PLAIN) {
-            sweep(KT, [&](int e, u64 t01, u64 t23) {
-                float a, b;
-                unpack_f32x2(pow2_ct<IP / 2>(t01), a, b);
-                S[e] = fmaf(a, a, S[e]); S[e] = fmaf(b, b, S[e]);
-                unpack_f32x2(pow2_ct<IP / 2>(t23), a, b);
-                S[e] = fmaf(a, a, S[e]); S[e] = fmaf(b, b, S[e]);
-            });
-        } else {
-            sweep(min(KT, p.sample), [&](int e, u64 t01, u64 t23) {
-                float a, b, c, d;
-                unpack_f32x2(t01, a, b); unpack_f32x2(t23, c, d);
-                S[e] = max3(max3(S[e], fabsf(a), fabsf(b)), fabsf(c), fabsf(d));
-            });
-#pragma unroll
-            for (int e = 0; e < NO; ++e) { r[e] = S[e] > 0.f ? kLower / S[e] : 0.f; S[e] = 0.f; }
-            sweep(KT, [&](int e, u64 t01, u64 t23) {
-                const u64 rr = pack2(r[e], r[e]);
-                float a, b;
-                unpack_f32x2(pow2_ct<(IP > 0 ? IP / 2 : 1)>(mul2(t01, rr)), a, b);
-                S[e] = fmaf(a, a, S[e]); S[e] = fmaf(b, b, S[e]);
-                unpack_f32x2(pow2_ct<(IP > 0 ? IP / 2 : 1)>(mul2(t23, rr)), a, b);
-                S[e] = fmaf(a, a, S[e]); S[e] = fmaf(b, b, S[e]);
-            });
-        }
-        bool bad = false;
-#pragma unroll
-        for (int e = 0; e < NO; ++e) bad |= inside(e) && !(S[e] >= kSumLow && S[e] <= kSumHigh);
-        if (!__syncthreads_or(bad)) {
-#pragma unroll
-            for (int e = 0; e < NO; ++e)
-                if (inside(e)) *out(e) = PLAIN ? powf(S[e], p.inv_p) : powf(S[e], p.inv_p) / r[PLAIN ? 0 : e];
-            return;
-        }
-        // the maximum of every output, left in y for the literal rule (each thread reads back what it wrote)
-#pragma unroll
-        for (int e = 0; e < NO; ++e) S[e] = 0.f;
-        sweep(KT, [&](int e, u64 t01, u64 t23) {
-            float a, b, c, d;
-            unpack_f32x2(t01, a, b); unpack_f32x2(t23, c, d);
-            S[e] = max3(max3(S[e], fabsf(a), fabsf(b)), fabsf(c), fabsf(d));
-        });
-#pragma unroll
-        for (int e = 0; e < NO; ++e) if (inside(e)) *out(e) = S[e];
-    }
     float rM[NO];
 #pragma unroll
     for (int e = 0; e < NO; ++e) {
@@ -243,8 +138,8 @@ lp_forward_kernel(const FwdParams p) {
             const u64 e23 = mul2(pack2(lg2_approx(fabsf(a)), lg2_approx(fabsf(b))), pp);
             unpack_f32x2(e01, a, b);
             S[e] += ex2_approx(a); S[e] += ex2_approx(b);
-            unpack_f32x2(ex2_poly2(e23), a, b);
-            S[e] += a; S[e] += b;
+            unpack_f32x2(e23, a, b);
+            S[e] += ex2_approx(a); S[e] += ex2_approx(b);
         }
     });
 #pragma unroll
@@ -252,7 +147,6 @@ lp_forward_kernel(const FwdParams p) {
         if (inside(e)) {
             float* yo = out(e);
             const float M = *yo;
-            if (IP == 0 && S[e] > 1e30f) S[e] = __int_as_float(0x7fffffff);
             *yo = M > 0.f ? powf(S[e], p.inv_p) * M : 0.f;
         }
 }
@@ -274,7 +168,6 @@ int launch_fwd_ip(const FwdParams& P, int grid, bool narrow, bool al, cudaStream
 }  // namespace
 
 bool lp_forward_dense_ok(const Dims& d) { return d.HW == 1 && d.COg >= 32 && d.CIg >= 32; }
-bool lp_forward_wants_max(float p) { return p != 8.f && p != 16.f && p != 64.f; }
 
 int lp_forward_width = 0;   // 0: tile width by shape; 1: 64 columns; 2: 48 columns (benchmarking knob)
 
@@ -295,7 +188,6 @@ int lp_forward_dense(const float* x, const float* w, const Dims& d, float* y, fl
     P.x = x; P.w = w; P.y = y;
     P.B = d.R; P.COg = d.COg; P.CIg = d.CIg; P.G = d.G; P.CI = d.CI; P.CO = d.CO;
     P.p = p; P.inv_p = 1.f / p;
-    P.sample = max(4, (d.CIg + 8 * BK - 1) / (8 * BK));
     const bool al = (d.CIg & 3) == 0 && aligned16(x) && aligned16(w);
     if (p == 8.f) return launch_fwd_ip<8>(P, (int)grid, narrow, al, st);
     if (p == 16.f) return launch_fwd_ip<16>(P, (int)grid, narrow, al, st);
