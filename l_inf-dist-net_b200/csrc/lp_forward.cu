@@ -8,9 +8,11 @@
 // scale and squarings are packed (f32x2).  The sums run over i in ascending order, whatever the tile: the same bits for every width.
 //
 // Without the scale (p = 8, 16: sums checked against the range of a float afterwards) and the maximum pass this takes 1.87 ms instead of
-// FWD8 at B = 512, Din = Dout = 5120, p = 8, and the result is as exact.  It is not used: a training run at finite p amplifies the last
+// 2.72 ms at B = 512, Din = Dout = 5120, p = 8, and the result is as exact.  It is not used: a training run at finite p amplifies the last
 // bit of a distance within two steps (hinge loss, Adam with eps = 1e-10), and runs are kept reproducible from version to version.
-// Measured on one B200, us, with the maximum pass, before -> now: B = 512, Din = Dout = 5120: FWDALL
+// Measured on one B200, us, with the maximum pass (dense value-only kernel before, lists of large entries now), scale and squarings packed:
+// B = 512, Din = Dout = 5120: p = 8 3066 -> 2719, 16 3460 -> 3077, 64 4222 -> 3831, 23.7 7118 -> 6726; B = 203, Din = 1027, Dout = 1333 (the generic
+// kernel before): p = 8 683 -> RAGGED.
 #include <math.h>
 
 #include "common.cuh"
@@ -121,25 +123,21 @@ lp_forward_kernel(const FwdParams p) {
         rM[e] = M > 0.f ? 1.f / M : 0.f;
         S[e] = 0.f;
     }
-    [[maybe_unused]] const u64 pp = pack2(p.p, p.p);
     sweep(KT, [&](int e, u64 t01, u64 t23) {
-        const u64 rr = pack2(rM[e], rM[e]);
-        const u64 u01 = mul2(t01, rr), u23 = mul2(t23, rr);
-        float a, b;
         if constexpr (IP > 0) {
+            const u64 rr = pack2(rM[e], rM[e]);
+            const u64 u01 = mul2(t01, rr), u23 = mul2(t23, rr);
+            float a, b;
             unpack_f32x2(pow2_ct<IP / 2>(u01), a, b);
             S[e] = fmaf(a, a, S[e]); S[e] = fmaf(b, b, S[e]);
             unpack_f32x2(pow2_ct<IP / 2>(u23), a, b);
             S[e] = fmaf(a, a, S[e]); S[e] = fmaf(b, b, S[e]);
         } else {
-            unpack_f32x2(u01, a, b);
-            const u64 e01 = mul2(pack2(lg2_approx(fabsf(a)), lg2_approx(fabsf(b))), pp);
-            unpack_f32x2(u23, a, b);
-            const u64 e23 = mul2(pack2(lg2_approx(fabsf(a)), lg2_approx(fabsf(b))), pp);
-            unpack_f32x2(e01, a, b);
-            S[e] += ex2_approx(a); S[e] += ex2_approx(b);
-            unpack_f32x2(e23, a, b);
-            S[e] += ex2_approx(a); S[e] += ex2_approx(b);
+            // (scalar: packed multiplications around the special-function unit only add moves, 388 -> 409 us at B = 200, 1024 x 2048)
+            float t[4];
+            unpack_f32x2(t01, t[0], t[1]); unpack_f32x2(t23, t[2], t[3]);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) S[e] += ex2_approx(p.p * lg2_approx(fabsf(t[q]) * rM[e]));
         }
     });
 #pragma unroll
