@@ -345,8 +345,8 @@ bool grid_ok(const dim3& g) { return g.y <= 65535u && g.z <= 65535u; }
 
 size_t lp_forward_workspace(const Dims& d, float p) {
     (void)p;
-    // (shorter rows: the value-only dense kernel is as fast, and for x and w both normal faster: 496 / 529 us at Din = 784)
-    return lp_forward_dense_ok(d) && d.CIg >= 2048 ? inf_forward_pruned_workspace(d) : 0;
+    // (shorter rows, unless they are no multiple of four floats: the value-only dense kernel is as fast, and for x and w both normal faster: 496 / 529 us at Din = 784)
+    return lp_forward_dense_ok(d) && (d.CIg >= 2048 || (d.CIg & 3) != 0) ? inf_forward_pruned_workspace(d) : 0;
 }
 
 int lp_forward(const float* x, const float* w, const Dims& d, float* y, float p, cudaStream_t st, void* ws, size_t ws_bytes) {
