@@ -81,8 +81,7 @@ _KEPT_BYTES = 64 << 20
 
 
 def _scratch(device, nbytes):
-    """Scratch of the list passes: the stream's kept buffer up to 64 MB, a tensor of its own beyond.  (Allocated per call, these
-    buffers were cut out of the cached blocks of released weights, and the next net's weights needed fresh device memory: 2 -> 9 ms.)"""
+    """Scratch of the list passes: the stream's kept buffer up to 64 MB, a tensor of its own beyond."""
     return _workspace(device, nbytes) if nbytes <= _KEPT_BYTES else torch.empty(nbytes, dtype=torch.uint8, device=device)
 
 
