@@ -283,7 +283,7 @@ int linf_inf_dist_bound_pruned(const float* input_lower, const float* input_uppe
 
 /*
  * Patches of a k x k convolution over input [B, C, H, W] as rows [B * Ho * Wo, C * k * k] of a dense layer (channel-major, zero
- * outside the image; the column order of the reference's unfold, model/norm_dist.py:126-131), and the adjoint: grad_input [B, C, H, W],
+ * outside the image; the column order of torch's unfold, which NormDistConv, model/norm_dist.py:102-169, uses), and the adjoint: grad_input [B, C, H, W],
  * fully overwritten, every cell summed over the output rows, then columns, ascending.
  */
 int linf_unfold_rows(const float* input, int B, int C, int H, int W, int kernel_size, int dilation, int padding, int stride,
