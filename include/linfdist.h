@@ -363,6 +363,7 @@ int linf_grad_rows_merge(float* grad, int rows, int cols, int cap, const int* co
  *   key 6  the same for the finite-p forward
  *   key 7  arg-max tracking windows of the forward: 0 = 16 terms for rows of 2048 terms and more, else 8 (default),
  *          1 = 8 terms always
+ *   key 8  a handful of input rows: 0 = kernel of their own (default), 1 = the tiled and generic kernels
  * Returns LINF_OK, the answer of key 2, or LINF_ERR_DIMS for an unknown key / value.
  */
 int linf_tune_set(int key, int value);

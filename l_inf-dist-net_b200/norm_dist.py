@@ -77,12 +77,10 @@ def _workspace(device, nbytes):
     return buf
 
 
-_KEPT_BYTES = 64 << 20
-
-
 def _scratch(device, nbytes):
-    """Scratch of the list passes: the stream's kept buffer up to 64 MB, a tensor of its own beyond."""
-    return _workspace(device, nbytes) if nbytes <= _KEPT_BYTES else torch.empty(nbytes, dtype=torch.uint8, device=device)
+    """Scratch of a list pass: a tensor per call, from the current stream's pool.  (Not the kept buffer of `_workspace`: the pass is several
+    launches, and two host threads on one stream could interleave theirs.)"""
+    return torch.empty(nbytes, dtype=torch.uint8, device=device)
 
 
 def _shape5(x, weight, group):

@@ -22,8 +22,8 @@ def _current_stream():
     return torch.cuda.Stream(stream_id=sid, device_index=index, device_type=kind)
 
 
-class _use_stream:
-    """torch.cuda.stream(side) for a stream of the current device."""
+class _StreamSwitch:
+    """torch.cuda.stream(side) for a stream of the current device, without its look-ups."""
 
     def __init__(self, side):
         self.side = side
@@ -35,6 +35,10 @@ class _use_stream:
     def __exit__(self, *exc):
         sid, index, kind = self.before
         torch._C._cuda_setStream(stream_id=sid, device_index=index, device_type=kind)
+
+
+def _use_stream(side):
+    return _StreamSwitch(side) if side.device_index == torch._C._cuda_getDevice() else torch.cuda.stream(side)
 
 
 def hinge(mix=0.75):
