@@ -448,13 +448,15 @@ int launch_ip(const BothParams& P, int grid, int warps, bool al, bool dox, bool 
 
 // Which calls take this path: dense layers with at least 32 channels per group on both sides, 2 <= p < 1026 (below 2 the power
 // s * |s|^(p-2) has no integer part to start from), and
-//   * channel counts that are no multiples of four, where the alternative is the generic kernels (figures above), or
+//   * channel counts that are no multiples of four and 8 <= p <= 100, where the alternative is the generic kernels (figures above; at p = 300 and
+//     1000 these are up to 1.4 times more exact), or
 //   * 2048 rows and more (the pixels of a convolution), where the tiled weight kernel has few CTAs and long sums: 1934 -> 391 us at R = 16384.
 // Other dense layers keep the two tiled kernels, although this one would take half their time at B = 512 as well: a training run at
 // finite p amplifies a changed order of summation within two steps, and such runs are kept reproducible bit for bit from version to version.
 static bool both_ok(const Dims& d, float p) {
     const bool ragged = ((d.CIg | d.COg) & 3) != 0;
-    return d.HW == 1 && d.COg >= 32 && d.CIg >= 32 && p >= 2.f && p < 1026.f && (ragged || d.R >= 2048);
+    return d.HW == 1 && d.COg >= 32 && d.CIg >= 32 && p >= 2.f && p < 1026.f &&
+           (ragged ? p >= 8.f && p <= 100.f : d.R >= 2048);
 }
 
 size_t lp_backward_both_workspace(const Dims& d, float p, bool dox, bool dow) {

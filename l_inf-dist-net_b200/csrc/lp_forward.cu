@@ -165,7 +165,13 @@ int launch_fwd_ip(const FwdParams& P, int grid, bool narrow, bool al, cudaStream
 
 }  // namespace
 
-bool lp_forward_dense_ok(const Dims& d) { return d.HW == 1 && d.COg >= 32 && d.CIg >= 32; }
+// Dense layers with at least 32 channels per group on both sides.  Channel counts that are no multiples of four: 8 <= p <= 100 only.  Below and above,
+// the generic kernels, whose whole powers are products and not exp2(p * log2), are up to 1.4 times more exact (y at p = 2 and 3; the gradients
+// behind y at p = 300 and 1000), and they have always served these layers.
+bool lp_forward_dense_ok(const Dims& d, float p) {
+    const bool ragged = ((d.CIg | d.COg) & 3) != 0;
+    return d.HW == 1 && d.COg >= 32 && d.CIg >= 32 && (!ragged || (p >= 8.f && p <= 100.f));
+}
 
 int lp_forward_width = 0;   // 0: tile width by shape; 1: 64 columns; 2: 48 columns (benchmarking knob)
 
