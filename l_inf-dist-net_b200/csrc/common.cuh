@@ -198,7 +198,7 @@ int inf_forward_skinny(const float* x, const float* w, const Dims& d, float* y, 
 int inf_bound_skinny(const float* xl, const float* xu, const float* w, const Dims& d, float* yl, float* yu,
                      cudaStream_t st, const Post& post);
 // finite-p forward of dense layers (lp_forward.cu); y holds max_i |x - w| on entry
-bool lp_forward_dense_ok(const Dims& d, float p);
+bool lp_forward_dense_ok(const Dims& d, float p, bool aligned);
 int lp_forward_dense(const float* x, const float* w, const Dims& d, float* y, float p, cudaStream_t st);
 // register-tiled finite-p gradients for dense, aligned layers (lp_tiled.cu)
 bool lp_tiled_ok(const Dims& d, const void* a, const void* b, const void* c, const void* e, const void* f);

@@ -345,11 +345,11 @@ bool grid_ok(const dim3& g) { return g.y <= 65535u && g.z <= 65535u; }
 
 size_t lp_forward_workspace(const Dims& d, float p) {
     // (shorter rows, unless they are no multiple of four floats: the value-only dense kernel is as fast, and for x and w both normal faster: 496 / 529 us at Din = 784)
-    return lp_forward_dense_ok(d, p) && (d.CIg >= 2048 || (d.CIg & 3) != 0) ? inf_forward_pruned_workspace(d) : 0;
+    return lp_forward_dense_ok(d, p, ((d.CIg | d.COg) & 3) == 0) && (d.CIg >= 2048 || (d.CIg & 3) != 0) ? inf_forward_pruned_workspace(d) : 0;
 }
 
 int lp_forward(const float* x, const float* w, const Dims& d, float* y, float p, cudaStream_t st, void* ws, size_t ws_bytes) {
-    const bool dense = lp_forward_dense_ok(d, p);
+    const bool dense = lp_forward_dense_ok(d, p, lp_tiled_ok(d, x, w, y, nullptr, nullptr));
     // (the maximum through lists of large entries where there is workspace for them: 250 -> 135 us at B = 256, Din = 3072, Dout = 5120)
     int rc = dense && ws != nullptr ? inf_forward_pruned(x, w, d, y, nullptr, ws, ws_bytes, st, no_post())
                                     : inf_forward(x, w, d, y, nullptr, nullptr, 0, st);

@@ -60,7 +60,7 @@ __device__ __forceinline__ void load_rows(float* dst, const float* __restrict__ 
     }
 }
 
-// IP: 8, 16, 64 at compile time, 0: p at run time.  TJ: output columns per thread.
+// IP: 8, 16, 64 at compile time, 0: p at run time.  TJ: output columns per thread.  AL: rows of x and w can be read 16 bytes at a time.
 template <int IP, int TJ, bool AL>
 __global__ void __launch_bounds__(NT, 3)
 lp_forward_kernel(const FwdParams p) {
@@ -165,12 +165,12 @@ int launch_fwd_ip(const FwdParams& P, int grid, bool narrow, bool al, cudaStream
 
 }  // namespace
 
-// Dense layers with at least 32 channels per group on both sides.  Channel counts that are no multiples of four: 8 <= p <= 100 only.  Below and above,
-// the generic kernels, whose whole powers are products and not exp2(p * log2), are up to 1.4 times more exact (y at p = 2 and 3; the gradients
-// behind y at p = 300 and 1000), and they have always served these layers.
-bool lp_forward_dense_ok(const Dims& d, float p) {
-    const bool ragged = ((d.CIg | d.COg) & 3) != 0;
-    return d.HW == 1 && d.COg >= 32 && d.CIg >= 32 && (!ragged || (p >= 8.f && p <= 100.f));
+// Dense layers with at least 32 channels per group on both sides.  `aligned`: channel counts are multiples of four and x, w and y lie on 16-byte
+// boundaries (lp_tiled_ok).  Other calls only at 8 <= p <= 100: below and above, the generic kernels, whose whole powers are products and
+// not exp2(p * log2), are up to 1.4 times more exact (y at p = 2 and 3; the gradients behind y at p = 300 and 1000), and they have always served
+// these calls.
+bool lp_forward_dense_ok(const Dims& d, float p, bool aligned) {
+    return d.HW == 1 && d.COg >= 32 && d.CIg >= 32 && (aligned || (p >= 8.f && p <= 100.f));
 }
 
 int lp_forward_width = 0;   // 0: tile width by shape; 1: 64 columns; 2: 48 columns (benchmarking knob)

@@ -76,3 +76,42 @@ def test_dense_large_common_offset(cuda, lib, p):
     x, w = x + 2.0 ** 20, w + 2.0 ** 20
     x[:, 0] += 1
     check(L, x, w, g, 1, p)
+
+
+def off_by_one_float(t):
+    """The same values in memory that starts 4 bytes past a 16-byte boundary (a view of a flat buffer)."""
+    flat = torch.empty(t.numel() + 4, device=t.device)
+    v = flat[1: 1 + t.numel()].view(t.shape)
+    assert v.data_ptr() % 16 == 4
+    return v.copy_(t)
+
+
+@pytest.mark.parametrize("p", [2.0, 3.0, 7.5, 100.5, 300.0])
+def test_unaligned_tensors_keep_the_generic_kernel(cuda, lib, p):
+    """Channel counts that are multiples of four do not make a dense layer an aligned one.  The generic kernel, which serves spatial layouts
+    as well, adds the same powers in the same order there: the same bits."""
+    import linfdist_b200 as L
+    torch.manual_seed(3)
+    B, CI, CO = 70, 96, 64
+    x, w = torch.randn(B, CI, 1, device="cuda"), torch.randn(CO, CI, device="cuda")
+    y = L.norm_dist(off_by_one_float(x), off_by_one_float(w), 1, p)
+    s = torch.cuda.current_stream().cuda_stream
+    spatial, want = x[:, :, 0].t().contiguous().view(1, CI, B), torch.empty(1, CO, B, device="cuda")
+    assert lib.linf_norm_dist_forward(spatial.data_ptr(), w.data_ptr(), 1, CO, CI, 1, B, want.data_ptr(), p, s) == 0
+    assert torch.equal(y[:, :, 0], want[0].t())
+
+
+@pytest.mark.parametrize("p", [2.5, 8.0, 16.0, 23.7, 64.0, 300.0])
+@pytest.mark.parametrize("B,CI,CO,G", [(33, 64, 36, 1), (70, 97, 65, 1), (130, 2052, 64, 1), (2100, 64, 64, 2)])
+def test_unaligned_tensors(cuda, lib, B, CI, CO, G, p):
+    import linfdist_b200 as L
+    torch.manual_seed(B)
+    CI, CO = CI * G, CO * G
+    x, w, g = (off_by_one_float(torch.randn(*s, device="cuda")) for s in ((B, CI, 1), (CO, CI // G), (B, CO, 1)))
+    x.requires_grad_(); w.requires_grad_()
+    y = L.norm_dist(x, w, G, p)
+    gx, gw = torch.autograd.grad(y, [x, w], g)
+    ref = reference(x.detach()[:, :, 0], w.detach(), g[:, :, 0], G, p)
+    limit = 2.0 ** -22 * 4 + p * 2.0 ** -23          # as in `check`
+    for name, a, b in zip(("y", "grad_input", "grad_weight"), (y.detach()[:, :, 0], gx[:, :, 0], gw), ref):
+        assert norm_error(a, b) <= limit, (name, norm_error(a, b), limit)
