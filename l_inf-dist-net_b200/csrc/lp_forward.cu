@@ -60,8 +60,19 @@ __device__ __forceinline__ void load_rows(float* dst, const float* __restrict__ 
     }
 }
 
+// One output by the rule of the generic kernel: a term counts min(|t| / M, 1)^p with min(NaN, 1) = 1, and M is the largest |t| that is a number.
+__device__ __noinline__ float clamped_output(const float* xr, const float* wr, int K, float p, float inv_p) {
+    float M = 0.f, S = 0.f;
+    for (int k = 0; k < K; ++k) M = fmaxf(M, fabsf(__ldg(xr + k) - __ldg(wr + k)));
+    const float rM = M > 0.f ? 1.f / M : 0.f;
+    for (int k = 0; k < K; ++k) S += powf(fminf(fabsf(__ldg(xr + k) - __ldg(wr + k)) * rM, 1.f), p);
+    return M > 0.f ? powf(S, inv_p) * M : 0.f;
+}
+
 // IP: 8, 16, 64 at compile time, 0: p at run time.  TJ: output columns per thread.  AL: rows of x and w can be read 16 bytes at a time.
-template <int IP, int TJ, bool AL>
+// CLAMP: calls that the generic kernel served before this one.  An infinite or NaN difference, or an M so small that 1 / M is infinite, leaves a sum
+// that is not finite, and nothing else does: such outputs are worked out again by that kernel's rule, one thread each.
+template <int IP, int TJ, bool AL, bool CLAMP>
 __global__ void __launch_bounds__(NT, 3)
 lp_forward_kernel(const FwdParams p) {
     extern __shared__ __align__(16) float smem[];
@@ -145,22 +156,29 @@ lp_forward_kernel(const FwdParams p) {
         if (inside(e)) {
             float* yo = out(e);
             const float M = *yo;
-            *yo = M > 0.f ? powf(S[e], p.inv_p) * M : 0.f;
+            float y = M > 0.f ? powf(S[e], p.inv_p) * M : 0.f;
+            if (CLAMP && !(S[e] < __int_as_float(0x7f800000)))
+                y = clamped_output(xg + (size_t)(m0 + row_off + 4 * (e / TJ)) * p.CI, wg + (size_t)(n0 + col_off + 8 * (e % TJ)) * p.CIg, p.CIg, p.p, p.inv_p);
+            *yo = y;
         }
 }
 
-template <int IP, int TJ, bool AL>
+template <int IP, int TJ, bool AL, bool CLAMP>
 int launch_fwd(const FwdParams& P, int grid, cudaStream_t st) {
     constexpr int bytes = STAGES * (TM + 16 * TJ) * LDK * 4;
-    auto kern = lp_forward_kernel<IP, TJ, AL>;
+    auto kern = lp_forward_kernel<IP, TJ, AL, CLAMP>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return LINF_ERR_LAUNCH;
     kern<<<grid, NT, bytes, st>>>(P);
     return launch_status();
 }
+template <int IP, int TJ>
+int launch_fwd_tj(const FwdParams& P, int grid, bool al, bool clamp, cudaStream_t st) {
+    if (!al) return launch_fwd<IP, TJ, false, true>(P, grid, st);
+    return clamp ? launch_fwd<IP, TJ, true, true>(P, grid, st) : launch_fwd<IP, TJ, true, false>(P, grid, st);
+}
 template <int IP>
-int launch_fwd_ip(const FwdParams& P, int grid, bool narrow, bool al, cudaStream_t st) {
-    if (narrow) return al ? launch_fwd<IP, 3, true>(P, grid, st) : launch_fwd<IP, 3, false>(P, grid, st);
-    return al ? launch_fwd<IP, 4, true>(P, grid, st) : launch_fwd<IP, 4, false>(P, grid, st);
+int launch_fwd_ip(const FwdParams& P, int grid, bool narrow, bool al, bool clamp, cudaStream_t st) {
+    return narrow ? launch_fwd_tj<IP, 3>(P, grid, al, clamp, st) : launch_fwd_tj<IP, 4>(P, grid, al, clamp, st);
 }
 
 }  // namespace
@@ -192,11 +210,11 @@ int lp_forward_dense(const float* x, const float* w, const Dims& d, float* y, fl
     P.x = x; P.w = w; P.y = y;
     P.B = d.R; P.COg = d.COg; P.CIg = d.CIg; P.G = d.G; P.CI = d.CI; P.CO = d.CO;
     P.p = p; P.inv_p = 1.f / p;
-    const bool al = (d.CIg & 3) == 0 && aligned16(x) && aligned16(w);
-    if (p == 8.f) return launch_fwd_ip<8>(P, (int)grid, narrow, al, st);
-    if (p == 16.f) return launch_fwd_ip<16>(P, (int)grid, narrow, al, st);
-    if (p == 64.f) return launch_fwd_ip<64>(P, (int)grid, narrow, al, st);
-    return launch_fwd_ip<0>(P, (int)grid, narrow, al, st);
+    const bool al = (d.CIg & 3) == 0 && aligned16(x) && aligned16(w), clamp = !lp_tiled_ok(d, x, w, y, nullptr, nullptr);
+    if (p == 8.f) return launch_fwd_ip<8>(P, (int)grid, narrow, al, clamp, st);
+    if (p == 16.f) return launch_fwd_ip<16>(P, (int)grid, narrow, al, clamp, st);
+    if (p == 64.f) return launch_fwd_ip<64>(P, (int)grid, narrow, al, clamp, st);
+    return launch_fwd_ip<0>(P, (int)grid, narrow, al, clamp, st);
 }
 
 }  // namespace linf

@@ -115,3 +115,51 @@ def test_unaligned_tensors(cuda, lib, B, CI, CO, G, p):
     limit = 2.0 ** -22 * 4 + p * 2.0 ** -23          # as in `check`
     for name, a, b in zip(("y", "grad_input", "grad_weight"), (y.detach()[:, :, 0], gx[:, :, 0], gw), ref):
         assert norm_error(a, b) <= limit, (name, norm_error(a, b), limit)
+
+
+def clamped(x, w, p, y=None, g=None):
+    """What a call that the generic kernel served gives for any data, in double precision: a term is min(|t| / M, 1)^p with min(NaN, 1) = 1, M the
+    largest |t| that is a number; in the gradients min(|t| / y, 1)^(p-1) with 1 / y = 0 where y is not positive, and the sign of x - w or w - x (minus for 0 and NaN)."""
+    t = x.double()[:, None, :] - w.double()[None]
+    unit = lambda u: torch.where(u < 1.0, u, torch.ones_like(u))
+    if g is None:
+        M = torch.where(t.isnan(), torch.zeros_like(t), t.abs()).amax(-1, keepdim=True)
+        S = (unit(t.abs() * torch.where(M > 0, 1 / M, torch.zeros_like(M))) ** p).sum(-1)
+        return torch.where(M[..., 0] > 0, S ** (1 / p) * M[..., 0], torch.zeros_like(S))
+    y = y.double()[..., None]
+    T = unit(t.abs() * torch.where(y > 0, 1 / y, torch.zeros_like(y))) ** (p - 1)
+    T = g.double()[..., None] * T
+    return torch.where(t > 0, T, -T).sum(1), torch.where(t < 0, T, -T).sum(0)
+
+
+def spoil(x, w):
+    x, w = x.clone(), w.clone()
+    x[1, 3, 0], x[2, 5, 0], x[4, 0, 0] = float("inf"), float("nan"), -float("inf")
+    x[7] = float("nan")
+    w[2, 6], w[5, 1], w[9] = float("inf"), float("nan"), float("nan")
+    w[8, 4], x[8, 4, 0] = float("inf"), float("inf")
+    return x, w
+
+
+def assert_same_kind(a, b, limit, what):
+    """Infinities and NaN in the same places, and the numbers close in the 2-norm."""
+    a, b = a.double(), b.double()
+    assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.isposinf(), b.isposinf()) and torch.equal(a.isneginf(), b.isneginf()), what
+    ok = b.isfinite()
+    assert norm_error(a[ok], b[ok]) <= limit, (what, norm_error(a[ok], b[ok]), limit)
+
+
+@pytest.mark.parametrize("p", [8.0, 16.0, 23.7, 64.0, 100.0])
+@pytest.mark.parametrize("B,CI,CO,aligned", [(70, 99, 65, True), (70, 96, 65, True), (203, 1027, 301, True), (130, 64, 36, False)])
+def test_infinities_and_nan_forward(cuda, lib, B, CI, CO, aligned, p):
+    """Calls that are no aligned dense layer: ragged channel counts, tensors off a 16-byte boundary."""
+    import linfdist_b200 as L
+    torch.manual_seed(B)
+    x, w = spoil(torch.randn(B, CI, 1, device="cuda"), torch.randn(CO, CI, device="cuda"))
+    place = (lambda t: t) if aligned else off_by_one_float
+    x, w = place(x), place(w)
+    y = L.norm_dist(x, w, 1, p)[:, :, 0]
+    assert_same_kind(y, clamped(x[:, :, 0], w, p), 2.0 ** -22 * 4 + p * 2.0 ** -23, "y")
+    tiny = 2.0 ** -140          # 1 / M is infinite: every term counts 1
+    y = L.norm_dist(place(torch.full_like(x, tiny)), place(torch.zeros_like(w)), 1, p)
+    assert torch.allclose(y, torch.full_like(y, CI ** (1 / p)) * tiny, rtol=1e-5, atol=2.0 ** -149)
