@@ -115,11 +115,44 @@ struct BothParams {
     size_t gx_step, gw_step;                             // floats between the partial results of consecutive ranges
     int B, Bp, COg, CIg, G, CI;
     int tiles_i, n_o, n_b;                               // 64-column tiles per group, ranges of outputs / of batch tiles
+    int clamp;                                           // results that are not finite: by the rule of `clamped_range`
+    const float* y; const float* gout; int CO;           // [B][CO], for that rule
+    float pm1;
     PowQ q;
 };
 
 template <int WARPS, bool SCALED>
 __host__ __device__ constexpr int stage_floats() { return KO * TI + (SCALED ? 2 : 1) * KO * WARPS * RW; }
+
+// Everything that a CTA owns, columns i0 .. i0 + TI - 1 of its rows b0 .. b1 - 1 of gx and of its outputs o0 .. o1 - 1 of gw, by the rule of the generic kernels: a term
+// counts min(|t| / y, 1)^(p-1) with min(NaN, 1) = 1 and the sign of x - w (gx) or w - x (gw), minus for 0 and NaN.  `gx` and `gw` (null: not wanted): this
+// CTA's partial results, of row 0 and output 0 of the group.  For infinities and NaN in calls that the generic kernels served before this one; slow.
+__device__ __noinline__ void clamped_range(const BothParams& p, int g, int i0, int b0, int b1, int o0, int o1, float* gx, float* gw) {
+    const float* wg = p.w + (size_t)g * p.COg * p.CIg;
+    auto term = [&](int b, int o, float t) {
+        const size_t at = (size_t)b * p.CO + (size_t)g * p.COg + o;
+        const float yv = __ldg(p.y + at), ry = yv > 0.f ? 1.f / yv : 0.f;
+        const float T = __ldg(p.gout + at) * powf(fminf(fabsf(t) * ry, 1.f), p.pm1);
+        return t > 0.f ? T : -T;
+    };
+    const int cols = min(TI, p.CIg - i0);
+    if (gx != nullptr)
+        for (int e = threadIdx.x; e < (b1 - b0) * cols; e += blockDim.x) {
+            const int b = b0 + e / cols, i = i0 + e % cols;
+            const float xv = __ldg(p.x + (size_t)b * p.CI + (size_t)g * p.CIg + i);
+            float a = 0.f;
+            for (int o = o0; o < o1; ++o) a += term(b, o, xv - __ldg(wg + (size_t)o * p.CIg + i));
+            gx[(size_t)b * p.CI + i] = a;
+        }
+    if (gw != nullptr)
+        for (int e = threadIdx.x; e < (o1 - o0) * cols; e += blockDim.x) {
+            const int o = o0 + e / cols, i = i0 + e % cols;
+            const float wv = __ldg(wg + (size_t)o * p.CIg + i);
+            float a = 0.f;
+            for (int b = b0; b < b1; ++b) a += term(b, o, wv - __ldg(p.x + (size_t)b * p.CI + (size_t)g * p.CIg + i));
+            gw[(size_t)o * p.CIg + i] = a;
+        }
+}
 
 template <int IP, int WARPS, bool DOX, bool DOW, bool AL, bool SCALED>
 __device__ __forceinline__ void both_body(const BothParams& p, float* smem) {
@@ -139,6 +172,8 @@ __device__ __forceinline__ void both_body(const BothParams& p, float* smem) {
     const float* sa = (SCALED ? p.g : p.h) + (size_t)g * p.COg * p.Bp;
     const float* sr = p.r + (size_t)g * p.COg * p.Bp;
     float* gw = p.gw + (DOW ? (size_t)rb * p.gw_step : 0) + (size_t)g * p.COg * p.CIg;
+    const float inf = __int_as_float(0x7f800000);
+    bool odd = false;                                    // an infinity or a NaN among the sums (a term enters both: one of the two is looked at)
 
     for (int bt = bt0; bt < bt1; ++bt) {
         const int b_first = bt * BT;
@@ -185,6 +220,7 @@ __device__ __forceinline__ void both_body(const BothParams& p, float* smem) {
                 }
                 const int o = kt * KO + r, i = i0 + c;
                 if (o < p.COg && i < p.CIg) {
+                    if (!DOX) odd |= !(fabsf(v.x) < inf) || (i + 1 < p.CIg && !(fabsf(v.y) < inf));
                     float* dst = gw + (size_t)o * p.CIg + i;
                     if (AL) {                            // CIg is a multiple of four: both columns exist and the pair is aligned
                         if (bt == bt0) *reinterpret_cast<float2*>(dst) = v;
@@ -280,6 +316,8 @@ __device__ __forceinline__ void both_body(const BothParams& p, float* smem) {
                 unpack_f32x2(acc[k][0], a0, a1);
                 unpack_f32x2(acc[k][1], b0, b1);
                 float* dst = gx + (size_t)b * p.CI;
+                // (rows past the batch are 0, columns past the edge anything)
+                odd |= (ic < p.CIg && !(fabsf(a0) < inf && fabsf(a1) < inf)) || (ic + 1 < p.CIg && !(fabsf(b0) < inf && fabsf(b1) < inf));
                 if (AL) {
                     if (ic < p.CIg && b < p.B) *reinterpret_cast<float2*>(dst) = make_float2(a0, b0);
                     if (ic < p.CIg && b + 1 < p.B) *reinterpret_cast<float2*>(dst + p.CI) = make_float2(a1, b1);
@@ -292,12 +330,15 @@ __device__ __forceinline__ void both_body(const BothParams& p, float* smem) {
             }
         }
     }
+    if (p.clamp && __syncthreads_or(odd))
+        clamped_range(p, g, i0, bt0 * BT, min(bt1 * BT, p.B), kt0 * KO, min(kt1 * KO, p.COg),
+                      DOX ? p.gx + (size_t)ro * p.gx_step + (size_t)g * p.CIg : nullptr, DOW ? gw : nullptr);
 }
 
 // 16 warps per SM whatever the CTA's width: 128 registers a thread
 template <int IP, int WARPS, bool DOX, bool DOW, bool AL>
 __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
-lp_backward_both_kernel(const BothParams p) {
+lp_backward_both_kernel(const __grid_constant__ BothParams p) {
     extern __shared__ __align__(16) float smem[];
     if constexpr (IP == 8 || IP == 16) {
         if (*p.flag == 0) { both_body<IP, WARPS, DOX, DOW, AL, false>(p, smem); return; }
@@ -335,7 +376,7 @@ lp_backward_prepare_kernel(const float* __restrict__ g, const float* __restrict_
                 const float rv = yv > 0.f ? 1.f / yv : 0.f;
                 const float off = pm1 * fmaf(rv, yv, -1.f);
                 rt[a] = rv;
-                gt[a] = fabsf(off) < 0.01f ? fmaf(gv, -off, gv) : gv;
+                gt[a] = fabsf(off) < 0.01f && fabsf(gv) < __int_as_float(0x7f800000) ? fmaf(gv, -off, gv) : gv;     // (inf - inf is NaN)
                 if (IP == 8 || IP == 16) {
                     bad |= b < B && !(yv >= LO && yv <= HI);
                     float pw = yv, sq = yv;                   // y^(2^k - 1): 7 or 15
@@ -484,6 +525,9 @@ int lp_backward_both(const float* g, const float* x, const float* w, const float
     P.B = d.R; P.Bp = pl.Bp; P.COg = d.COg; P.CIg = d.CIg; P.G = d.G; P.CI = d.CI;
     P.tiles_i = pl.tiles_i; P.n_o = pl.n_o; P.n_b = pl.n_b;
     P.gx = gx; P.gw = gw;
+    // the tiled kernels never had a rule for infinities and NaN
+    P.clamp = !lp_tiled_ok(d, x, w, y, g, dox ? gx : gw) || (dow && !aligned16(gw)) || p >= 1025.f;
+    P.y = y; P.gout = g; P.CO = d.CO; P.pm1 = p - 1.f;
     if (dox && pl.n_o > 1) { P.gx = next; P.gx_step = pl.gx_step; next += pl.n_o * pl.gx_step; }
     if (dow && pl.n_b > 1) { P.gw = next; P.gw_step = pl.gw_step; }
     const float e = p - 2.f, fl = floorf(e);

@@ -163,3 +163,29 @@ def test_infinities_and_nan_forward(cuda, lib, B, CI, CO, aligned, p):
     tiny = 2.0 ** -140          # 1 / M is infinite: every term counts 1
     y = L.norm_dist(place(torch.full_like(x, tiny)), place(torch.zeros_like(w)), 1, p)
     assert torch.allclose(y, torch.full_like(y, CI ** (1 / p)) * tiny, rtol=1e-5, atol=2.0 ** -149)
+
+
+@pytest.mark.parametrize("p", [8.0, 16.0, 23.7, 64.0, 100.0])
+@pytest.mark.parametrize("B,CI,CO,aligned", [(70, 99, 65, True), (20, 96, 65, True), (203, 1027, 301, True), (2100, 64, 36, False), (2100, 64, 36, True)])
+def test_infinities_and_nan_backward(cuda, lib, B, CI, CO, aligned, p):
+    import linfdist_b200 as L
+    torch.manual_seed(B)
+    x, w = torch.randn(B, CI, 1, device="cuda"), torch.randn(CO, CI, device="cuda")
+    generic = not aligned or CI % 4 != 0 or CO % 4 != 0
+    if generic:
+        x, w = spoil(x, w)      # (aligned layers have no rule for such data: NaN)
+    g = torch.randn(B, CO, 1, device="cuda")
+    place = (lambda t: t) if aligned else off_by_one_float
+    x, w = place(x).requires_grad_(), place(w).requires_grad_()
+    y = L.norm_dist(x, w, 1, p)
+    with torch.no_grad():
+        xs, ws, ys = x[:, :, 0].detach(), w.detach(), y[:, :, 0].detach()
+    limit = 2.0 ** -22 * 4 + p * 2.0 ** -23
+    for bad in (None, float("inf")):
+        if bad is not None and p > 8.0:
+            break               # (factors that underflow in 32 bits: inf * 0)
+        if bad is not None:
+            g[3, 7, 0] = bad
+        grads = torch.autograd.grad(y, [x, w], g, retain_graph=True)
+        for name, a, b in zip(("grad_input", "grad_weight"), (grads[0][:, :, 0], grads[1]), clamped(xs, ws, p, ys, g[:, :, 0])):
+            assert_same_kind(a, b, limit, (name, bad))
