@@ -500,6 +500,14 @@ static bool both_ok(const Dims& d, float p) {
            (ragged ? p >= 8.f && p <= 100.f : d.R >= 2048);
 }
 
+// Calls among them that the two kernels of the separate entry points do better after all.  `tiled`: those would be the tiled ones (lp_tiled_ok).
+// The generic kernels clamp |t| / y to 1, which keeps the error of large powers down: against the same sums in 64 bits, error here / there with p = 150, 300,
+// 1000 (unaligned tensors, 2100 rows, 64 x 64): 1.26, 1.67, 3.0; with p = 64 and 33, 42, 50, 66, 130 inputs: 1.05, 1.03, 1.01, 0.99, 0.96; elsewhere in 8 <= p <= 100, behind
+// the distances as they are now, 0.81 - 0.95.  Against the tiled kernels 0.2 - 0.98 everywhere.
+static bool separate_better(const Dims& d, float p, bool tiled) {
+    return !tiled && (p > 100.f || (p == 64.f && d.CIg < 64));
+}
+
 size_t lp_backward_both_workspace(const Dims& d, float p, bool dox, bool dow) {
     if (!both_ok(d, p) || !(dox || dow)) return 0;
     return plan_both(d, p, dox, dow).words * sizeof(float);
@@ -508,8 +516,9 @@ size_t lp_backward_both_workspace(const Dims& d, float p, bool dox, bool dow) {
 int lp_backward_both(const float* g, const float* x, const float* w, const float* y, const Dims& d,
                      float* gx, float* gw, float p, void* ws, size_t ws_bytes, cudaStream_t st) {
     const bool dox = gx != nullptr, dow = gw != nullptr;
+    const bool tiled = lp_tiled_ok(d, x, w, y, g, dox ? gx : gw) && (!dow || aligned16(gw)) && p < 1025.f;
     const size_t need = lp_backward_both_workspace(d, p, dox, dow);
-    if (need == 0 || ws == nullptr) {        // another path, one gradient at a time
+    if (need == 0 || ws == nullptr || separate_better(d, p, tiled)) {        // one gradient at a time
         if (dox) { const int rc = lp_backward_input(g, x, w, y, d, gx, p, st); if (rc) return rc; }
         return dow ? lp_backward_weight(g, x, w, y, d, gw, p, st) : LINF_OK;
     }
@@ -525,8 +534,7 @@ int lp_backward_both(const float* g, const float* x, const float* w, const float
     P.B = d.R; P.Bp = pl.Bp; P.COg = d.COg; P.CIg = d.CIg; P.G = d.G; P.CI = d.CI;
     P.tiles_i = pl.tiles_i; P.n_o = pl.n_o; P.n_b = pl.n_b;
     P.gx = gx; P.gw = gw;
-    // the tiled kernels never had a rule for infinities and NaN
-    P.clamp = !lp_tiled_ok(d, x, w, y, g, dox ? gx : gw) || (dow && !aligned16(gw)) || p >= 1025.f;
+    P.clamp = !tiled;                        // (the tiled kernels never had a rule for infinities and NaN)
     P.y = y; P.gout = g; P.CO = d.CO; P.pm1 = p - 1.f;
     if (dox && pl.n_o > 1) { P.gx = next; P.gx_step = pl.gx_step; next += pl.n_o * pl.gx_step; }
     if (dow && pl.n_b > 1) { P.gw = next; P.gw_step = pl.gw_step; }

@@ -189,3 +189,27 @@ def test_infinities_and_nan_backward(cuda, lib, B, CI, CO, aligned, p):
         grads = torch.autograd.grad(y, [x, w], g, retain_graph=True)
         for name, a, b in zip(("grad_input", "grad_weight"), (grads[0][:, :, 0], grads[1]), clamped(xs, ws, p, ys, g[:, :, 0])):
             assert_same_kind(a, b, limit, (name, bad))
+
+
+def separate_gradients(lib, x, w, y, g, G, p):
+    """Both gradients by the entry points that work out one each."""
+    B, CI, _ = x.shape
+    CO, s = w.shape[0], torch.cuda.current_stream().cuda_stream
+    gx, gw = torch.empty_like(x), torch.empty_like(w)
+    a = (g.data_ptr(), x.data_ptr(), w.data_ptr(), y.data_ptr(), B, CO, CI, G, 1)
+    assert lib.linf_norm_dist_backward_input(*a, gx.data_ptr(), p, s) == 0
+    assert lib.linf_norm_dist_backward_weight(*a, gw.data_ptr(), p, s) == 0
+    return gx, gw
+
+
+@pytest.mark.parametrize("B,CI,CO,p,aligned", [(2100, 64, 64, 150.0, False), (2048, 36, 40, 1000.0, False), (70, 35, 65, 64.0, True), (2100, 60, 64, 64.0, False)])
+def test_large_powers_keep_the_clamped_kernels(cuda, lib, B, CI, CO, p, aligned):
+    import linfdist_b200 as L
+    torch.manual_seed(B)
+    place = (lambda t: t) if aligned else off_by_one_float
+    x, w, g = (place(torch.randn(*s, device="cuda")) for s in ((B, CI, 1), (CO, CI), (B, CO, 1)))
+    x.requires_grad_(); w.requires_grad_()
+    y = L.norm_dist(x, w, 1, p)
+    got = torch.autograd.grad(y, [x, w], g)
+    want = separate_gradients(lib, x.detach(), w.detach(), y.detach(), g, 1, p)
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
