@@ -12,8 +12,8 @@
 // eight outputs.  All arithmetic is packed two rows at a time (f32x2).
 //
 // p = 8 and 16 run without the division by y: T = h * t^(p-1) with h = g / y^(p-1) worked out once per (b, o)
-// by the preparation kernel, which also looks whether every y lies where neither factor can leave the range of
-// a float; if one does not, the kernel takes the scaled form instead (`flag`).  Per term of both gradients:
+// by the preparation kernel, which also looks whether every y lies where t^(p-1) cannot leave the range of
+// a float and whether every h is 0 for g = 0 or else a normal number; if not, the kernel takes the scaled form instead (`flag`).  Per term of both gradients:
 // 7 lane operations at p = 8 (subtraction, four products, two multiply-adds) against 2 x 7 of two separate passes.
 //
 // Work split.  A CTA owns 64 input columns, a range of outputs and a range of batch tiles (16 rows per warp).
@@ -347,7 +347,7 @@ lp_backward_both_kernel(const __grid_constant__ BothParams p) {
 }
 
 // 1 / y (0 where y is not positive) and grad_output, less the rounding of 1 / y, transposed to [CO][Bp] (rows past the batch: zero), and for
-// p = 8 / 16 the factor h = g / y^(p-1) with the look at the range of y.  With y in [2^-8, 2^8] (p = 8) or [2^-3, 2^4] (p = 16)
+// p = 8 / 16 the factor h = g / y^(p-1) with the look at the range of y and h.  With y in [2^-8, 2^8] (p = 8) or [2^-3, 2^4] (p = 16)
 // y^(p-1) and its reciprocal stay within 2^+-60, and a difference whose power underflows is below 2^-70 of its row's y^(p-1).
 template <int IP>
 __global__ void __launch_bounds__(256)
@@ -382,7 +382,9 @@ lp_backward_prepare_kernel(const float* __restrict__ g, const float* __restrict_
                     float pw = yv, sq = yv;                   // y^(2^k - 1): 7 or 15
 #pragma unroll
                     for (int n = 2; n < IP; n *= 2) { sq *= sq; pw *= sq; }
-                    ht[a] = b < B ? gv / pw : 0.f;
+                    const float hv = b < B ? gv / pw : 0.f;
+                    bad |= gv != 0.f && !(fabsf(hv) >= 0x1p-126f && fabsf(hv) < __int_as_float(0x7f800000));
+                    ht[a] = hv;
                 }
             }
         }

@@ -213,3 +213,12 @@ def test_large_powers_keep_the_clamped_kernels(cuda, lib, B, CI, CO, p, aligned)
     got = torch.autograd.grad(y, [x, w], g)
     want = separate_gradients(lib, x.detach(), w.detach(), y.detach(), g, 1, p)
     assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("p,size,g_size", [(16.0, 2.0, 2.0 ** -75), (16.0, 2.0, 2.0 ** -100), (8.0, 16.0, 2.0 ** -95), (8.0, 1.0, 2.0 ** -60)])
+def test_gradients_of_small_grad_output(cuda, lib, p, size, g_size):
+    """g / y^(p-1) below the normal numbers although the gradients are not."""
+    import linfdist_b200 as L
+    torch.manual_seed(4)
+    x, w, g = (torch.randn(*s, device="cuda") for s in ((70, 99, 1), (65, 99), (70, 65, 1)))
+    check(L, x * size, w * size, g * g_size, 1, p)
