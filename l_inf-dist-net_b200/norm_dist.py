@@ -444,7 +444,7 @@ class NormDistConv(nn.Module):
         return (x.is_cuda and x.dtype == torch.float32 and x.dim() == 4 and x.numel() > 0 and ho > 0 and wo > 0 and ho * wo > 1
                 and not (self.kernel_size == 1 and self.stride == 1 and self.padding == 0)
                 and self.weight[0].numel() % 4 == 0 and self.weight.size(0) // self.group >= 32
-                and x.size(0) * ho * wo * x.size(1) * self.kernel_size ** 2 < 2 ** 31)
+                and x.numel() < 2 ** 31 and x.size(0) * ho * wo * x.size(1) * self.kernel_size ** 2 < 2 ** 31)
 
     def _post(self, t):
         if self.normalize is not None:
