@@ -274,9 +274,10 @@ inf_bound_tiled_kernel(const BoundParams p) {
     }
 }
 
-// The per-channel epilogue as a pass of its own, for launches that combined partial results in memory.
+// The per-channel epilogue as a pass of its own, for launches that combined partial results in memory.  only_if: as above.
 __global__ void __launch_bounds__(256)
-inf_bound_post_kernel(float* __restrict__ yl, float* __restrict__ yu, size_t n, int CO, Post post) {
+inf_bound_post_kernel(float* __restrict__ yl, float* __restrict__ yu, size_t n, int CO, Post post, const int* __restrict__ only_if) {
+    if (only_if != nullptr && *only_if == 0) return;
     for (size_t e = (size_t)blockIdx.x * 256 + threadIdx.x; e < n; e += (size_t)gridDim.x * 256) {
         const int c = (int)(e % (size_t)CO);
         const float lo = post_apply(post, yl[e], c), up = post_apply(post, yu[e], c);
@@ -285,8 +286,17 @@ inf_bound_post_kernel(float* __restrict__ yl, float* __restrict__ yu, size_t n, 
     }
 }
 
+// CTAs per output tile, each with an equal share of the reduction.  Output tiles that leave much of their last wave of CTAs idle, with long rows: two
+// (1.58 -> 1.2 ms at B = 512, Din = 3072, Dout = 5120: 640 tiles on 444 CTA slots; B = 256, 13000 x 1024: 1.53 -> 0.75 ms).
+int k_split(int tiles, int KT) {
+    const int slots = 3 * sm_count();
+    auto fill = [&](int n) { return (double)n / ((double)((n + slots - 1) / slots) * slots); };
+    return KT >= 64 && fill(2 * tiles) > 1.15 * fill(tiles) ? 2 : 1;
+}
+
 }  // namespace
 
+// only_if: not null: nothing is done where this word is 0, and where it is not, the outputs have been cleared on the device.
 int inf_bound(const float* xl, const float* xu, const float* w, const Dims& d,
               float* yl, float* yu, cudaStream_t st, const Post& post, const int* only_if) {
     const bool tiled = d.HW == 1 && (d.CIg % 4) == 0 && aligned16(xl) && aligned16(xu) && aligned16(w) &&
@@ -304,23 +314,14 @@ int inf_bound(const float* xl, const float* xu, const float* w, const Dims& d,
     p.M = d.R; p.N = d.COg; p.K = d.CIg; p.G = d.G; p.lda = d.CI; p.ldo = d.CO;
     p.post = post;
     p.only_if = only_if;
-    p.ksplit = 1;
     p.tiles_m = (d.R + BM - 1) / BM; p.tiles_n = (d.COg + BN - 1) / BN;
     p.KT = (d.CIg + BK - 1) / BK;
     int grid = p.tiles_m * p.tiles_n * d.G;
-    {
-        // Output tiles that leave much of their last wave of CTAs idle, with long rows: two CTAs per tile (1.58 ->
-        // 1.2 ms at B = 512, Din = 3072, Dout = 5120: 640 tiles on 444 CTA slots).
-        const int slots = 3 * sm_count();
-        auto fill = [&](int n) { return (double)n / ((double)((n + slots - 1) / slots) * slots); };
-        // (not behind the list pass: the outputs would have to be cleared under its condition)
-        if (only_if == nullptr && p.KT >= 64 && fill(2 * grid) > 1.15 * fill(grid)) {
-            const size_t bytes = (size_t)d.R * d.CO * sizeof(float);
-            if (cudaMemsetAsync(yl, 0, bytes, st) != cudaSuccess || cudaMemsetAsync(yu, 0, bytes, st) != cudaSuccess)
-                return LINF_ERR_LAUNCH;
-            p.ksplit = 2;
-            grid *= 2;
-        }
+    p.ksplit = k_split(grid, p.KT);
+    grid *= p.ksplit;
+    if (p.ksplit > 1 && only_if == nullptr) {
+        const size_t bytes = (size_t)d.R * d.CO * sizeof(float);
+        if (cudaMemsetAsync(yl, 0, bytes, st) != cudaSuccess || cudaMemsetAsync(yu, 0, bytes, st) != cudaSuccess) return LINF_ERR_LAUNCH;
     }
     // opting in to > 48 KB of dynamic shared memory is per function and per device; repeating it on
     // every call is cheap and keeps the launcher free of per-device state
@@ -331,7 +332,7 @@ int inf_bound(const float* xl, const float* xu, const float* w, const Dims& d,
     int launched = 1;
     if (p.ksplit > 1 && (post.sub != nullptr || post.add != nullptr || post.negate)) {
         const size_t n = (size_t)d.R * d.CO;
-        inf_bound_post_kernel<<<2 * sm_count(), 256, 0, st>>>(yl, yu, n, d.CO, post);
+        inf_bound_post_kernel<<<2 * sm_count(), 256, 0, st>>>(yl, yu, n, d.CO, post, only_if);
         launched = 2;
     }
     return launch_status(launched);

@@ -443,14 +443,18 @@ __global__ void __launch_bounds__(128)
 fail_kernel(const PruneParams p) {
     __shared__ float s_t[4], s_u[4];
     __shared__ int s_i[4];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n = p.head->n_fail;
-    if (n > p.fail_cap) {
-        // too many: the dense kernel behind this one does the layer
-        if (blockIdx.x == 0 && threadIdx.x == 0) p.head->dense = 1;
+    if (n > p.fail_cap || p.head->dense) {
+        // too many, or lists that do not serve: the dense kernel behind this one does the layer.  That of the bounds may combine partial
+        // results in memory: the outputs are cleared for it.
+        if (blockIdx.x == 0 && tid == 0) p.head->dense = 1;
+        if (BOUND) {
+            const size_t outs = (size_t)p.R * p.CO;
+            for (size_t e = (size_t)blockIdx.x * 128 + tid; e < outs; e += (size_t)gridDim.x * 128) { p.y0[e] = 0.f; p.y1[e] = 0.f; }
+        }
         return;
     }
-    if (p.head->dense) return;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (int q = blockIdx.x; q < n; q += gridDim.x) {
         const int e = p.fail[q], r = e / p.CO, c = e - r * p.CO, g = c / p.N;
         const size_t xa = (size_t)r * p.CI + (size_t)g * p.K;

@@ -64,3 +64,27 @@ def test_same_bits_as_the_full_scan(cuda, lib, B, CI, CO, G, kind):
         assert lib.linf_inf_dist_bound_pruned(lo.data_ptr(), up.data_ptr(), w.data_ptr(), *sizes, *post, a[0].data_ptr(), a[1].data_ptr(), ws.data_ptr(), n, s) == 0
         assert lib.linf_inf_dist_bound_forward_post(lo.data_ptr(), up.data_ptr(), w.data_ptr(), *sizes, *post, a[2].data_ptr(), a[3].data_ptr(), s) == 0
         assert torch.equal(clean(a[0]), clean(a[2])) and torch.equal(clean(a[1]), clean(a[3]))
+
+
+@pytest.mark.parametrize("kind", ["tight", "spikes", "special"])
+@pytest.mark.parametrize("B,CI,CO,G", [(256, 2048, 1024, 1), (520, 2060, 1300, 2)])
+def test_bounds_by_two_halves_behind_the_lists(cuda, lib, B, CI, CO, G, kind):
+    """Data that the lists do not serve, at sizes where the dense kernel behind them splits the reduction: the halves meet in outputs that
+    the list pass has written before."""
+    torch.manual_seed(B)
+    CI, CO = CI * G, CO * G
+    x, w = make_x(kind, B, CI, 1), torch.randn(CO, CI // G, device="cuda")
+    if kind == "tight":
+        x, w = torch.rand_like(x), torch.rand_like(w)
+    lo, up = x - 0.03, x + 0.03
+    if kind == "special":
+        lo[2, 4] = up[2, 4] + 1.0
+    s, sizes = torch.cuda.current_stream().cuda_stream, (B, CO, CI, G, 1)
+    sub, add = torch.randn(CO, device="cuda"), torch.randn(CO, device="cuda")
+    n = lib.linf_inf_dist_bound_pruned_workspace_bytes(*sizes)
+    ws = torch.empty(n, dtype=torch.uint8, device="cuda")
+    for post in ((None, None, 0), (sub.data_ptr(), add.data_ptr(), 1)):
+        a = [torch.full((B, CO, 1), 1e30, device="cuda") for _ in range(4)]
+        assert lib.linf_inf_dist_bound_pruned(lo.data_ptr(), up.data_ptr(), w.data_ptr(), *sizes, *post, a[0].data_ptr(), a[1].data_ptr(), ws.data_ptr(), n, s) == 0
+        assert lib.linf_inf_dist_bound_forward_post(lo.data_ptr(), up.data_ptr(), w.data_ptr(), *sizes, *post, a[2].data_ptr(), a[3].data_ptr(), s) == 0
+        assert torch.equal(a[0].nan_to_num(7.0), a[2].nan_to_num(7.0)) and torch.equal(a[1].nan_to_num(7.0), a[3].nan_to_num(7.0))
