@@ -336,7 +336,9 @@ gather_kernel(const PruneParams p, int blocks_a, int splits) {
     const int per = ((NL + splits - 1) / splits + RW - 1) / RW * RW;
     const int l_end = min(NL, (split + 1) * per);
     const float bound = p.head->bound;
+    [[maybe_unused]] bool lost = false;
     for (int l0 = split * per + (tid >> 5) * RW; l0 < l_end; l0 += (nt >> 5) * RW) {
+        if (W_LISTS && __any_sync(FULL, lost)) return;      // more outputs failed than fail_kernel takes: the dense kernel does the layer
         const int l = l0 + lane / LG;
         const int n = l < l_end ? __ldg(cnt + l) : 0;
         const int most = __reduce_max_sync(FULL, n);
@@ -410,7 +412,7 @@ gather_kernel(const PruneParams p, int blocks_a, int splits) {
                         L = p.post.negate ? up : lo; U2 = p.post.negate ? lo : up;
                     } else {
                         const int s = atomicAdd(&p.head->n_fail, 1);
-                        if (s < p.fail_cap) p.fail[s] = (int)e;
+                        if (s < p.fail_cap) p.fail[s] = (int)e; else lost = true;
                     }
                 }
                 p.y0[e] = L; p.y1[e] = U2;
@@ -425,7 +427,7 @@ gather_kernel(const PruneParams p, int blocks_a, int splits) {
                     }
                     if (!(best > bound)) {
                         const int s = atomicAdd(&p.head->n_fail, 1);
-                        if (s < p.fail_cap) p.fail[s] = (int)e;
+                        if (s < p.fail_cap) p.fail[s] = (int)e; else lost = true;
                     }
                     best = post_apply(p.post, best, c);
                 }
