@@ -31,7 +31,7 @@ namespace {
 constexpr unsigned FULL = 0xffffffffu;
 constexpr int kBins = 4096, kBinShift = 19;     // bins of |v|: exponent and four bits of the mantissa
 constexpr int kSampleCtas = 128;
-constexpr int kMaxList = 512;                   // slots per row (the thresholds aim at 0.6 of them at most)
+constexpr int kMaxList = 512;                   // slots per row at most (the thresholds aim at 0.6 of them)
 constexpr int kMaxK = 14000;                    // 16 bytes each in shared memory
 
 struct Head {                                   // zeroed before every call
@@ -517,8 +517,12 @@ struct PruneSizes { size_t head, cnt_x, cnt_w, list_x, list_w, fail, total; int 
 
 PruneSizes prune_sizes(const Dims& d, bool bound) {
     PruneSizes s;
-    s.slots = kMaxList < d.CIg ? kMaxList : d.CIg;
     const size_t nx = (size_t)d.R * d.G, outs = (size_t)d.R * d.CO;
+    // The lists take 64 MB or, where that is more, half of the call's own tensors: the rows of a large convolution would ask for more than those
+    // (131072 rows: 0.5 GB, bounds 1 GB).  20 to 250 entries are what rows have; longer lists than the slots hold send the layer to the dense kernel.
+    const size_t own = sizeof(float) * ((bound ? 2 : 1) * (size_t)d.R * d.CI + (size_t)d.CO * d.CIg + 2 * outs);
+    const size_t slots = max((size_t)64 << 20, own / 2) / (nx * (bound ? 16 : 8) + (size_t)d.CO * 8);
+    s.slots = (int)min(slots, (size_t)min(kMaxList, d.CIg));
     s.fail_cap = (int)(outs / 128 + 1024);
     size_t at = 0;
     s.head = at; at += up256(sizeof(Head) + 2 * kBins * sizeof(int));
