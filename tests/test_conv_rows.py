@@ -36,3 +36,8 @@ def test_weight_gradient_of_few_rows(cuda, lib, R, CI, CO, G):
     gd, pd, gw = g.cuda(), pos.cuda(), torch.empty(CO, CI // G, device="cuda")
     assert lib.linf_inf_dist_backward_weight(gd.data_ptr(), pd.data_ptr(), R, CO, CI, G, 1, gw.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
     assert np.array_equal(gw.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("above", [0, 1])
+def test_weight_gradient_at_the_most_rows_of_the_bins_kernel(cuda, lib, above):
+    test_weight_gradient_of_few_rows(cuda, lib, 1100, 52, torch.cuda.get_device_properties(0).multi_processor_count + above, 1)
