@@ -189,7 +189,7 @@ int inf_backward_ordered_both(const float* g, const int* pos, const Dims& d, flo
 int unfold_rows(const float* x, int B, int C, int H, int W, int k, int dil, int pad, int stride, float* rows, cudaStream_t st);
 int fold_rows(const float* rows, int B, int C, int H, int W, int k, int dil, int pad, int stride, float* gx, cudaStream_t st);
 // a handful of input rows (few_rows.cu)
-bool inf_few_rows_ok(const Dims& d);
+bool inf_few_rows_ok(const Dims& d, bool tiled);
 int inf_forward_few_rows(const float* x, const float* w, const Dims& d, float* y, int* pos, cudaStream_t st, const Post& post);
 // few output channels per group (skinny.cu)
 bool skinny_ok(const Dims& d, const void* a, const void* b, const void* c);

@@ -73,8 +73,17 @@ int launch_few(const float* x, const float* w, const Dims& d, float* y, int* pos
 
 }  // namespace
 
-bool inf_few_rows_ok(const Dims& d) { 
-    return d.HW == 1 && d.COg >= 32 && (d.R <= 8 || (d.R <= 16 && (long long)d.CO * d.CIg <= 16000000));
+// tiled: the alternative is the tiled kernel (else the generic one, which is 6 - 40 times slower).  That one is faster for rows so long that the warps of a CTA,
+// each at its own place, do not find them in L1 any more, unless there are few weights (then it has few CTAs).  us, tiled / here, rows x Din x Dout:
+// 8 x 16384 x 2048 199 / 183, 8 x 24576 x 1024 189 / 287, 8 x 24576 x 512 > 170 / 145, 5 x 24576 x 1024 186 / 165, 3 x 49152 x 512 249 / 200, 4 x 49152 x 512 248 / 280, 8 x 49152 x 128
+// 452 / 247, 4 x 65536 x 512 285 / 375; 2 x 98304 x 512 391 / 327, 2 x 150528 x 256 450 / 508; 8 x 150528 x 64 848 / 747, 8 x 196608 x 64 866 / 972; 1 x 196608 x 512 590 / 513.
+bool inf_few_rows_ok(const Dims& d, bool tiled) {
+    const double weights = (double)d.CO * d.CIg;
+    if (!(d.HW == 1 && d.COg >= 32 && (d.R <= 8 || (d.R <= 16 && weights <= 16e6)))) return false;
+    const int rows = d.R < 8 ? d.R : 8;
+    const double staged = (double)rows * d.CIg;
+    if (!tiled || rows == 1) return true;
+    return staged <= 1.3e6 && !(rows == 2 ? staged > 2.5e5 && weights > 32e6 : staged > 1.6e5 && weights > 16e6);
 }
 
 int inf_forward_few_rows(const float* x, const float* w, const Dims& d, float* y, int* pos, cudaStream_t st, const Post& post) {

@@ -809,7 +809,7 @@ static int launch_tiled(const Kernels& k, const TiledParams& p, bool track, cuda
 
 int inf_forward(const float* x, const float* w, const Dims& d, float* y, int* pos,
                 void* ws, size_t ws_bytes, cudaStream_t st, const Post& post, const int* only_if) {
-    if (inf_few_rows_ok(d) && inf_forward_rows != 1) return inf_forward_few_rows(x, w, d, y, pos, st, post);
+    if (inf_few_rows_ok(d, tiled_ok(x, w, d)) && inf_forward_rows != 1) return inf_forward_few_rows(x, w, d, y, pos, st, post);
     if (!tiled_ok(x, w, d)) {
         if (only_if == nullptr && skinny_ok(d, x, w, nullptr)) return inf_forward_skinny(x, w, d, y, pos, st, post);
         dim3 grid((d.R + GT - 1) / GT, (d.COg + GT - 1) / GT, d.G);

@@ -28,3 +28,9 @@ def test_same_bits(cuda, lib, B, CI, CO, G):
         lib.linf_tune_set(8, 0)
     for a, b in zip(*got):
         assert torch.equal(torch.nan_to_num(a), torch.nan_to_num(b))
+
+
+@pytest.mark.parametrize("B,CI,CO", [(8, 20000, 800), (8, 20004, 1024), (2, 125004, 264), (3, 53400, 304), (16, 165000, 33)])
+def test_same_bits_at_long_rows(cuda, lib, B, CI, CO):
+    """Either side of the line above which the tiled kernel takes long rows."""
+    test_same_bits(cuda, lib, B, CI, CO, 1)
