@@ -9,10 +9,10 @@
 //
 // Without the scale (p = 8, 16: sums checked against the range of a float afterwards) and the maximum pass this takes 1.87 ms instead of
 // 2.72 ms at B = 512, Din = Dout = 5120, p = 8, and the result is as exact.  It is not used: a training run at finite p amplifies the last
-// bit of a distance within two steps (hinge loss, Adam with eps = 1e-10), and runs are kept reproducible from version to version.
+// bit of a distance within two steps (hinge loss, Adam with eps = 1e-10), and the nets, whose layers are all aligned, give the same bits from version to version.
 // Measured on one B200, us, with the maximum pass (dense value-only kernel before, lists of large entries now), scale and squarings packed:
-// B = 512, Din = Dout = 5120: p = 8 3066 -> 2719, 16 3460 -> 3077, 64 4222 -> 3831, 23.7 7118 -> 6726; B = 203, Din = 1027, Dout = 1333 (the generic
-// kernel before): p = 8 683 -> 310 with the generic kernel's maximum; B = 500, Din = 2050, Dout = 3001: 6266 -> 942.
+// B = 512, Din = Dout = 5120: p = 8 3066 -> 2719, 16 3460 -> 3077, 64 4222 -> 3831, 23.7 7118 -> 6726; ragged layers (the generic kernel before): B = 203, Din = 1027,
+// Dout = 1333, p = 8 677 -> 221, 23.7 897 -> 377; B = 500, Din = 2050, Dout = 3001, p = 8: 6260 -> 938, 23.7 8050 -> 2030.
 #include <math.h>
 
 #include "common.cuh"
@@ -60,12 +60,12 @@ __device__ __forceinline__ void load_rows(float* dst, const float* __restrict__ 
     }
 }
 
-// One output by the rule of the generic kernel: a term counts min(|t| / M, 1)^p with min(NaN, 1) = 1, and M is the largest |t| that is a number.
-__device__ __noinline__ float clamped_output(const float* xr, const float* wr, int K, float p, float inv_p) {
-    float M = 0.f, S = 0.f;
-    for (int k = 0; k < K; ++k) M = fmaxf(M, fabsf(__ldg(xr + k) - __ldg(wr + k)));
+// One output by the rule of the generic kernel: a term counts min(|t| / M, 1)^p with min(NaN, 1) = 1, where M is the largest |t| that is a number.
+__device__ __noinline__ float clamped_output(const float* xr, const float* wr, int K, float M, float p, float inv_p) {
     const float rM = M > 0.f ? 1.f / M : 0.f;
-    for (int k = 0; k < K; ++k) S += powf(fminf(fabsf(__ldg(xr + k) - __ldg(wr + k)) * rM, 1.f), p);
+    float S = 0.f;
+#pragma unroll 8
+    for (int k = 0; k < K; ++k) S += ex2_approx(p * lg2_approx(fminf(fabsf(__ldg(xr + k) - __ldg(wr + k)) * rM, 1.f)));
     return M > 0.f ? powf(S, inv_p) * M : 0.f;
 }
 
@@ -158,7 +158,7 @@ lp_forward_kernel(const FwdParams p) {
             const float M = *yo;
             float y = M > 0.f ? powf(S[e], p.inv_p) * M : 0.f;
             if (CLAMP && !(S[e] < __int_as_float(0x7f800000)))
-                y = clamped_output(xg + (size_t)(m0 + row_off + 4 * (e / TJ)) * p.CI, wg + (size_t)(n0 + col_off + 8 * (e % TJ)) * p.CIg, p.CIg, p.p, p.inv_p);
+                y = clamped_output(xg + (size_t)(m0 + row_off + 4 * (e / TJ)) * p.CI, wg + (size_t)(n0 + col_off + 8 * (e % TJ)) * p.CIg, p.CIg, M, p.p, p.inv_p);
             *yo = y;
         }
 }
