@@ -527,8 +527,15 @@ static bool both_ok(const Dims& d, float p) {
 // The generic kernels clamp |t| / y to 1, which keeps the error of large powers down: against the same sums in 64 bits, error here / there with p = 150, 300,
 // 1000 (unaligned tensors, 2100 rows, 64 x 64): 1.26, 1.67, 3.0; with p = 64 and 33, 42, 50, 66, 130 inputs: 1.05, 1.03, 1.01, 0.99, 0.96; elsewhere in 8 <= p <= 100, behind
 // the distances as they are now, 0.81 - 0.95.  Against the tiled kernels 0.2 - 0.98 everywhere.
-static bool separate_better(const Dims& d, float p, bool tiled) {
-    return !tiled && (p > 100.f || (p == 64.f && d.CIg < 64));
+// One gradient alone: the power is not shared, and small calls are a matter of launches (this path has two or three).  us, there / here, rows x Din x Dout: grad_input against the
+// tiled kernel, p = 8: 2048 x 64 x 64 18 / 26, 16384 x 144 x 64 64 / 80, 4096 x 128 x 64 18 / 30, 2048 x 128 x 128 32 / 30, 3000 x 300 x 300 104 / 98; p = 23.7: 2048 x 64 x 64 71 / 26,
+// 16384 x 64 x 64 73 / 88.  Against the generic kernels, p = 8: grad_weight 8 x 514 x 514 12 / 21, 16 x 300 x 130 13 / 19, 32 x 65 x 65 17 / 19, 16 x 1027 x 1333 41 / 28; grad_input
+// 64 x 99 x 37 20 / 22, 64 x 300 x 130 55 / 22.
+static bool separate_better(const Dims& d, float p, bool tiled, bool dox, bool dow) {
+    if (!tiled && (p > 100.f || (p == 64.f && d.CIg < 64))) return true;
+    if (dox && dow) return false;
+    if (tiled) return dox && d.COg < 128 && (p == 8.f || p == 16.f || p == 64.f || (d.R >= 8192 && p < 64.f));
+    return (double)d.R * d.CO * d.CIg < 4e6 && (dow ? d.R <= 16 : d.COg < 48 && p <= 16.f);
 }
 
 size_t lp_backward_both_workspace(const Dims& d, float p, bool dox, bool dow) {
@@ -541,7 +548,7 @@ int lp_backward_both(const float* g, const float* x, const float* w, const float
     const bool dox = gx != nullptr, dow = gw != nullptr;
     const bool tiled = lp_tiled_ok(d, x, w, y, g, dox ? gx : gw) && (!dow || aligned16(gw)) && p < 1025.f;
     const size_t need = lp_backward_both_workspace(d, p, dox, dow);
-    if (need == 0 || ws == nullptr || separate_better(d, p, tiled)) {        // one gradient at a time
+    if (need == 0 || ws == nullptr || separate_better(d, p, tiled, dox, dow)) {        // one gradient at a time
         if (dox) { const int rc = lp_backward_input(g, x, w, y, d, gx, p, st); if (rc) return rc; }
         return dow ? lp_backward_weight(g, x, w, y, d, gw, p, st) : LINF_OK;
     }

@@ -222,3 +222,15 @@ def test_gradients_of_small_grad_output(cuda, lib, p, size, g_size):
     torch.manual_seed(4)
     x, w, g = (torch.randn(*s, device="cuda") for s in ((70, 99, 1), (65, 99), (70, 65, 1)))
     check(L, x * size, w * size, g * g_size, 1, p)
+
+
+@pytest.mark.parametrize("B,CI,CO,p,alone", [(2048, 64, 64, 8.0, "input"), (8200, 64, 36, 23.7, "input"), (16, 130, 65, 23.7, "weight"), (70, 99, 37, 8.0, "input")])
+def test_one_gradient_that_its_own_kernel_does(cuda, lib, B, CI, CO, p, alone):
+    import linfdist_b200 as L
+    torch.manual_seed(B)
+    x, w, g = (torch.randn(*s, device="cuda") for s in ((B, CI, 1), (CO, CI), (B, CO, 1)))
+    (x if alone == "input" else w).requires_grad_()
+    y = L.norm_dist(x, w, 1, p)
+    got, = torch.autograd.grad(y, [x if alone == "input" else w], g)
+    want = separate_gradients(lib, x.detach(), w.detach(), y.detach(), g, 1, p)
+    assert torch.equal(got, want[0 if alone == "input" else 1])
