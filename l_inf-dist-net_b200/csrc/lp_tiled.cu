@@ -9,8 +9,8 @@
 //
 // s * |s|^(p-2) equals |t/y|^(p-1) * sign(t) and keeps the sign for free.  IP > 0 instantiates an
 // integer p known at compile time (8, 16, 64: the powers are a handful of multiplies on the FP32
-// pipe); IP == 0 takes p at run time (integer part by square-and-multiply, fractional part by one
-// log2/exp2 pair on the special-function unit, skipped when p is an integer).
+// pipe); IP < 0 takes p at run time, the integer part of p - 1 having at most -IP bits (integer part by square-and-multiply,
+// fractional part by one log2/exp2 pair on the special-function unit, skipped when p is an integer).
 #include <math.h>
 
 #include "common.cuh"
@@ -45,8 +45,6 @@ __device__ __forceinline__ float pow_bits(float a, const Pw q) {
     return r;
 }
 
-// Template parameter IP of the kernels: IP > 0 is an integer p fixed at compile time; IP <= 0 takes
-// p at run time (backward: -IP = number of bits of the integer part of p - 1).
 
 // a^E of a pair, E >= 1
 template <int E>
@@ -78,7 +76,7 @@ __device__ __forceinline__ void add_terms(const float* fixed, const float* other
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const float s = (fixed[j] - other[j]) * ry;
-            acc[j] = fmaf(g, copysignf(pow_bits<(IP < 0 ? -IP : 2)>(fabsf(s), q), s), acc[j]);
+            acc[j] = fmaf(g, copysignf(pow_bits<-IP>(fabsf(s), q), s), acc[j]);
         }
     }
 }
