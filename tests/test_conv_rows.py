@@ -41,3 +41,30 @@ def test_weight_gradient_of_few_rows(cuda, lib, R, CI, CO, G):
 @pytest.mark.parametrize("above", [0, 1])
 def test_weight_gradient_at_the_most_rows_of_the_bins_kernel(cuda, lib, above):
     test_weight_gradient_of_few_rows(cuda, lib, 1100, 52, torch.cuda.get_device_properties(0).multi_processor_count + above, 1)
+
+
+@pytest.mark.parametrize("p", [float("inf"), 8.0, 23.7])
+@pytest.mark.parametrize("form", ["contiguous", "channels_last", "sliced"])
+@pytest.mark.parametrize("group,stride,padding,dilation", [(1, 1, 1, 1), (2, 2, 0, 2)])
+def test_module_on_patch_rows(cuda, lib, p, form, group, stride, padding, dilation):
+    """Value and gradients of a NormDistConv against torch's unfold and one dense call per image, whatever the image's strides."""
+    import linfdist_b200 as L
+    torch.manual_seed(5)
+    layer = L.NormDistConv(16, 64, 3, stride=stride, padding=padding, dilation=dilation, group=group, p=p, bias=True).cuda()
+    x = torch.randn(6, 16, 13, 14, device="cuda")
+    if form == "channels_last":
+        x = x.contiguous(memory_format=torch.channels_last)
+    if form == "sliced":
+        x = torch.randn(6, 20, 13, 20, device="cuda")[:, 2:18, :, 3:17]
+    x.requires_grad_()
+    y = layer(x)[0]
+    g = torch.randn_like(y)
+    got = torch.autograd.grad(y, [x, layer.weight, layer.bias], g)
+    cols = F.unfold(x, 3, dilation, padding, stride)                     # [B, C * 9, L]
+    per_image = [L.norm_dist(c.t().unsqueeze(-1).contiguous(), layer.weight.view(64, -1), group, p) for c in cols]
+    want_y = torch.stack([v[:, :, 0].t() for v in per_image]).view_as(y) + layer.bias.view(1, -1, 1, 1)
+    want = torch.autograd.grad(want_y, [x, layer.weight, layer.bias], g)
+    limit = 1e-6 if p == float("inf") else 2.0 ** -20 + p * 2.0 ** -22       # rounding of the terms, twice that of a call against 64 bits
+    assert torch.linalg.norm(y - want_y) <= limit * torch.linalg.norm(want_y)
+    for a, b in zip(got, want):
+        assert torch.linalg.norm(a - b) <= max(limit, 1e-5) * torch.linalg.norm(b)

@@ -88,3 +88,101 @@ def test_bounds_by_two_halves_behind_the_lists(cuda, lib, B, CI, CO, G, kind):
         assert lib.linf_inf_dist_bound_pruned(lo.data_ptr(), up.data_ptr(), w.data_ptr(), *sizes, *post, a[0].data_ptr(), a[1].data_ptr(), ws.data_ptr(), n, s) == 0
         assert lib.linf_inf_dist_bound_forward_post(lo.data_ptr(), up.data_ptr(), w.data_ptr(), *sizes, *post, a[2].data_ptr(), a[3].data_ptr(), s) == 0
         assert torch.equal(a[0].nan_to_num(7.0), a[2].nan_to_num(7.0)) and torch.equal(a[1].nan_to_num(7.0), a[3].nan_to_num(7.0))
+
+
+def off_by_one_float(t):
+    """The same values in memory that starts 4 bytes past a 16-byte boundary."""
+    return torch.empty(t.numel() + 4, dtype=t.dtype, device=t.device)[1: 1 + t.numel()].view(t.shape).copy_(t)
+
+
+def pruned_forward(lib, x, w, y, pos, ws):
+    B, CO, CI, s = x.size(0), w.size(0), x.size(1), torch.cuda.current_stream().cuda_stream
+    assert lib.linf_inf_dist_forward_pruned(x.data_ptr(), w.data_ptr(), B, CO, CI, 1, 1, None, None, 0, y.data_ptr(), pos.data_ptr(), ws.data_ptr(), ws.numel(), s) == 0
+
+
+def new_outputs(lib, x, w):
+    n = lib.linf_inf_dist_forward_pruned_workspace_bytes(x.size(0), w.size(0), x.size(1), 1, 1)
+    assert n > 0
+    shape = (x.size(0), w.size(0), 1)
+    return (torch.full(shape, -7.0, device="cuda"), torch.full(shape, -7, dtype=torch.int32, device="cuda"), torch.empty(n, dtype=torch.uint8, device="cuda"))
+
+
+def full_scan(lib, x, w):
+    y, pos, _ = new_outputs(lib, x, w)
+    assert lib.linf_inf_dist_forward(x.data_ptr(), w.data_ptr(), x.size(0), w.size(0), x.size(1), 1, 1, y.data_ptr(), pos.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+    return y, pos
+
+
+@pytest.mark.parametrize("kind", ["normal", "narrow", "spikes"])
+@pytest.mark.parametrize("which", ["x", "w", "outputs", "all"])
+def test_unaligned_tensors(cuda, lib, which, kind):
+    torch.manual_seed(1)
+    x, w = make_x(kind, 640, 1024, 1), torch.randn(2304, 1024, device="cuda")
+    want, want_pos = full_scan(lib, x, w)
+    lo, up = x - 0.03, x + 0.03
+    s, sizes = torch.cuda.current_stream().cuda_stream, (640, 2304, 1024, 1, 1)
+    want_lo, want_up = torch.empty_like(want), torch.empty_like(want)
+    assert lib.linf_inf_dist_bound_forward(lo.data_ptr(), up.data_ptr(), w.data_ptr(), *sizes, want_lo.data_ptr(), want_up.data_ptr(), s) == 0
+    y, pos, ws = new_outputs(lib, x, w)
+    out_lo, out_up = torch.empty_like(y), torch.empty_like(y)
+    if which in ("x", "all"):
+        x, lo, up = off_by_one_float(x), off_by_one_float(lo), off_by_one_float(up)
+    if which in ("w", "all"):
+        w = off_by_one_float(w)
+    if which in ("outputs", "all"):
+        y, pos, out_lo, out_up = (off_by_one_float(t) for t in (y, pos, out_lo, out_up))
+    pruned_forward(lib, x, w, y, pos, ws)
+    assert torch.equal(y, want) and torch.equal(pos, want_pos)
+    n = lib.linf_inf_dist_bound_pruned_workspace_bytes(*sizes)
+    ws = torch.empty(n, dtype=torch.uint8, device="cuda")
+    assert lib.linf_inf_dist_bound_pruned(lo.data_ptr(), up.data_ptr(), w.data_ptr(), *sizes, None, None, 0, out_lo.data_ptr(), out_up.data_ptr(), ws.data_ptr(), n, s) == 0
+    assert torch.equal(out_lo, want_lo) and torch.equal(out_up, want_up)
+
+
+def test_under_graph_capture(cuda, lib):
+    """The decision between the lists and the dense kernel is taken on the device, at each replay on the data that are there then."""
+    torch.manual_seed(2)
+    w = torch.randn(2304, 1024, device="cuda")
+    x = make_x("narrow", 640, 1024, 1)
+    y, pos, ws = new_outputs(lib, x, w)
+    pruned_forward(lib, x, w, y, pos, ws)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        pruned_forward(lib, x, w, y, pos, ws)
+    for kind in ("narrow", "equal", "uniform", "spikes", "narrow"):
+        x.copy_(make_x(kind, 640, 1024, 1))
+        y.fill_(-7.0); pos.fill_(-7)
+        graph.replay()
+        want, want_pos = full_scan(lib, x, w)
+        assert torch.equal(y, want) and torch.equal(pos, want_pos), kind
+
+
+@pytest.mark.parametrize("streams", [1, 2])
+def test_two_host_threads(cuda, lib, streams):
+    """Two threads that call at the same time, on one stream or on one each, do not disturb each other's scratch."""
+    import threading
+    import linfdist_b200 as L
+    torch.manual_seed(3)
+    w = torch.randn(2304, 1024, device="cuda")
+    xs = [make_x("narrow", 640, 1024, 1), make_x("uniform", 640, 1024, 1)]
+    wants = [full_scan(lib, x, w)[0] for x in xs]
+    torch.cuda.synchronize()
+    side = [torch.cuda.Stream() for _ in range(streams)]
+    got, errors = [[], []], []
+
+    def work(k):
+        try:
+            with torch.cuda.stream(side[k % streams]):
+                for _ in range(20):
+                    got[k].append(L.norm_dist(xs[k], w, 1, float("inf")))
+        except Exception as e:                  # (a thread's exception would be lost)
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in (0, 1)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not errors
+    assert all(torch.equal(y, wants[k]) for k in (0, 1) for y in got[k])
