@@ -20,9 +20,9 @@
 // Bound: shared-memory gathers (a random 16-byte load of a warp takes about 10 cycles for 4 x 32 terms) and the 8-byte list entries
 // from L2.  How many entries there are depends on the data.  Dout = Din = 5120, B = 512: x uniform in [0,1) or activations of a
 // distance net, w ~ N(0,1): 20-45 of 5120; x and w ~ N(0,1): 240.  A gathered term costs as much as eight terms of the
-// dense kernel (bounds: five), which sets `budget`.  Measured on one B200, us, full scan -> here, B = 512, Dout = 5120: Din = 784, x uniform 176 -> 102;
-// Din = 3072, uniform 560 -> 150; Din = 5120, normal 908 -> 400, 0.25 * normal 902 -> 235; bounds Din = 3072, uniform 1403 -> 220, Din = 5120, normal
-// 2325 -> 600.  At Din = 5120, normal: sample 25, lists 28, gathers 2 x 160 (73-81 % of the shared-memory data path), failed outputs 8-30.
+// dense kernel (bounds: five), which sets `budget`.  Measured on one B200, us, full scan -> here, B = 512, Dout = 5120: Din = 784, x uniform 175 -> 100;
+// Din = 3072, uniform 560 -> 130; Din = 5120, normal 908 -> 400, 0.25 * normal 902 -> 223; bounds Din = 3072, uniform 1404 -> 190, Din = 5120, normal
+// 2325 -> 590.  At Din = 5120, normal: sample 25, lists 28, gathers 2 x 160 (73-81 % of the shared-memory data path), failed outputs 8-30.
 #include "common.cuh"
 
 namespace linf {
@@ -596,8 +596,9 @@ int run_pruned(const PruneParams& p, bool vec, cudaStream_t st) {
 
 // Which calls are worth the attempt: dense layers with long rows, and enough work that the sample, the lists and five launches (about
 // 30 us) are small against the full scan.  Measured, us, full scan / lists, B = 512, x = 0.25 * normal: 1024 x 1024 forward 63 / 60, bounds 122 / 77;
-// 784 x 5120 (x uniform) forward 176 / 107.  Data that turn out not to suit cost 25 us on top of the scan.  The kernels for rows that are no
-// multiple of four floats are three times slower, so that the line lies lower there (203 x 1027 x 1333, normal: 153 / 67).
+// 784 x 5120 (x uniform) forward 175 / 100.  The kernels for rows that are no multiple of four floats are three times slower, so that the line lies lower
+// there (203 x 1027 x 1333, normal: 153 / 67).  Data that do not suit cost, full scan alone / behind the lists, Dout = 5120: found by the sample 176 / 208 (Din = 784), 563 / 603 (3072), 910 / 956
+// (5120), bounds 409 / 443, 1405 / 1437, 2326 / 2364; found when half of the outputs have failed 173 / 245, 557 / 649, 899 / 1020, bounds 409 / 504, 1404 / 1521, 2326 / 2483.
 bool inf_prune_ok(const Dims& d, bool bound) {
     const double least = (d.CIg & 3) != 0 ? 1.5e8 : bound ? 5e8 : 1.5e9;
     return d.HW == 1 && d.CIg >= 256 && d.CIg <= kMaxK && d.COg >= 64 && d.R >= 64 &&
