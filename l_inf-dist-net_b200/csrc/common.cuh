@@ -147,7 +147,7 @@ size_t inf_forward_workspace(const Dims& d);
 bool inf_prune_ok(const Dims& d, bool bound);
 size_t inf_prune_workspace(const Dims& d, bool bound);
 int inf_prune(const float* xl, const float* xu, const float* w, const Dims& d, float* y0, int* pos, float* y1, bool bound,
-              void* ws, cudaStream_t st, const Post& post, float dense_speed, const int** only_if);
+              void* ws, cudaStream_t st, const Post& post, float dense_speed, const int** only_if, int* tickets = nullptr, int n_tickets = 0);
 size_t inf_forward_pruned_workspace(const Dims& d);
 int inf_forward_pruned(const float* x, const float* w, const Dims& d, float* y, int* pos,
                        void* ws, size_t ws_bytes, cudaStream_t st, const Post& post);
@@ -155,7 +155,7 @@ size_t inf_bound_pruned_workspace(const Dims& d);
 int inf_bound_pruned(const float* xl, const float* xu, const float* w, const Dims& d, float* yl, float* yu,
                      void* ws, size_t ws_bytes, cudaStream_t st, const Post& post);
 int inf_bound(const float* xl, const float* xu, const float* w, const Dims& d,
-              float* yl, float* yu, cudaStream_t st, const Post& post = Post{nullptr, nullptr, 0}, const int* only_if = nullptr);
+              float* yl, float* yu, cudaStream_t st, const Post& post = Post{nullptr, nullptr, 0}, const int* only_if = nullptr, int* tickets = nullptr);
 // batch-mean shift of a [rows, cols] activation (epilogue.cu)
 // sparse_exchange.cu: row lists of a sparse gradient, merged across ranks over peer memory
 int grad_rows_compact(float* grad, int rows, int cols, int cap, int* cnt, void* ent, int* err, cudaStream_t st);

@@ -95,8 +95,9 @@ struct BoundParams {
     const float* xl; const float* xu; const float* w; float* yl; float* yu;
     int M, N, K, G, lda, ldo, tiles_m, tiles_n, KT;
     int ksplit;            // CTAs per output tile, each with an equal share of the k-tiles (1 or 2)
-    Post post;             // per-channel epilogue of the stored bounds (all null: none; ksplit == 1 only)
+    Post post;             // per-channel epilogue of the stored bounds (all null: none; ksplit > 1: with tickets only)
     const int* only_if;    // not null: the launch does nothing where this word is 0
+    int* tickets;          // ksplit > 1: null, or one word per tile, 0: the CTA that comes second applies `post`
 };
 
 __device__ __forceinline__ void load_stage(float* stage, const BoundParams& p, int g, int m0, int n0,
@@ -253,6 +254,20 @@ inf_bound_tiled_kernel(const BoundParams p) {
                 }
             }
         }
+        if (p.tickets == nullptr) return;
+        __threadfence();
+        __syncthreads();
+        if (!__syncthreads_or(tid == 0 && atomicAdd(p.tickets + tile, 1) == 1)) return;
+        __threadfence();
+        for (int e = tid; e < BM * BN; e += NT) {
+            const int m = m0 + e / BN, n = n0 + e % BN;
+            if (m < p.M && n < p.N) {
+                const size_t o = (size_t)m * p.ldo + (size_t)g * p.N + n;
+                const float lo = post_apply(p.post, __ldcg(p.yl + o), g * p.N + n), up = post_apply(p.post, __ldcg(p.yu + o), g * p.N + n);
+                p.yl[o] = p.post.negate ? up : lo;
+                p.yu[o] = p.post.negate ? lo : up;
+            }
+        }
         return;
     }
 #pragma unroll
@@ -274,10 +289,9 @@ inf_bound_tiled_kernel(const BoundParams p) {
     }
 }
 
-// The per-channel epilogue as a pass of its own, for launches that combined partial results in memory.  only_if: as above.
+// The per-channel epilogue as a pass of its own, for launches that combined partial results in memory without tickets.
 __global__ void __launch_bounds__(256)
-inf_bound_post_kernel(float* __restrict__ yl, float* __restrict__ yu, size_t n, int CO, Post post, const int* __restrict__ only_if) {
-    if (only_if != nullptr && *only_if == 0) return;
+inf_bound_post_kernel(float* __restrict__ yl, float* __restrict__ yu, size_t n, int CO, Post post) {
     for (size_t e = (size_t)blockIdx.x * 256 + threadIdx.x; e < n; e += (size_t)gridDim.x * 256) {
         const int c = (int)(e % (size_t)CO);
         const float lo = post_apply(post, yl[e], c), up = post_apply(post, yu[e], c);
@@ -296,9 +310,10 @@ int k_split(int tiles, int KT) {
 
 }  // namespace
 
-// only_if: not null: nothing is done where this word is 0, and where it is not, the outputs have been cleared on the device.
+// only_if: not null: nothing is done where this word is 0, and where it is not, the outputs and tickets (one per tile) have been cleared on the device.  (A
+// second launch for the epilogue would cost the calls that the lists serve 4 us.)
 int inf_bound(const float* xl, const float* xu, const float* w, const Dims& d,
-              float* yl, float* yu, cudaStream_t st, const Post& post, const int* only_if) {
+              float* yl, float* yu, cudaStream_t st, const Post& post, const int* only_if, int* tickets) {
     const bool tiled = d.HW == 1 && (d.CIg % 4) == 0 && aligned16(xl) && aligned16(xu) && aligned16(w) &&
                        d.COg >= 32;
     if (!tiled) {
@@ -314,6 +329,8 @@ int inf_bound(const float* xl, const float* xu, const float* w, const Dims& d,
     p.M = d.R; p.N = d.COg; p.K = d.CIg; p.G = d.G; p.lda = d.CI; p.ldo = d.CO;
     p.post = post;
     p.only_if = only_if;
+    const bool has_post = post.sub != nullptr || post.add != nullptr || post.negate;
+    p.tickets = has_post ? tickets : nullptr;
     p.tiles_m = (d.R + BM - 1) / BM; p.tiles_n = (d.COg + BN - 1) / BN;
     p.KT = (d.CIg + BK - 1) / BK;
     int grid = p.tiles_m * p.tiles_n * d.G;
@@ -330,16 +347,22 @@ int inf_bound(const float* xl, const float* xu, const float* w, const Dims& d,
         return LINF_ERR_LAUNCH;
     inf_bound_tiled_kernel<<<grid, NT, SMEM_BYTES, st>>>(p);
     int launched = 1;
-    if (p.ksplit > 1 && (post.sub != nullptr || post.add != nullptr || post.negate)) {
+    if (p.ksplit > 1 && has_post && tickets == nullptr) {
         const size_t n = (size_t)d.R * d.CO;
-        inf_bound_post_kernel<<<2 * sm_count(), 256, 0, st>>>(yl, yu, n, d.CO, post, only_if);
+        inf_bound_post_kernel<<<2 * sm_count(), 256, 0, st>>>(yl, yu, n, d.CO, post);
         launched = 2;
     }
     return launch_status(launched);
 }
 
 // The bounds through lists of large entries where that may pay (inf_prune.cu), the dense kernel behind.
-size_t inf_bound_pruned_workspace(const Dims& d) { return inf_prune_workspace(d, true); }
+static size_t up256(size_t n) { return (n + 255) & ~(size_t)255; }
+static size_t tile_count(const Dims& d) { return (size_t)((d.R + BM - 1) / BM) * ((d.COg + BN - 1) / BN) * d.G; }
+
+size_t inf_bound_pruned_workspace(const Dims& d) {
+    const size_t lists = inf_prune_workspace(d, true);
+    return lists == 0 ? 0 : up256(lists) + tile_count(d) * sizeof(int);
+}
 
 int inf_bound_pruned(const float* xl, const float* xu, const float* w, const Dims& d, float* yl, float* yu,
                      void* ws, size_t ws_bytes, cudaStream_t st, const Post& post) {
@@ -347,10 +370,11 @@ int inf_bound_pruned(const float* xl, const float* xu, const float* w, const Dim
     if (need == 0 || ws == nullptr) return inf_bound(xl, xu, w, d, yl, yu, st, post);
     if (ws_bytes < need || (reinterpret_cast<uintptr_t>(ws) & 255u)) return LINF_ERR_WORKSPACE;
     const int* only_if = nullptr;
+    int* tickets = reinterpret_cast<int*>(reinterpret_cast<char*>(ws) + up256(inf_prune_workspace(d, true)));
     const bool tiled = (d.CIg % 4) == 0 && aligned16(xl) && aligned16(xu) && aligned16(w);
-    const int rc = inf_prune(xl, xu, w, d, yl, nullptr, yu, true, ws, st, post, tiled ? 1.f : 0.25f, &only_if);
+    const int rc = inf_prune(xl, xu, w, d, yl, nullptr, yu, true, ws, st, post, tiled ? 1.f : 0.25f, &only_if, tickets, (int)tile_count(d));
     if (rc) return rc;
-    return inf_bound(xl, xu, w, d, yl, yu, st, post, only_if);
+    return inf_bound(xl, xu, w, d, yl, yu, st, post, only_if, tickets);
 }
 
 }  // namespace linf

@@ -57,6 +57,7 @@ struct PruneParams {
     int slots;
     int vec;                                    // y and pos take 16-byte stores at multiples of four outputs
     float budget;                               // entries per output at which the dense kernel is as fast
+    int* tickets; int n_tickets;                // words that the dense kernel of the bounds wants cleared
     Post post;
 };
 
@@ -454,6 +455,7 @@ fail_kernel(const PruneParams p) {
         if (BOUND) {
             const size_t outs = (size_t)p.R * p.CO;
             for (size_t e = (size_t)blockIdx.x * 128 + tid; e < outs; e += (size_t)gridDim.x * 128) { p.y0[e] = 0.f; p.y1[e] = 0.f; }
+            for (int e = blockIdx.x * 128 + tid; e < p.n_tickets; e += gridDim.x * 128) p.tickets[e] = 0;
         }
         return;
     }
@@ -608,9 +610,9 @@ bool inf_prune_ok(const Dims& d, bool bound) {
 size_t inf_prune_workspace(const Dims& d, bool bound) { return inf_prune_ok(d, bound) ? prune_sizes(d, bound).total : 0; }
 
 // The list pass over a workspace of inf_prune_workspace bytes.  *only_if receives the device flag under which the dense kernel must
-// run behind it.  dense_speed: terms per second of the kernel behind, relative to the tiled ones.
+// run behind it.  dense_speed: terms per second of the kernel behind, relative to the tiled ones.  tickets: words to clear for that kernel (bounds).
 int inf_prune(const float* xl, const float* xu, const float* w, const Dims& d, float* y0, int* pos, float* y1, bool bound,
-              void* ws, cudaStream_t st, const Post& post, float dense_speed, const int** only_if) {
+              void* ws, cudaStream_t st, const Post& post, float dense_speed, const int** only_if, int* tickets, int n_tickets) {
     const PruneSizes s = prune_sizes(d, bound);
     char* base = reinterpret_cast<char*>(ws);
     PruneParams p;
@@ -627,6 +629,7 @@ int inf_prune(const float* xl, const float* xu, const float* w, const Dims& d, f
     const float gather_cost = bound ? 5.f : 8.5f;
     p.budget = 0.9f * d.CIg / (gather_cost * dense_speed);
     p.post = post;
+    p.tickets = tickets; p.n_tickets = n_tickets;
     *only_if = &p.head->dense;
     const bool vec = (d.CIg & 3) == 0 && aligned16(xl) && aligned16(xu) && aligned16(w);
     if (bound) return run_pruned<true, false>(p, vec, st);
