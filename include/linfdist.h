@@ -245,6 +245,9 @@ int linf_norm_dist_backward_weight(const float* grad_output, const float* input,
 
 /*
  * linf_norm_dist_forward with scratch for the maximum pass (same rules for the workspace as below; same result).
+ * Infinities and NaN (here, in linf_norm_dist_forward and in linf_norm_dist_backward): a term counts min(|t| / M, 1)^p, in the gradients min(|t| / y, 1)^(p-1),
+ * with min(NaN, 1) = 1, for every call but dense ones (HW == 1) whose channel counts per group are multiples of four from 32 on with all tensors 16-byte aligned: those have no
+ * rule for such data, and their results are NaN.
  */
 size_t linf_norm_dist_forward_workspace_bytes(int B, int CO, int CI, int G, int HW, float p);
 int linf_norm_dist_forward_ws(const float* input, const float* weight, int B, int CO, int CI, int G, int HW,
