@@ -57,6 +57,7 @@ struct PruneParams {
     int slots;
     int vec;                                    // y and pos take 16-byte stores at multiples of four outputs
     float budget;                               // entries per output at which the dense kernel is as fast
+    float x_pass;                               // what a pass with lists of x costs, in entries per output
     int* tickets; int n_tickets;                // words that the dense kernel of the bounds wants cleared
     Post post;
 };
@@ -192,7 +193,7 @@ sample_kernel(const PruneParams p) {
         // Lists of x that are (with a bin to spare) empty spare a pass over the weights and the outputs, about a dozen entries' worth, and the building and reading of
         // those lists, a fixed time per row of x.  Measured on bounds, entries' worth per output: 58 with 64 outputs per group, 32 - 36 with 128, 23 with 256, 12 with 1000, 2 - 5 with
         // 3000 and more (100000 x 256 x 64, x = 0.2 * normal, where a constant 12 chose the lists: 300 us by the full scan, 700 by the lists, 357 now).
-        const float c = nx + nw + (hx[j - 1] == 0 ? 0.f : 12.f + 3000.f / p.N);
+        const float c = nx + nw + (hx[j - 1] == 0 ? 0.f : p.x_pass);
         if (nx <= 0.6f * p.slots && nw <= 0.6f * p.slots && c < cost) { cost = c; bin = j; }
     }
 #pragma unroll
@@ -631,6 +632,7 @@ int inf_prune(const float* xl, const float* xu, const float* w, const Dims& d, f
     const float gather_cost = bound ? 5.f : 8.5f;
     p.budget = 0.9f * d.CIg / (gather_cost * dense_speed);
     p.post = post;
+    p.x_pass = 12.f + 3000.f / d.COg;
     p.tickets = tickets; p.n_tickets = n_tickets;
     *only_if = &p.head->dense;
     const bool vec = (d.CIg & 3) == 0 && aligned16(xl) && aligned16(xu) && aligned16(w);
